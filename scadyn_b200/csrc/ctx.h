@@ -93,9 +93,8 @@ struct scd_ctx {
     // the octant transposed for the fused y-z FFT pass (fft_yz.cuh), FP64 and
     // complex64, rebuilt after every new Green spectrum
     bool yz_on = true;                   // take the fused y-z pass where its lengths allow
-    // right-hand sides per warp of the anterpolation and interpolation
-    // kernels (0 = all of a call's; smaller spans give more warps in flight,
-    // larger ones reuse the projector rows from L1)
+    // right-hand sides per block of the anterpolation and per warp of the
+    // interpolation (0 = chosen from the sizes, rhs_span)
     int scatter_span = 0, gather_span = 0;
     bool fyz_ready = false, fyz_ready_f = false;
     cd *d_Fyz = nullptr;

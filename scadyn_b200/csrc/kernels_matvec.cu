@@ -23,16 +23,15 @@
 namespace {
 
 constexpr int WARPS_PER_CTA = 4;
-// anterpolation of eight or more right-hand sides with one CTA per cube
-// (k_scatter_cta) instead of one warp
-#ifndef SCD_SG_CTA
-#define SCD_SG_CTA 1
-#endif
 // resident CTAs per SM the complex64 interpolation kernel is compiled for
 // (its register cap): at C2 with 32 right-hand sides 0.75 ms with 3 (160
 // registers), 0.90 with 1 (174), 1.07 with 4 or 5 (spills)
 #ifndef SCD_GATHER_MINB
 #define SCD_GATHER_MINB 3
+#endif
+// interpolation warps per SM that the spans of right-hand sides aim at
+#ifndef SCD_GATHER_WARPS
+#define SCD_GATHER_WARPS 24
 #endif
 
 // slot order <-> the reference's unknown order (nb basis functions per tet:
@@ -56,117 +55,76 @@ __global__ void k_permute_out(const cd *__restrict__ xs, cd *__restrict__ xo, co
 }
 
 // ---------------------------------------------------------------- scatter
-// Anterpolation (sparse_T_matmul, src/sparse.f90:13-43), one warp per
-// (cube, span of rspan right-hand sides): lane j < 27 accumulates the four
-// box-node sums of node j over the cube's tets, SC_RG right-hand sides at a
-// time (projector values are read once per group of SC_RG and stay in L1 for
-// the next group of the span).  The spans are the grid's y index; rspan is a
-// multiple of SC_RG.  Projectors are stored P[(g*27 + j)*T + slot].
-// bpart[((r*ncubes + c)*4 + g)*27 + j].
-template <typename C, int SC_RG>
-__global__ void __launch_bounds__(32 * WARPS_PER_CTA)
-k_scatter(const C *__restrict__ x, long long ld, const C *__restrict__ P, int T,
-          const int *__restrict__ cube_off, int ncubes, C *__restrict__ bpart, const int *skip, int nrhs, int rspan) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = blockIdx.x * WARPS_PER_CTA + warp;
-    if (c >= ncubes || lane >= 27) return;
-    const int s0 = cube_off[c], s1 = cube_off[c + 1];
-    const C *P0 = P + (size_t)lane * T, *PX = P + (size_t)(27 + lane) * T;
-    const C *PY = P + (size_t)(54 + lane) * T, *PZ = P + (size_t)(81 + lane) * T;
-    const int rend = min(nrhs, (int)(blockIdx.y + 1) * rspan);
-    for (int r0 = blockIdx.y * rspan; r0 < rend; r0 += SC_RG) {
-        C acc[SC_RG][4];
-#pragma unroll
-        for (int q = 0; q < SC_RG; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = czero<C>();
-#pragma unroll 4
-        for (int s = s0; s < s1; ++s) {
-            const C p0 = P0[s], px = PX[s], py = PY[s], pz = PZ[s];
-#pragma unroll
-            for (int q = 0; q < SC_RG; ++q) {
-                const int r = r0 + q;
-                if (r < nrhs) {
-                    const C *xr = x + r * ld + 3LL * s;
-                    const C x0 = xr[0], x1 = xr[1], x2 = xr[2];
-                    cfma(acc[q][0], p0, x0);
-                    cfma(acc[q][1], p0, x1);
-                    cfma(acc[q][2], p0, x2);
-                    cfma(acc[q][3], px, x0);
-                    cfma(acc[q][3], py, x1);
-                    cfma(acc[q][3], pz, x2);
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < SC_RG; ++q) {
-            const int r = r0 + q;
-            if (r < nrhs && !(skip && skip[r])) {
-                C *o = bpart + ((long long)r * ncubes + c) * 4 * 27 + lane;
-                o[0] = acc[q][0];
-                o[27] = acc[q][1];
-                o[54] = acc[q][2];
-                o[81] = acc[q][3];
-            }
-        }
-    }
+// Anterpolation (sparse_T_matmul, src/sparse.f90:13-43): the four box-node
+// sums of the 27 nodes of every cube, one CTA per (cube, span of right-hand
+// sides).  Projectors are stored P[(g*27 + j)*T + slot]; the cube's 108 rows
+// are contiguous runs of its tets and are staged in shared memory NTC tets
+// at a time by asynchronous copies, 16 threads to a row, all in flight at
+// once, with the right-hand sides' x segments beside them, so that the sums
+// read shared memory only.  Each sum runs over the tets in ascending order
+// (grid 3: x, y, z of a tet in turn) in every variant, so a column gives the
+// same bits alone and in a batch.  The row stride NTC + 1 keeps the lanes'
+// reads of one tet in distinct banks.  bpart[((r*ncubes + c)*4 + g)*27 + j].
+constexpr int SCB = 128;
+template <typename C, int NTC>
+__device__ __forceinline__ void stage_projectors(C (*Ps)[NTC + 1], const C *__restrict__ P, int T, int s, int m) {
+    for (int row = threadIdx.x >> 4; row < 108; row += SCB / 16)
+        for (int t = threadIdx.x & 15; t < m; t += 16)
+            cp_async_el<(int)sizeof(C)>(&Ps[row][t], P + (size_t)row * T + s + t, true);
 }
 
-// The same anterpolation for many right-hand sides, one CTA per (cube, span
-// of right-hand sides): the cube's projector rows are staged in shared
-// memory by the whole CTA (coalesced over the cube's tets, NTC at a time),
-// and the four warps take SR right-hand sides each per round, lane j < 27
-// summing node j over the tets in ascending order from shared memory -- the
-// order of k_scatter, so a column gives the same bits through either.  The
-// row stride NTC + 1 keeps the lanes' reads of one tet in distinct banks.
-constexpr int SCB = 128;
+// Eight or more right-hand sides: the four warps take SR of them each per
+// round, lane j < 27 sums node j.  Bound by latency, so everything a round
+// reads is in flight before the sums start: 16 FP64 right-hand sides of a
+// 12,864-tet sphere take 29 us (68 with x read from global memory tet by tet
+// and rows staged through registers), 32 complex64 ones of 60k tets 106 us
+// (178).
 template <typename C, int NTC, int SR>
 __global__ void __launch_bounds__(SCB)
 k_scatter_cta(const C *__restrict__ x, long long ld, const C *__restrict__ P, int T, const int *__restrict__ cube_off,
               int ncubes, C *__restrict__ bpart, const int *skip, int nrhs, int rspan) {
     __shared__ C Ps[108][NTC + 1];
+    __shared__ C xs[4][SR][3 * NTC];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x;
     const int s0 = cube_off[c], nt = cube_off[c + 1] - s0;
     const int rlo = blockIdx.y * rspan, rhi = min(nrhs, rlo + rspan);
     const int nround = (rhi - rlo + 4 * SR - 1) / (4 * SR);
     const bool one = nt <= NTC;
-    auto stage = [&](int t0) {
-        const int m = min(NTC, nt - t0);
-        for (int e = threadIdx.x; e < 108 * m; e += SCB) {
-            const int row = e / m, t = e - row * m;
-            Ps[row][t] = P[(size_t)row * T + s0 + t0 + t];
-        }
-    };
-    if (one && nt > 0) stage(0);
-    __syncthreads();
+    if (one) stage_projectors<C, NTC>(Ps, P, T, s0, nt);
     for (int rd = 0; rd < nround; ++rd) {
         const int rb = rlo + (rd * 4 + warp) * SR;
         C acc[SR][4];
 #pragma unroll
         for (int q = 0; q < SR; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = czero<C>();
         for (int t0 = 0; t0 < nt; t0 += NTC) {
+            const int m = min(NTC, nt - t0);
             if (!one) {
                 __syncthreads();
-                stage(t0);
-                __syncthreads();
+                stage_projectors<C, NTC>(Ps, P, T, s0 + t0, m);
             }
-            const int m = min(NTC, nt - t0);
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < SR; ++q) {
+                const C *xr = x + (rb + q) * ld + 3LL * (s0 + t0);
+                for (int e = lane; e < 3 * m; e += 32)
+                    if (rb + q < rhi) cp_async_el<(int)sizeof(C)>(&xs[warp][q][e], xr + e, true);
+            }
+            cp_async_wait_all();
+            if (!one || rd == 0) __syncthreads();
+            else __syncwarp();
             if (lane < 27) {
                 for (int t = 0; t < m; ++t) {
                     const C p0 = Ps[lane][t], px = Ps[27 + lane][t], py = Ps[54 + lane][t], pz = Ps[81 + lane][t];
-                    const long long s = s0 + t0 + t;
 #pragma unroll
                     for (int q = 0; q < SR; ++q) {
-                        const int r = rb + q;
-                        if (r < rhi) {
-                            const C *xr = x + r * ld + 3LL * s;
-                            const C x0 = xr[0], x1 = xr[1], x2 = xr[2];
-                            cfma(acc[q][0], p0, x0);
-                            cfma(acc[q][1], p0, x1);
-                            cfma(acc[q][2], p0, x2);
-                            cfma(acc[q][3], px, x0);
-                            cfma(acc[q][3], py, x1);
-                            cfma(acc[q][3], pz, x2);
-                        }
+                        const C x0 = xs[warp][q][3 * t], x1 = xs[warp][q][3 * t + 1], x2 = xs[warp][q][3 * t + 2];
+                        cfma(acc[q][0], p0, x0);
+                        cfma(acc[q][1], p0, x1);
+                        cfma(acc[q][2], p0, x2);
+                        cfma(acc[q][3], px, x0);
+                        cfma(acc[q][3], py, x1);
+                        cfma(acc[q][3], pz, x2);
                     }
                 }
             }
@@ -182,6 +140,64 @@ k_scatter_cta(const C *__restrict__ x, long long ld, const C *__restrict__ P, in
                     o[54] = acc[q][2];
                     o[81] = acc[q][3];
                 }
+            }
+        }
+    }
+}
+
+// Fewer than eight right-hand sides: warp g sums grid g for SR of them at a
+// time, so that all four warps work on a single one.  Bound by the projector
+// rows (4*27*T values, read once): one FP64 right-hand side takes 69 us at
+// 150,720 tets, 3.8 TB/s of them, and 8 us at 1,680 (157 and 24 with one
+// warp per cube reading its rows a tet at a time).
+template <typename C, int NTC, int SR>
+__global__ void __launch_bounds__(SCB)
+k_scatter_few(const C *__restrict__ x, long long ld, const C *__restrict__ P, int T, const int *__restrict__ cube_off,
+              int ncubes, C *__restrict__ bpart, const int *skip, int nrhs) {
+    __shared__ C Ps[108][NTC + 1];
+    __shared__ C xs[SR][3 * NTC];
+    const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int c = blockIdx.x;
+    const int s0 = cube_off[c], nt = cube_off[c + 1] - s0;
+    for (int r0 = 0; r0 < nrhs; r0 += SR) {
+        C acc[SR];
+#pragma unroll
+        for (int q = 0; q < SR; ++q) acc[q] = czero<C>();
+        for (int t0 = 0; t0 < nt; t0 += NTC) {
+            const int m = min(NTC, nt - t0);
+            __syncthreads();
+            if (r0 == 0 || nt > NTC) stage_projectors<C, NTC>(Ps, P, T, s0 + t0, m);
+#pragma unroll
+            for (int q = 0; q < SR; ++q)
+                if (r0 + q < nrhs)
+                    for (int e = threadIdx.x; e < 3 * m; e += SCB)
+                        cp_async_el<(int)sizeof(C)>(&xs[q][e], x + (r0 + q) * ld + 3LL * (s0 + t0) + e, true);
+            cp_async_wait_all();
+            __syncthreads();
+            if (lane >= 27) continue;
+            if (g < 3) {
+                for (int t = 0; t < m; ++t) {
+                    const C p0 = Ps[lane][t];
+#pragma unroll
+                    for (int q = 0; q < SR; ++q) cfma(acc[q], p0, xs[q][3 * t + g]);
+                }
+            } else {
+                for (int t = 0; t < m; ++t) {
+                    const C px = Ps[27 + lane][t], py = Ps[54 + lane][t], pz = Ps[81 + lane][t];
+#pragma unroll
+                    for (int q = 0; q < SR; ++q) {
+                        cfma(acc[q], px, xs[q][3 * t]);
+                        cfma(acc[q], py, xs[q][3 * t + 1]);
+                        cfma(acc[q], pz, xs[q][3 * t + 2]);
+                    }
+                }
+            }
+        }
+        if (lane < 27) {
+#pragma unroll
+            for (int q = 0; q < SR; ++q) {
+                const int r = r0 + q;
+                if (r < nrhs && !(skip && skip[r])) bpart[((long long)r * ncubes + c) * 4 * 27 + 27 * g + lane] = acc[q];
             }
         }
     }
@@ -1149,6 +1165,24 @@ bool ensure_fyz(scd_ctx *c) {
     return true;
 }
 
+// Right-hand sides that one block of the anterpolation (one warp of the
+// interpolation) walks: a tuned span, or the most that still gives every SM
+// `per_sm` of the `items` x spans blocks (the anterpolation's five resident
+// CTAs; two waves of the interpolation's twelve warps).  A longer span reads
+// the projector rows fewer times, a shorter one keeps a small mesh from
+// leaving SMs idle: 32 complex64 right-hand sides of 6,144 tets (300 groups)
+// interpolate in 32 us with spans of 4, in 91 with one span of 32; at 60k
+// tets both take 335.
+int rhs_span(const scd_ctx *c, int tuned, int nrhs, int items, int unit, int per_sm) {
+    int sp = tuned;
+    if (sp <= 0) {
+        const long long want = (long long)per_sm * c->nsm;
+        const long long spans = std::min<long long>((nrhs + unit - 1) / unit, (want + items - 1) / std::max(items, 1));
+        sp = (int)((nrhs + spans - 1) / std::max<long long>(spans, 1));
+    }
+    return (sp + unit - 1) / unit * unit;
+}
+
 #define SCD_DISPATCH_P(PV, CALL)                     \
     switch (PV) {                                    \
         case 8: CALL(8); break;                      \
@@ -1168,28 +1202,19 @@ template <typename C>
 void fft_chain_t(scd_ctx *c, const C *x, int nrhs, const int *done) {
     const GridDims G = dims_of(c);
     {
-        const unsigned gx = (unsigned)((c->ncubes + WARPS_PER_CTA - 1) / WARPS_PER_CTA);
         const C *P = Res<C>::P(c);
-        // spans of right-hand sides per warp (c->scatter_span, 0 = all of them)
-        auto span = [&](int rg) { int sp = c->scatter_span > 0 ? c->scatter_span : nrhs; return (sp + rg - 1) / rg * rg; };
-        if (nrhs >= 8 && SCD_SG_CTA) {
-            // one CTA per cube (projector rows shared through shared memory)
-            constexpr int NTC = sizeof(C) == 8 ? 32 : 16;
-            const int sp = span(4);
+        constexpr int NTC = sizeof(C) == 8 ? 32 : 16, NTF = sizeof(C) == 8 ? 32 : 24;   // static shared memory: 48 KB
+        const dim3 gx((unsigned)c->ncubes);
+        if (nrhs >= 8) {
+            const int sp = rhs_span(c, c->scatter_span, nrhs, c->ncubes, 16, 5);
             k_scatter_cta<C, NTC, 4><<<dim3((unsigned)c->ncubes, (nrhs + sp - 1) / sp), SCB, 0, c->st>>>(
                 x, c->n, P, c->T, c->d_cube_off, c->ncubes, Res<C>::bpart(c), done, nrhs, sp);
-        } else if (nrhs >= 8) {
-            const int sp = span(8);
-            k_scatter<C, 8><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(
-                x, c->n, P, c->T, c->d_cube_off, c->ncubes, Res<C>::bpart(c), done, nrhs, sp);
-        } else if (nrhs >= 4) {
-            const int sp = span(4);
-            k_scatter<C, 4><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(
-                x, c->n, P, c->T, c->d_cube_off, c->ncubes, Res<C>::bpart(c), done, nrhs, sp);
+        } else if (nrhs >= 2) {
+            k_scatter_few<C, NTF, 4><<<gx, SCB, 0, c->st>>>(x, c->n, P, c->T, c->d_cube_off, c->ncubes,
+                                                            Res<C>::bpart(c), done, nrhs);
         } else {
-            const int sp = span(1);
-            k_scatter<C, 1><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(
-                x, c->n, P, c->T, c->d_cube_off, c->ncubes, Res<C>::bpart(c), done, nrhs, sp);
+            k_scatter_few<C, NTF, 1><<<gx, SCB, 0, c->st>>>(x, c->n, P, c->T, c->d_cube_off, c->ncubes,
+                                                            Res<C>::bpart(c), done, nrhs);
         }
     }
     const int nrg = 4 * nrhs;
@@ -1292,15 +1317,13 @@ void gather_t(scd_ctx *c, C *y, int nrhs, const int *done) {
     if (c->ngroups == 0) return;
     typedef typename CReal<C>::type R;
     const R k2 = (R)(c->k * c->k);
-    // spans of right-hand sides per warp (c->gather_span, 0 = all of them)
-    auto span = [&](int rg) { int sp = c->gather_span > 0 ? c->gather_span : nrhs; return (sp + rg - 1) / rg * rg; };
     if (nrhs >= 4) {
-        const int sp = span(4);
+        const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, 4, SCD_GATHER_WARPS);
         k_gather<C, 4><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(
             Res<C>::R(c), Res<C>::P(c), c->T, c->d_grp_off, c->d_grp_cube, c->ngroups, G, k2, Res<C>::part(c),
             c->part_len, c->d_pslot_base, c->d_pslot_cnt, y, c->n, done, nrhs, sp);
     } else {
-        const int sp = span(1);
+        const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, 1, SCD_GATHER_WARPS);
         k_gather<C, 1><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(
             Res<C>::R(c), Res<C>::P(c), c->T, c->d_grp_off, c->d_grp_cube, c->ngroups, G, k2, Res<C>::part(c),
             c->part_len, c->d_pslot_base, c->d_pslot_cnt, y, c->n, done, nrhs, sp);
