@@ -50,12 +50,14 @@ template <typename C>
 struct TickArgs {
     Slot *slots;
     int ns;
-    C *V;           // [slot][m+1][n]
+    C *V;           // [slot][chunk][m+1][L], see basis_of
     cd *H;          // [slot][(m+1) m]
     cd *cs, *sn, *g, *y;   // [slot][m+1]
     C *x, *rhs, *w; // [slot][n]
     double *red;    // [2][grid][NSMAX*4]
-    double *cpart;  // [NSMAX][NCH][4] chunk partials
+    double *cpart;  // [slot][nch][4] chunk partials
+    double *rnorm;  // [slot][nch] chunk partials of ||w||^2 (resident Gram-Schmidt)
+    int res;        // resident Gram-Schmidt: items per warp, 0 = off
     double *ctot;   // [2][NSMAX][4] slot totals
     int *ccnt;      // [NSMAX] chunks published in the current reduction
     int *qctr;      // [QMAX] work-queue counters, one per phase of the tick
@@ -66,7 +68,7 @@ struct TickArgs {
     double tol;
     int mixed;      // inner solve of the mixed form: finish -> INNER_DONE
     int cgs;        // classical Gram-Schmidt for the Arnoldi steps (complex64 inner solves, opt-in)
-    double *cpm;    // cgs: [slot][NCH][CGS_NV] chunk partials of the dots
+    double *cpm;    // cgs: [slot][CGS_NV][nch] chunk partials of the dots
     double *ctm;    // cgs: [slot][CGS_NV] slot totals
 };
 
@@ -86,30 +88,76 @@ template <> __device__ __forceinline__ cd rounded<cf>(cd v) { return widen(make_
 constexpr int TU = 4;
 
 // ---- reductions over fixed chunks
-// Every slot vector is cut into NCH fixed chunks; chunk c of slot s is
-// always handled by global warp (s*NCH + c) mod (warps in the grid), its
-// lanes take elements q = c*L + lane + 32t in order (TU at a time, loads
-// first), the lanes' sums meet in an xor tree, and the last warp to finish a
-// slot adds its NCH chunk partials (lane l: chunks l, l+32, ..., then an xor
-// tree) into the slot's total.  The arithmetic of a slot therefore depends
-// on n and the grid only -- never on which other slots are active -- and
-// each warp streams long contiguous runs (deep memory-level parallelism).
-constexpr int NCH = 512;
+// Every slot vector is cut into nch <= NCH fixed chunks of L elements: CHUNK
+// elements (eight per lane) while NCH chunks cover the vector, longer ones
+// beyond.  The partition depends on n only.  A chunk's lanes take elements
+// q = c*L + lane + 32t in order (TU at a time, loads first), the lanes' sums
+// meet in an xor tree, and the chunk partials of a slot are added in chunk
+// order (lane l: chunks l, l+32, ..., then an xor tree).  The arithmetic of a
+// slot therefore depends on n only -- never on which other slots are active
+// or which warp took a chunk.  Short chunks cost more than they spread: with
+// 512 chunks for every n, a vector of 18,432 unknowns gave a warp 36 elements
+// and 16 partials to each lane of the final sums, and the tick of 32 slots
+// took 160 us; 72 chunks of 256 and the phases below take 43.
+constexpr int NCH = 2048;
+constexpr int CHUNK = 256;
 // values per slot of the classical Gram-Schmidt reduction: <v_k, w> for k <=
 // SCD_M_MAX (two doubles each) and ||w||^2
 constexpr int CGS_NV = 2 * SCD_M_MAX + 2;
 
+// lane's share of nch chunk partials p[c * stride], c = lane, lane + 32, ...:
+// added in chunk order, up to sixteen loads at a time
+template <int NV>
+__device__ __forceinline__ void lane_partials(const double *p, int stride, int nch, int lane, double (&t)[NV]) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) t[k] = 0.0;
+    constexpr int U = NV == 1 ? 16 : NV == 2 ? 8 : 4;
+    for (int c0 = lane; c0 < nch; c0 += 32 * U) {
+        double pv[U][NV];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) pv[j][k] = c0 + 32 * j < nch ? __ldcg(p + (size_t)(c0 + 32 * j) * stride + k) : 0.0;
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) t[k] += pv[j][k];
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+}
+
 struct Chunks {
     long long L;    // chunk length
+    int nch;        // chunks
     int gw, nw;     // this warp, warps in the grid
     int lane;
-    __device__ Chunks(long long n, int nch) {
-        L = (n + nch - 1) / nch;
+    static __host__ __device__ long long length(long long n) {
+        return n <= (long long)NCH * CHUNK ? CHUNK : ((n + NCH - 1) / NCH + CHUNK - 1) / CHUNK * CHUNK;
+    }
+    static __host__ __device__ int count(long long n) { return (int)((n + length(n) - 1) / length(n)); }
+    __device__ explicit Chunks(long long n) {
+        L = length(n);
+        nch = count(n);
         gw = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
         nw = (int)(((long long)gridDim.x * blockDim.x) >> 5);
         lane = threadIdx.x & 31;
     }
 };
+
+// The basis vectors of chunk c of slot s, vector k at + k * L, indexed by the
+// element number q of the whole vector (c L <= q): the m + 1 pieces of a
+// chunk lie together, so that an item streams one contiguous run, and every
+// piece is whole (zero past n), so that its loads carry no bound: with a bound
+// on each, the compiler put every load of a batch in a branch of its own, and
+// the dots of 28 vectors of 62,208 unknowns for 32 slots took 240 us; they take
+// 75 (6.0 TB/s).
+template <typename C>
+__device__ __forceinline__ C *basis_of(const TickArgs<C> &a, const Chunks &ch, int s, int c) {
+    return a.V + ((size_t)s * ch.nch + c) * (a.m + 1) * ch.L - c * ch.L;
+}
 
 // Work items (slot, chunk) of a phase.  With at least two items per warp
 // they are handed out in runs of QG by an atomic counter, the slots with the
@@ -148,7 +196,7 @@ struct WorkQueue {
 // the per-lane sums v of chunk c of slot s: fold, publish, and let the
 // slot's last warp form the total
 template <int NV, typename C>
-__device__ __forceinline__ void chunk_done(const TickArgs<C> &a, int s, int c, double (&v)[NV], int parity, int lane) {
+__device__ __forceinline__ void chunk_done(const TickArgs<C> &a, int s, int c, int nch, double (&v)[NV], int parity, int lane) {
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
 #pragma unroll
@@ -156,35 +204,17 @@ __device__ __forceinline__ void chunk_done(const TickArgs<C> &a, int s, int c, d
     }
     int last = 0;
     if (lane == 0) {
-        double *p = a.cpart + ((size_t)s * NCH + c) * 4;
+        double *p = a.cpart + ((size_t)s * nch + c) * 4;
 #pragma unroll
         for (int k = 0; k < NV; ++k) p[k] = v[k];
         __threadfence();
-        last = atomicAdd(&a.ccnt[s], 1) == NCH - 1;
+        last = atomicAdd(&a.ccnt[s], 1) == nch - 1;
     }
     last = __shfl_sync(0xffffffffu, last, 0);
     if (last) {
         __threadfence();
-        // all loads first (they are independent), then the sums in chunk order
-        double pv[NCH / 32][NV];
-#pragma unroll
-        for (int j = 0; j < NCH / 32; ++j) {
-            const double *p = a.cpart + ((size_t)s * NCH + lane + 32 * j) * 4;
-#pragma unroll
-            for (int k = 0; k < NV; ++k) pv[j][k] = __ldcg(p + k);
-        }
         double t[NV];
-#pragma unroll
-        for (int k = 0; k < NV; ++k) t[k] = 0.0;
-#pragma unroll
-        for (int j = 0; j < NCH / 32; ++j)
-#pragma unroll
-            for (int k = 0; k < NV; ++k) t[k] += pv[j][k];
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
-        }
+        lane_partials<NV>(a.cpart + (size_t)s * nch * 4, 4, nch, lane, t);
         if (lane == 0) {
 #pragma unroll
             for (int k = 0; k < NV; ++k) a.ctot[((size_t)parity * NSMAX + s) * 4 + k] = t[k];
@@ -204,26 +234,26 @@ __device__ __forceinline__ void load_totals(const TickArgs<C> &a, int parity, in
 }
 
 // Givens update of the new H column, residual estimate and, when a cycle
-// ends, y = H^-1 g (back substitution) for every Arnoldi slot: CTA 0, one
-// warp per slot.  H column i-1 is complete except H(i, i-1) = shn[s];
+// ends, y = H^-1 g (back substitution) for every Arnoldi slot: one warp per
+// slot, the last of CTA s (mod the grid), while the other warps normalise the
+// new vectors.  H column i-1 is complete except H(i, i-1) = shn[s];
 // sreo[s] flags a re-orthogonalised step (counted).  The warp stages the
 // column in shared memory (hw) so that lane 0 applies the rotations in their
 // order without a global-memory round trip per step; the back substitution
 // runs column by column over the warp, lane r holding rows r and r + 32.
 template <typename C>
 __device__ void givens_step(const TickArgs<C> &a, const int *smode, const int *sstep, const double *shn, const int *sreo,
-                            cd (*hws)[SCD_M_MAX + 1]) {
+                            cd *hw) {
     const int ldh = a.m + 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    cd *hw = hws[warp];
-    for (int s = warp; s < a.ns; s += BW) {
+    const int lane = threadIdx.x & 31;
+    for (int s = blockIdx.x; s < a.ns; s += gridDim.x) {
         if (smode[s] != SLOT_ARNOLDI) continue;   // uniform across the warp
         Slot &sl = a.slots[s];
         const int i = sstep[s] + 1;
         cd *Hc = a.H + (size_t)s * ldh * a.m + (size_t)ldh * (i - 1);
         cd *cs = a.cs + (size_t)s * (a.m + 1), *sn = a.sn + (size_t)s * (a.m + 1), *g = a.g + (size_t)s * (a.m + 1);
         __syncwarp();
-        for (int k = lane; k < i; k += 32) hw[k] = Hc[k];
+        for (int k = lane; k < i; k += 32) hw[k] = make_double2(__ldcg(&Hc[k].x), __ldcg(&Hc[k].y));
         if (lane == 0) hw[i] = cmk(shn[s], 0.0);
         // the rotations so far, two per lane (k = lane, lane + 32)
         cd c0 = cmk(0, 0), s0 = cmk(0, 0), c1 = cmk(0, 0), s1 = cmk(0, 0);
@@ -321,7 +351,7 @@ __device__ void cycle_end(const TickArgs<C> &a, const Chunks &ch, int nch, const
             for (int cc = lane; cc < kd; cc += 32) yw[cc] = make_double2(__ldcg(&ys[cc].x), __ldcg(&ys[cc].y));
             __syncwarp();
             const long long qa = c * ch.L, qb = min(n, qa + ch.L);
-            const C *Vs = a.V + (size_t)s * (a.m + 1) * n;
+            const C *Vs = basis_of(a, ch, s, c);
             C *xs = a.x + (size_t)s * n;
             for (long long q = qa + lane; q < qb; q += 32 * TUC) {
                 cd acc[TUC];
@@ -329,7 +359,7 @@ __device__ void cycle_end(const TickArgs<C> &a, const Chunks &ch, int nch, const
                 for (int e = 0; e < TUC; ++e) acc[e] = cmk(0, 0);
                 for (int cc = 0; cc < kd; ++cc) {
                     const cd yc = yw[cc];
-                    const C *vc = Vs + (size_t)cc * n;
+                    const C *vc = Vs + cc * ch.L;
 #pragma unroll
                     for (int e = 0; e < TUC; ++e) {
                         const long long qq = q + 32 * e;
@@ -359,63 +389,190 @@ __device__ void cycle_end(const TickArgs<C> &a, const Chunks &ch, int nch, const
     }
 }
 
-// Classical Gram-Schmidt, first pass, chunk c of slot s: the dots <v_k, w>,
-// k = 1..i, and ||w||^2 in one sweep over the chunk (w is re-read from cache
-// for each k), published per chunk; the slot's last warp sums the NCH chunk
-// partials of every value in chunk order into ctm.
-template <typename C, int TUC>
-__device__ __forceinline__ void cgs_dots(const TickArgs<C> &a, int s, int c, int i, const C *Vs, const C *ws,
-                                         long long qa, long long qb, int lane) {
-    const long long n = a.n;
-    double *pp = a.cpm + ((size_t)s * NCH + c) * CGS_NV;
+// 16 bytes of a basis vector from element q, a multiple of VW.  A chunk's
+// pieces are whole (L elements, zero past n), so no load needs a bound.
+template <typename C> constexpr int VW = 16 / (int)sizeof(C);
+__device__ __forceinline__ float4 ld_vec(const cf *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ double2 ld_vec(const cd *p) { return *p; }
+__device__ __forceinline__ cd vec_el(float4 v, int h) { return h ? cmk((double)v.z, (double)v.w) : cmk((double)v.x, (double)v.y); }
+__device__ __forceinline__ cd vec_el(double2 v, int) { return v; }
+
+// Classical Gram-Schmidt works on a chunk CE 16-byte units per lane and CK
+// basis vectors at a time: CE * CK independent 16-byte loads in flight, w (or
+// the updated element) in registers across the vectors of a chunk.
+constexpr int CE = 4, CK = 2;
+
+// First pass, chunk c of slot s: the dots <v_k, w>, k = 1..i, and ||w||^2,
+// each lane's elements in order, the lanes' sums folded pairwise (four values
+// over 32 lanes in six exchanges) and published per chunk; cgs_totals adds
+// the chunks.
+template <typename C>
+__device__ __forceinline__ void cgs_dots(const TickArgs<C> &a, const Chunks &ch, int s, int c, int i, const C *Vs,
+                                         const C *ws, long long qa, long long qb) {
+    constexpr int W = VW<C>, EL = CE * W;
+    const int lane = ch.lane, nch = ch.nch;
+    double *pp = a.cpm + (size_t)s * CGS_NV * nch + c;
     double nw = 0.0;
-    for (int k = 1; k <= i; ++k) {
-        const C *vk = Vs + (size_t)(k - 1) * n;
-        double d[2] = {0.0, 0.0};
-        for (long long q = qa + lane; q < qb; q += 32 * TUC) {
-            C w[TUC], z[TUC];
+    const long long qe = qa + ch.L;
+    const bool once = ch.L <= 32 * EL;
+    cd w[EL];
+    for (int k0 = 0; k0 < i; k0 += CK) {
+        double d[2 * CK];
 #pragma unroll
-            for (int e = 0; e < TUC; ++e) {
-                const long long qq = q + 32 * e;
-                w[e] = z[e] = C{};
-                if (qq < qb) { w[e] = ws[qq]; z[e] = vk[qq]; }
+        for (int h = 0; h < 2 * CK; ++h) d[h] = 0.0;
+        for (long long q = qa + lane * W; q < qe; q += 32 * EL) {
+            decltype(ld_vec(Vs)) z[CK][CE];
+#pragma unroll
+            for (int k = 0; k < CK; ++k)
+#pragma unroll
+                for (int e = 0; e < CE; ++e) z[k][e] = ld_vec(Vs + min(k0 + k, i - 1) * ch.L + q + 32 * W * e);
+            if (!once || k0 == 0) {
+#pragma unroll
+                for (int e = 0; e < CE; ++e)
+#pragma unroll
+                    for (int h = 0; h < W; ++h) {
+                        const long long qq = q + 32 * W * e + h;
+                        w[e * W + h] = qq < qb ? to_cd(ws[qq]) : cmk(0, 0);
+                    }
             }
 #pragma unroll
-            for (int e = 0; e < TUC; ++e) {
-                if (q + 32 * e >= qb) break;
-                const cd wv = to_cd(w[e]);
-                cdot_acc(d[0], d[1], to_cd(z[e]), wv);
-                if (k == 1) nw += cabs2(wv);
-            }
+            for (int e = 0; e < CE; ++e)
+#pragma unroll
+                for (int h = 0; h < W; ++h) {
+                    const cd wv = w[e * W + h];
+#pragma unroll
+                    for (int k = 0; k < CK; ++k) cdot_acc(d[2 * k], d[2 * k + 1], vec_el(z[k][e], h), wv);
+                    if (k0 == 0) nw += cabs2(wv);
+                }
         }
+        // fold: lanes 8v .. 8v+7 end with value v
+        static_assert(CK == 2, "four values");
+        const bool b4 = lane & 16, b3 = lane & 8;
+        double e0 = b4 ? d[2] : d[0], e1 = b4 ? d[3] : d[1];
+        e0 += __shfl_xor_sync(0xffffffffu, b4 ? d[0] : d[2], 16);
+        e1 += __shfl_xor_sync(0xffffffffu, b4 ? d[1] : d[3], 16);
+        double f = b3 ? e1 : e0;
+        f += __shfl_xor_sync(0xffffffffu, b3 ? e0 : e1, 8);
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) d[h] += __shfl_xor_sync(0xffffffffu, d[h], o);
-        if (lane == 0) { pp[2 * (k - 1)] = d[0]; pp[2 * (k - 1) + 1] = d[1]; }
+        for (int o = 4; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+        if ((lane & 7) == 0 && 2 * k0 + (lane >> 3) < 2 * i) pp[(size_t)(2 * k0 + (lane >> 3)) * nch] = f;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) nw += __shfl_xor_sync(0xffffffffu, nw, o);
-    int last = 0;
-    if (lane == 0) {
-        pp[CGS_NV - 1] = nw;
-        __threadfence();
-        last = atomicAdd(&a.ccnt[s], 1) == NCH - 1;
+    if (lane == 0) pp[(size_t)(CGS_NV - 1) * nch] = nw;
+}
+
+// the dots' chunk partials added in chunk order, one warp per (slot, value)
+template <typename C>
+__device__ __forceinline__ void cgs_totals(const TickArgs<C> &a, const Chunks &ch, const int *smode, const int *sstep, int imax) {
+    const int nval = 2 * imax + 1;
+    for (int it = ch.gw; it < a.ns * nval; it += ch.nw) {
+        const int s = it / nval, k = it - s * nval, v = k == 2 * imax ? CGS_NV - 1 : k;
+        if (smode[s] != SLOT_ARNOLDI || (v < CGS_NV - 1 && v >= 2 * (sstep[s] + 1))) continue;
+        double t[1];
+        lane_partials<1>(a.cpm + ((size_t)s * CGS_NV + v) * ch.nch, 1, ch.nch, ch.lane, t);
+        if (ch.lane == 0) a.ctm[(size_t)s * CGS_NV + v] = t[0];
     }
-    last = __shfl_sync(0xffffffffu, last, 0);
-    if (!last) return;
-    __threadfence();
-    double *tt = a.ctm + (size_t)s * CGS_NV;
-    for (int v = 0; v < CGS_NV; ++v) {
-        if (v >= 2 * i && v != CGS_NV - 1) continue;
-        double t = 0.0;
+}
+
+// Modified Gram-Schmidt with w resident in shared memory, for solves whose
+// (slot, chunk) items are at most RES per warp: each warp keeps its items
+// for the whole orthogonalisation, publishes a chunk partial per term, and
+// after the barrier adds its own slot's partials itself, so that a term costs
+// one barrier and one read of the partials instead of a round through the
+// slot's last warp.  The next basis vector is read before the barrier.  The
+// sums run in the order of the streaming variant below it (the same bits).
+// The complex64 form, whose default is classical, has no registers to spare
+// for it.
+template <typename C> constexpr int RES = sizeof(C) == 16 ? 3 : 0;   // items per warp at most
+template <typename C>
+__device__ void mgs_first(const TickArgs<C> &a, const Chunks &ch, const int *smode, const int *swpos, C *wsh, C (&z)[CHUNK / 32]) {
+    const int lane = ch.lane;
+    for (int j = 0; j < a.res; ++j) {
+        const int it = ch.gw + j * ch.nw;
+        if (it >= a.ns * ch.nch) break;
+        const int s = it / ch.nch, c = it - s * ch.nch;
+        if (smode[s] != SLOT_ARNOLDI) continue;
+        const long long qa = c * ch.L, qb = min(a.n, qa + ch.L);
+        const C *ws = a.w + (size_t)swpos[s] * a.n, *v0 = basis_of(a, ch, s, c);
+        C *wj = wsh + j * CHUNK, w[CHUNK / 32], p[CHUNK / 32];
 #pragma unroll
-        for (int j = 0; j < NCH / 32; ++j) t += __ldcg(a.cpm + ((size_t)s * NCH + lane + 32 * j) * CGS_NV + v);
+        for (int e = 0; e < CHUNK / 32; ++e) {
+            const long long q = qa + lane + 32 * e;
+            w[e] = p[e] = C{};
+            if (q < qb) { w[e] = ws[q]; p[e] = v0[q]; }
+        }
+        double v[3] = {0, 0, 0};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (lane == 0) tt[v] = t;
+        for (int e = 0; e < CHUNK / 32; ++e) {
+            wj[lane + 32 * e] = w[e];
+            if (j == 0) z[e] = p[e];
+            if (qa + lane + 32 * e >= qb) continue;
+            const cd wv = to_cd(w[e]);
+            v[0] += cabs2(wv);
+            cdot_acc(v[1], v[2], to_cd(p[e]), wv);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+        if (lane == 0) {
+            a.rnorm[(size_t)s * ch.nch + c] = v[0];
+            *reinterpret_cast<double2 *>(a.cpart + ((size_t)s * ch.nch + c) * 4) = cmk(v[1], v[2]);
+        }
     }
-    if (lane == 0) a.ccnt[s] = 0;
+}
+// term k (1-based): partials of term k - 1 lie in pair (k - 1) & 1 of cpart
+template <typename C>
+__device__ void mgs_term(const TickArgs<C> &a, const Chunks &ch, int k, const int *smode, const int *sstep, const int *swpos,
+                         C *wsh, C (&z)[CHUNK / 32]) {
+    const int lane = ch.lane, ldh = a.m + 1;
+    for (int j = 0; j < a.res; ++j) {
+        const int it = ch.gw + j * ch.nw;
+        if (it >= a.ns * ch.nch) break;
+        const int s = it / ch.nch, c = it - s * ch.nch;
+        const int i = sstep[s] + 1;
+        if (smode[s] != SLOT_ARNOLDI || k > i) continue;
+        const long long qa = c * ch.L, qb = min(a.n, qa + ch.L);
+        const C *vk = basis_of(a, ch, s, c) + (k - 1) * ch.L, *vn = vk + ch.L;
+        C *wj = wsh + j * CHUNK, zk[CHUNK / 32], zn[CHUNK / 32];
+        const bool more = k < i;
+#pragma unroll
+        for (int e = 0; e < CHUNK / 32; ++e) {
+            const long long q = qa + lane + 32 * e;
+            zk[e] = j == 0 ? z[e] : q < qb ? vk[q] : C{};
+            zn[e] = more && q < qb ? vn[q] : C{};
+        }
+        double t[2];
+        lane_partials<2>(a.cpart + (size_t)s * ch.nch * 4 + 2 * ((k - 1) & 1), 4, ch.nch, lane, t);
+        const cd h = cmk(t[0], t[1]);
+        if (c == 0 && lane == 0) a.H[(size_t)s * ldh * a.m + (size_t)ldh * (i - 1) + (k - 1)] = h;
+        double u[2] = {0, 0};
+        C *ws = a.w + (size_t)swpos[s] * a.n;
+#pragma unroll
+        for (int e = 0; e < CHUNK / 32; ++e) {
+            const long long q = qa + lane + 32 * e;
+            if (q >= qb) continue;
+            cd wv = to_cd(wj[lane + 32 * e]);
+            csub_mul(wv, h, to_cd(zk[e]));
+            store_c(wj[lane + 32 * e], wv);
+            const cd wr = rounded<C>(wv);
+            if (more) {
+                cdot_acc(u[0], u[1], to_cd(zn[e]), wr);
+            } else {
+                u[0] += cabs2(wr);
+                store_c(ws[q], wv);
+            }
+        }
+#pragma unroll
+        for (int h2 = 0; h2 < 2; ++h2)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) u[h2] += __shfl_xor_sync(0xffffffffu, u[h2], o);
+        if (lane == 0) *reinterpret_cast<double2 *>(a.cpart + ((size_t)s * ch.nch + c) * 4 + 2 * (k & 1)) = cmk(u[0], u[1]);
+        if (j == 0)
+#pragma unroll
+            for (int e = 0; e < CHUNK / 32; ++e) z[e] = zn[e];
+    }
 }
 
 // One tick: cycle starts (r = rhs - A x, V0 = r/||r||) and Arnoldi steps
@@ -430,9 +587,10 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
     const long long n = a.n;
     constexpr int TUC = sizeof(C) == 8 ? 2 * TU : TU;   // complex64: twice the elements in flight
     const int ldh = a.m + 1;
-    const Chunks ch(n, NCH);
+    const Chunks ch(n);
+    const int nch = ch.nch;
     const int lane = ch.lane;
-    const int nitems = a.ns * NCH;
+    const int nitems = a.ns * nch;
     for (int s = threadIdx.x; s < a.ns; s += blockDim.x) {
         smode[s] = a.slots[s].mode;
         sstep[s] = a.slots[s].step;
@@ -441,32 +599,44 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
     }
     __syncthreads();
     // slots by cost (Krylov vectors a step reads), largest first, ties by index
-    __shared__ int sorder[NSMAX];
-    if (threadIdx.x == 0) {
-        auto cost = [&](int s) { return smode[s] == SLOT_ARNOLDI ? sstep[s] + 2 : smode[s] == SLOT_START ? 1 : 0; };
-        for (int s = 0; s < a.ns; ++s) {
-            const int cs = cost(s);
-            int j = s - 1;
-            while (j >= 0 && cost(sorder[j]) < cs) { sorder[j + 1] = sorder[j]; --j; }
-            sorder[j + 1] = s;
-        }
+    __shared__ int sorder[NSMAX], scost[NSMAX], simax;
+    if (threadIdx.x == 0) simax = 0;
+    if (threadIdx.x < a.ns) {
+        const int md = smode[threadIdx.x];
+        scost[threadIdx.x] = md == SLOT_ARNOLDI ? sstep[threadIdx.x] + 2 : md == SLOT_START ? 1 : 0;
     }
     __syncthreads();
+    if (threadIdx.x < a.ns) {
+        const int me = threadIdx.x, mine = scost[me];
+        int rank = 0;
+        for (int s = 0; s < a.ns; ++s) rank += scost[s] > mine || (scost[s] == mine && s < me);
+        sorder[rank] = me;
+        if (mine >= 2) atomicMax(&simax, mine - 1);   // steps of the longest Arnoldi slot
+    }
+    const bool any_start = __syncthreads_or(threadIdx.x < a.ns && smode[min((int)threadIdx.x, NSMAX - 1)] == SLOT_START);
+    const int imax = simax, kmax = a.cgs ? 0 : imax;
+    const bool resident = RES<C> > 0 && a.res > 0 && kmax > 0;
+    extern __shared__ __align__(16) unsigned char tick_dyn[];
+    C *const wsh = reinterpret_cast<C *>(tick_dyn) + (size_t)(threadIdx.x >> 5) * a.res * CHUNK;
+    C zres[CHUNK / 32];
     int ph = 0;        // phases so far: each takes the next work-queue counter
     int parity = 0;
     // ---- phase A: first reduction of every active slot
-    for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-        const int s = sorder[q.it / NCH], c = q.it % NCH;
+    if constexpr (RES<C> > 0)
+        if (resident) mgs_first<C>(a, ch, smode, swpos, wsh, zres);
+    for (WorkQueue q(a.qctr + ph++, resident && !any_start ? 0 : nitems, ch); q.next();) {
+        const int s = sorder[q.it / nch], c = q.it % nch;
         const int md = smode[s];
-        if (md != SLOT_START && md != SLOT_ARNOLDI) continue;
+        if (md != SLOT_START && (md != SLOT_ARNOLDI || resident)) continue;
         const long long qa = c * ch.L, qb = min(n, qa + ch.L);
         double v[3] = {0, 0, 0};
         const C *ws = a.w + (size_t)swpos[s] * n;
-        C *V0 = a.V + (size_t)s * (a.m + 1) * n;
+        C *V0 = basis_of(a, ch, s, c);
         if (md == SLOT_START) {
             const C *bs = a.rhs + (size_t)s * n;
             const bool zx = szero[s] != 0;
-            for (long long q = qa + lane; q < qb; q += 32 * TUC) {
+            const long long qe = qa + ch.L;
+            for (long long q = qa + lane; q < qe; q += 32 * TUC) {
                 cd b[TUC], w[TUC];
 #pragma unroll
                 for (int u = 0; u < TUC; ++u) {
@@ -480,15 +650,15 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
 #pragma unroll
                 for (int u = 0; u < TUC; ++u) {
                     const long long qq = q + 32 * u;
-                    if (qq >= qb) break;
-                    const cd r = zx ? b[u] : csub(b[u], w[u]);
+                    if (qq >= qe) break;
+                    const cd r = zx ? b[u] : csub(b[u], w[u]);   // zero past n
                     store_c(V0[qq], r);
                     v[0] += cabs2(r);
                     v[1] += cabs2(b[u]);
                 }
             }
         } else if (a.cgs) {
-            cgs_dots<C, TUC>(a, s, c, sstep[s] + 1, V0, ws, qa, qb, lane);
+            cgs_dots<C>(a, ch, s, c, sstep[s] + 1, V0, ws, qa, qb);
             continue;
         } else {
             for (long long q = qa + lane; q < qb; q += 32 * TUC) {
@@ -507,32 +677,31 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
                 }
             }
         }
-        chunk_done<3>(a, s, c, v, parity, lane);
+        chunk_done<3>(a, s, c, nch, v, parity, lane);
     }
     for (int s = threadIdx.x; s < a.ns; s += blockDim.x)
-        sact[s] = smode[s] == SLOT_START || (smode[s] == SLOT_ARNOLDI && !a.cgs);
+        sact[s] = smode[s] == SLOT_START || (smode[s] == SLOT_ARNOLDI && !a.cgs && !resident);
     grid_barrier(a.bar, gridDim.x, a.err);
     load_totals(a, parity, 3, sact, tot);
-    int kmax = 0;
-    for (int s = 0; s < a.ns; ++s) {
-        if (smode[s] == SLOT_ARNOLDI && !a.cgs) kmax = max(kmax, sstep[s] + 1);
-        if (threadIdx.x == 0) {
-            if (smode[s] == SLOT_ARNOLDI && a.cgs) {
-                snormav[s] = sqrt(__ldcg(a.ctm + (size_t)s * CGS_NV + CGS_NV - 1));
-            } else {
-                snormav[s] = sqrt(tot[s][0]);
-                sh_h[s] = cmk(tot[s][1], tot[s][2]);
-            }
-        }
+    if (threadIdx.x < a.ns && sact[threadIdx.x]) {
+        const int s = threadIdx.x;
+        snormav[s] = sqrt(tot[s][0]);
+        sh_h[s] = cmk(tot[s][1], tot[s][2]);
+    }
+    if (a.cgs && imax > 0) {
+        cgs_totals<C>(a, ch, smode, sstep, imax);
+        grid_barrier(a.bar, gridDim.x, a.err);
+        if (threadIdx.x < a.ns && smode[threadIdx.x] == SLOT_ARNOLDI)
+            snormav[threadIdx.x] = sqrt(__ldcg(a.ctm + (size_t)threadIdx.x * CGS_NV + CGS_NV - 1));
     }
     __syncthreads();
     // cycle starts: normalise V0, set g, b_norm
-    for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-        const int s = sorder[q.it / NCH], c = q.it % NCH;
+    for (WorkQueue q(a.qctr + ph++, any_start ? nitems : 0, ch); q.next();) {
+        const int s = sorder[q.it / nch], c = q.it % nch;
         if (smode[s] != SLOT_START) continue;
         const double beta = sqrt(tot[s][0]);
         const long long qa = c * ch.L, qb = min(n, qa + ch.L);
-        C *V0 = a.V + (size_t)s * (a.m + 1) * n;
+        C *V0 = basis_of(a, ch, s, c);
         for (long long q = qa + lane; q < qb; q += 32 * TUC) {
             cd r[TUC];
 #pragma unroll
@@ -565,9 +734,24 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
         }
     }
     // ---- MGS for the Arnoldi slots: one barrier per term
-    for (int k = 1; k <= kmax; ++k) {
+    if (resident) {
+        for (int k = 1; k <= kmax; ++k) {
+            if constexpr (RES<C> > 0) mgs_term<C>(a, ch, k, smode, sstep, swpos, wsh, zres);
+            grid_barrier(a.bar, gridDim.x, a.err);
+        }
+        // every CTA: ||w|| before and after of every Arnoldi slot
+        for (int s = threadIdx.x >> 5; s < a.ns; s += BW) {
+            if (smode[s] != SLOT_ARNOLDI) continue;
+            double t[1], h[1];
+            lane_partials<1>(a.rnorm + (size_t)s * nch, 1, nch, lane, t);
+            lane_partials<1>(a.cpart + (size_t)s * nch * 4 + 2 * ((sstep[s] + 1) & 1), 4, nch, lane, h);
+            if (lane == 0) { snormav[s] = sqrt(t[0]); shn[s] = sqrt(h[0]); }
+        }
+        __syncthreads();
+    }
+    for (int k = 1; k <= (resident ? 0 : kmax); ++k) {
         for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-            const int s = sorder[q.it / NCH], c = q.it % NCH;
+            const int s = sorder[q.it / nch], c = q.it % nch;
             if (smode[s] != SLOT_ARNOLDI) continue;
             const int i = sstep[s] + 1;
             if (k > i) continue;
@@ -575,9 +759,9 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
             if (c == 0 && lane == 0) a.H[(size_t)s * ldh * a.m + (size_t)ldh * (i - 1) + (k - 1)] = h;
             const long long qa = c * ch.L, qb = min(n, qa + ch.L);
             C *ws = a.w + (size_t)swpos[s] * n;
-            const C *Vs = a.V + (size_t)s * (a.m + 1) * n;
-            const C *vk = Vs + (size_t)(k - 1) * n;
-            const C *vn = (k < i) ? Vs + (size_t)k * n : nullptr;
+            const C *Vs = basis_of(a, ch, s, c);
+            const C *vk = Vs + (k - 1) * ch.L;
+            const C *vn = (k < i) ? Vs + k * ch.L : nullptr;
             double u[2] = {0, 0};
             for (long long q = qa + lane; q < qb; q += 32 * TUC) {
                 C w[TUC], p[TUC], z[TUC];      // raw elements, widened at use
@@ -603,7 +787,7 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
                     else u[0] += cabs2(wr);
                 }
             }
-            chunk_done<2>(a, s, c, u, parity ^ 1, lane);
+            chunk_done<2>(a, s, c, nch, u, parity ^ 1, lane);
         }
         for (int s = threadIdx.x; s < a.ns; s += blockDim.x) sact[s] = smode[s] == SLOT_ARNOLDI && k <= sstep[s] + 1;
         parity ^= 1;
@@ -620,51 +804,55 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
     }
     // ---- classical Gram-Schmidt update: w -= sum_k h_k v_k (k ascending,
     // FP64 per element, one rounding to the storage precision), ||w||^2
-    if (a.cgs) {
+    if (a.cgs && imax > 0) {
         cd *hs = ysm[threadIdx.x >> 5];
         for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-            const int s = sorder[q.it / NCH], c = q.it % NCH;
+            const int s = sorder[q.it / nch], c = q.it % nch;
             if (smode[s] != SLOT_ARNOLDI) continue;
             const int i = sstep[s] + 1;
             const double *tt = a.ctm + (size_t)s * CGS_NV;
             __syncwarp();   // every lane is done with the previous item's coefficients
             for (int k = lane; k < i; k += 32) hs[k] = cmk(__ldcg(tt + 2 * k), __ldcg(tt + 2 * k + 1));
             __syncwarp();
-            if (c == 0 && lane == 0)
-                for (int k = 0; k < i; ++k) a.H[(size_t)s * ldh * a.m + (size_t)ldh * (i - 1) + k] = hs[k];
+            if (c == 0)
+                for (int k = lane; k < i; k += 32) a.H[(size_t)s * ldh * a.m + (size_t)ldh * (i - 1) + k] = hs[k];
             const long long qa = c * ch.L, qb = min(n, qa + ch.L);
             C *ws = a.w + (size_t)swpos[s] * n;
-            const C *Vs = a.V + (size_t)s * (a.m + 1) * n;
+            const C *Vs = basis_of(a, ch, s, c);
+            constexpr int W = VW<C>, EL = CE * W;
             double u[1] = {0.0};
-            for (long long q = qa + lane; q < qb; q += 32 * TUC) {
-                cd acc[TUC];
+            for (long long q = qa + lane * W; q < qa + ch.L; q += 32 * EL) {
+                cd acc[EL];
 #pragma unroll
-                for (int e = 0; e < TUC; ++e) {
-                    const long long qq = q + 32 * e;
+                for (int e = 0; e < EL; ++e) {
+                    const long long qq = q + 32 * W * (e / W) + e % W;
                     acc[e] = qq < qb ? to_cd(ws[qq]) : cmk(0, 0);
                 }
-                for (int k = 0; k < i; ++k) {
-                    const cd hk = hs[k];
-                    const C *vk = Vs + (size_t)k * n;
-                    C p[TUC];
+                for (int k0 = 0; k0 < i; k0 += CK) {
+                    decltype(ld_vec(Vs)) p[CK][CE];
 #pragma unroll
-                    for (int e = 0; e < TUC; ++e) {
-                        const long long qq = q + 32 * e;
-                        p[e] = qq < qb ? vk[qq] : C{};
+                    for (int k = 0; k < CK; ++k)
+#pragma unroll
+                        for (int e = 0; e < CE; ++e)
+                            p[k][e] = ld_vec(Vs + min(k0 + k, i - 1) * ch.L + q + 32 * W * e);
+#pragma unroll
+                    for (int k = 0; k < CK; ++k) {
+                        if (k0 + k >= i) break;
+                        const cd hk = hs[k0 + k];
+#pragma unroll
+                        for (int e = 0; e < EL; ++e) csub_mul(acc[e], hk, vec_el(p[k][e / W], e % W));
                     }
-#pragma unroll
-                    for (int e = 0; e < TUC; ++e) csub_mul(acc[e], hk, to_cd(p[e]));
                 }
 #pragma unroll
-                for (int e = 0; e < TUC; ++e) {
-                    const long long qq = q + 32 * e;
-                    if (qq >= qb) break;
+                for (int e = 0; e < EL; ++e) {
+                    const long long qq = q + 32 * W * (e / W) + e % W;
+                    if (qq >= qb) continue;
                     store_c(ws[qq], acc[e]);
                     u[0] += cabs2(rounded<C>(acc[e]));
                 }
             }
             __syncwarp();
-            chunk_done<1>(a, s, c, u, parity ^ 1, lane);
+            chunk_done<1>(a, s, c, nch, u, parity ^ 1, lane);
         }
         for (int s = threadIdx.x; s < a.ns; s += blockDim.x) sact[s] = smode[s] == SLOT_ARNOLDI;
         parity ^= 1;
@@ -676,16 +864,16 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
     // ---- conditional re-orthogonalisation (src/gmres_module.f90:251-258)
     for (int s = threadIdx.x; s < a.ns; s += blockDim.x)
         sro[s] = smode[s] == SLOT_ARNOLDI && snormav[s] + (double)0.001f * shn[s] == snormav[s];
-    __syncthreads();
     int jmax = 0;
-    for (int s = 0; s < a.ns; ++s)
-        if (sro[s]) jmax = max(jmax, sstep[s] + 1);
+    if (__syncthreads_or(threadIdx.x < a.ns && sro[min((int)threadIdx.x, NSMAX - 1)]))
+        for (int s = 0; s < a.ns; ++s)
+            if (sro[s]) jmax = max(jmax, sstep[s] + 1);
     for (int j = 1; j <= jmax; ++j) {
         for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-            const int s = sorder[q.it / NCH], c = q.it % NCH;
+            const int s = sorder[q.it / nch], c = q.it % nch;
             if (!sro[s] || j > sstep[s] + 1) continue;
             const long long qa = c * ch.L, qb = min(n, qa + ch.L);
-            const C *vj = a.V + (size_t)s * (a.m + 1) * n + (size_t)(j - 1) * n;
+            const C *vj = basis_of(a, ch, s, c) + (j - 1) * ch.L;
             const C *ws = a.w + (size_t)swpos[s] * n;
             double u[2] = {0, 0};
             for (long long q = qa + lane; q < qb; q += 32 * TUC) {
@@ -702,7 +890,7 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
                     cdot_acc(u[0], u[1], z[e], w[e]);
                 }
             }
-            chunk_done<2>(a, s, c, u, parity ^ 1, lane);
+            chunk_done<2>(a, s, c, nch, u, parity ^ 1, lane);
         }
         for (int s = threadIdx.x; s < a.ns; s += blockDim.x) sact[s] = sro[s] && j <= sstep[s] + 1;
         parity ^= 1;
@@ -717,11 +905,11 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
             }
         }
         for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-            const int s = sorder[q.it / NCH], c = q.it % NCH;
+            const int s = sorder[q.it / nch], c = q.it % nch;
             if (!sact[s]) continue;
             const cd hr = cmk(tot[s][0], tot[s][1]);
             const long long qa = c * ch.L, qb = min(n, qa + ch.L);
-            const C *vj = a.V + (size_t)s * (a.m + 1) * n + (size_t)(j - 1) * n;
+            const C *vj = basis_of(a, ch, s, c) + (j - 1) * ch.L;
             C *ws = a.w + (size_t)swpos[s] * n;
             for (long long q = qa + lane; q < qb; q += 32 * TUC) {
                 cd w[TUC], p[TUC];
@@ -744,7 +932,7 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
     }
     if (jmax > 0) {
         for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-            const int s = sorder[q.it / NCH], c = q.it % NCH;
+            const int s = sorder[q.it / nch], c = q.it % nch;
             if (!sro[s]) continue;
             const long long qa = c * ch.L, qb = min(n, qa + ch.L);
             const C *ws = a.w + (size_t)swpos[s] * n;
@@ -762,7 +950,7 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
                     u[0] += cabs2(w[e]);
                 }
             }
-            chunk_done<1>(a, s, c, u, parity ^ 1, lane);
+            chunk_done<1>(a, s, c, nch, u, parity ^ 1, lane);
         }
         parity ^= 1;
         grid_barrier(a.bar, gridDim.x, a.err);
@@ -771,15 +959,20 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
         __syncthreads();
     }
     // ---- v_i = w / h(i+1,i) and the Givens update
+    if (imax == 0) return;   // no Arnoldi slot: no column to finish either
+    if (threadIdx.x < a.ns)
+        sact[threadIdx.x] = snormav[threadIdx.x] + (double)0.001f * shn[threadIdx.x] == snormav[threadIdx.x];
+    __syncthreads();
+    if ((threadIdx.x >> 5) == BW - 1) givens_step(a, smode, sstep, shn, sact, ysm[BW - 1]);
     for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-        const int s = sorder[q.it / NCH], c = q.it % NCH;
+        const int s = sorder[q.it / nch], c = q.it % nch;
         if (smode[s] != SLOT_ARNOLDI) continue;
         const int i = sstep[s] + 1;
         const double hn = shn[s];
         const long long qa = c * ch.L, qb = min(n, qa + ch.L);
         const C *ws = a.w + (size_t)swpos[s] * n;
-        C *vi = a.V + (size_t)s * (a.m + 1) * n + (size_t)i * n;
-        for (long long q = qa + lane; q < qb; q += 32 * TUC) {
+        C *vi = basis_of(a, ch, s, c) + i * ch.L;
+        for (long long q = qa + lane; q < qa + ch.L; q += 32 * TUC) {
             cd w[TUC];
 #pragma unroll
             for (int e = 0; e < TUC; ++e) {
@@ -789,17 +982,14 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
 #pragma unroll
             for (int e = 0; e < TUC; ++e) {
                 const long long qq = q + 32 * e;
-                if (qq < qb) store_c(vi[qq], (hn != 0.0) ? cmk(w[e].x / hn, w[e].y / hn) : w[e]);
+                if (qq < qa + ch.L) store_c(vi[qq], (hn != 0.0) ? cmk(w[e].x / hn, w[e].y / hn) : w[e]);
             }
         }
     }
-    if (blockIdx.x == 0) {
-        if (threadIdx.x < a.ns) sact[threadIdx.x] = snormav[threadIdx.x] + (double)0.001f * shn[threadIdx.x] == snormav[threadIdx.x];
-        __syncthreads();
-        givens_step(a, smode, sstep, shn, sact, ysm);
-    }
     grid_barrier(a.bar, gridDim.x, a.err);
-    cycle_end(a, ch, NCH, smode, ysm, sorder, a.qctr + ph);
+    if (__syncthreads_or(threadIdx.x < a.ns && smode[min((int)threadIdx.x, NSMAX - 1)] == SLOT_ARNOLDI &&
+                         __ldcg(&a.slots[min((int)threadIdx.x, a.ns - 1)].finish)))
+        cycle_end(a, ch, nch, smode, ysm, sorder, a.qctr + ph);
 }
 
 // matvec input per slot, compacted: x at a cycle start, v_step during
@@ -809,10 +999,14 @@ __global__ void k_stage(const Slot *slots, int ns, const C *V, const C *x, C *Xi
     const int s = blockIdx.y;
     const int md = slots[s].mode, pos = slots[s].mpos;
     if (pos < 0) return;
-    const C *src = md == SLOT_START ? x + (size_t)s * n : V + ((size_t)s * (m + 1) + slots[s].step) * n;
+    const long long L = Chunks::length(n);
+    const int nch = Chunks::count(n), step = slots[s].step;
     C *dst = Xin + (size_t)pos * n;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x)
-        dst[q] = src[q];
+    for (int c = blockIdx.x; c < nch; c += gridDim.x) {
+        const long long qa = c * L, len = min(L, n - qa);
+        const C *src = md == SLOT_START ? x + (size_t)s * n + qa : V + (((size_t)s * nch + c) * (m + 1) + step) * L;
+        for (long long q = threadIdx.x; q < len; q += blockDim.x) dst[qa + q] = src[q];
+    }
 }
 
 // ---- mixed form: the FP64 outer refinement
@@ -946,7 +1140,7 @@ struct BatchBuffers {
     Slot *slots = nullptr;
     Slot *h_slots = nullptr;
     double *red = nullptr;
-    double *cpart = nullptr, *ctot = nullptr;
+    double *cpart = nullptr, *ctot = nullptr, *rnorm = nullptr;
     double *cpm = nullptr, *ctm = nullptr;   // classical Gram-Schmidt reductions (opt-in)
     int *ccnt = nullptr;
     int grid = 0;                        // CTAs of the cooperative FP64 tick and residual kernels
@@ -955,7 +1149,7 @@ struct BatchBuffers {
 
 static void free_bb(BatchBuffers &b) {
     void *p[] = {b.V, b.H, b.cs, b.sn, b.g, b.y, b.x, b.rhs, b.Xin, b.W, b.x64, b.b64, b.Xin64, b.W64,
-                 b.slots, b.red, b.cpart, b.ctot, b.ccnt, b.cpm, b.ctm};
+                 b.slots, b.red, b.cpart, b.ctot, b.ccnt, b.cpm, b.ctm, b.rnorm};
     for (void *q : p) if (q) cudaFree(q);
     if (b.h_slots) cudaFreeHost(b.h_slots);
     b = BatchBuffers();
@@ -973,13 +1167,14 @@ int batch_prepare(scd_ctx *c, int ns, int m, int mixed, BatchBuffers &b) {
         return SCD_OK;
     free_bb(b);
     const long long n = c->n;
+    const int nch = Chunks::count(n);
     const size_t es = mixed ? sizeof(cf) : sizeof(cd);
     auto al = [&](void **p, size_t bytes, const char *what) -> int {
         if (cudaMalloc(p, bytes) != cudaSuccess) { cudaGetLastError(); return set_error(c, SCD_OOM, "batch %s (%zu bytes)", what, bytes); }
         return SCD_OK;
     };
     int rc;
-    if ((rc = al(&b.V, es * (size_t)ns * (m + 1) * n, "Krylov bases"))) return rc;
+    if ((rc = al(&b.V, es * (size_t)ns * (m + 1) * nch * Chunks::length(n), "Krylov bases"))) return rc;
     if ((rc = al((void **)&b.H, sizeof(cd) * (size_t)ns * (m + 1) * m, "H"))) return rc;
     if ((rc = al((void **)&b.cs, sizeof(cd) * (size_t)ns * (m + 1), "cs"))) return rc;
     if ((rc = al((void **)&b.sn, sizeof(cd) * (size_t)ns * (m + 1), "sn"))) return rc;
@@ -996,29 +1191,34 @@ int batch_prepare(scd_ctx *c, int ns, int m, int mixed, BatchBuffers &b) {
         if ((rc = al((void **)&b.W64, sizeof(cd) * (size_t)ns * n, "W64"))) return rc;
     }
     if ((rc = al((void **)&b.slots, sizeof(Slot) * ns, "slots"))) return rc;
-    if ((rc = al((void **)&b.cpart, sizeof(double) * (size_t)NSMAX * NCH * 4, "chunk partials"))) return rc;
+    if ((rc = al((void **)&b.cpart, sizeof(double) * (size_t)ns * nch * 4, "chunk partials"))) return rc;
+    if ((rc = al((void **)&b.rnorm, sizeof(double) * (size_t)ns * nch, "norm partials"))) return rc;
     if ((rc = al((void **)&b.ctot, sizeof(double) * 2 * NSMAX * 4, "slot totals"))) return rc;
     if ((rc = al((void **)&b.ccnt, sizeof(int) * (NSMAX + QMAX), "chunk and work-queue counters"))) return rc;
     if (mixed && c->cgs_on) {
-        if ((rc = al((void **)&b.cpm, sizeof(double) * (size_t)ns * NCH * CGS_NV, "Gram-Schmidt partials"))) return rc;
+        if ((rc = al((void **)&b.cpm, sizeof(double) * (size_t)ns * nch * CGS_NV, "Gram-Schmidt partials"))) return rc;
         if ((rc = al((void **)&b.ctm, sizeof(double) * (size_t)ns * CGS_NV, "Gram-Schmidt totals"))) return rc;
     }
 
     if (cudaMallocHost((void **)&b.h_slots, sizeof(Slot) * ns) != cudaSuccess) return set_error(c, SCD_OOM, "pinned slots");
     int per_sm = 0, per_sm2 = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tick<cd>, BT, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_tick<cf>, BT, 0);
-    per_sm = std::min(per_sm, per_sm2);
+    // with the most shared memory a tick asks for, so that the grid is resident in every variant
+    auto tick_ctas = [](const void *k, int res, size_t el) {
+        const size_t dyn = (size_t)BW * res * CHUNK * el;
+        int ctas = 0;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k, BT, dyn);
+        return ctas;
+    };
+    per_sm = tick_ctas((const void *)k_tick<cd>, RES<cd>, sizeof(cd));
+    const int per_f = tick_ctas((const void *)k_tick<cf>, RES<cf>, sizeof(cf));
+    per_sm = std::min(per_sm, per_f);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_resid, BT, 0);
     per_sm = std::min(per_sm, per_sm2);
     if (per_sm < 1) return set_error(c, SCD_CUDA_ERROR, "tick kernel cannot be resident");
     per_sm = std::min(per_sm, 2);
     b.grid = per_sm * c->nsm;
-    {
-        int per_f = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_f, k_tick<cf>, BT, 0);
-        b.grid_f = std::max(1, std::min(per_f, SCD_TICK_MINB)) * c->nsm;
-    }
+    b.grid_f = std::max(1, std::min(per_f, SCD_TICK_MINB)) * c->nsm;
     if ((rc = al((void **)&b.red, sizeof(double) * 2 * (size_t)b.grid * NSMAX * 4, "partials"))) return rc;
     b.ns = ns;
     b.m = m;
@@ -1063,21 +1263,31 @@ static int launch_tick(scd_ctx *c, BatchBuffers &bb, int ns, int nact, int m, in
     TickArgs<C> a;
     a.slots = bb.slots; a.ns = ns; a.V = (C *)bb.V; a.H = bb.H; a.cs = bb.cs; a.sn = bb.sn; a.g = bb.g; a.y = bb.y;
     a.x = (C *)bb.x; a.rhs = (C *)bb.rhs; a.w = (C *)bb.W; a.red = bb.red; a.bar = c->d_bar; a.err = c->d_err;
+    a.rnorm = bb.rnorm;
     a.cpart = bb.cpart; a.ctot = bb.ctot; a.ccnt = bb.ccnt; a.qctr = bb.ccnt + NSMAX;
     a.n = c->n; a.m = m; a.max_cycles = cycles; a.tol = tol; a.mixed = mixed;
     a.cgs = (mixed && c->cgs_on && bb.cpm) ? 1 : 0;
     a.cpm = bb.cpm; a.ctm = bb.ctm;
     const long long n = c->n;
     if (nact > 0) {
-        k_stage<C><<<dim3(std::min<long long>((n + 255) / 256, 1024), ns), 256, 0, c->st>>>(bb.slots, ns, (C *)bb.V,
-                                                                                           (C *)bb.x, (C *)bb.Xin, n, m);
+        k_stage<C><<<dim3(Chunks::count(n), ns), 256, 0, c->st>>>(bb.slots, ns, (C *)bb.V, (C *)bb.x, (C *)bb.Xin, n, m);
         multi_matvec<C>(c, ops, (const C *)bb.Xin, (C *)bb.W, cnt);
     }
     NvtxRange r("arnoldi tick");
     void *args[] = {&a};
     cudaMemsetAsync(bb.ccnt, 0, sizeof(int) * (NSMAX + QMAX), c->st);
-    const int grid = std::is_same<C, cf>::value ? bb.grid_f : bb.grid;
-    cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_tick<C>, dim3(grid), dim3(BT), args, 0, c->st);
+    // no more CTAs than the (slot, chunk) items have warps for: a barrier of
+    // fewer CTAs is shorter, and no sum depends on the grid
+    const long long items = (long long)ns * Chunks::count(n);
+    const int grid = (int)std::min<long long>(std::is_same<C, cf>::value ? bb.grid_f : bb.grid, (items + BW - 1) / BW);
+    // modified Gram-Schmidt keeps w resident while every warp's items of the
+    // slots fit its share of shared memory (two CTAs of 96 KB per SM) and a
+    // warp can add a slot's partials itself (512: sixteen loads per lane)
+    const long long warps = (long long)grid * BW, per = (items + warps - 1) / warps;
+    a.res = !a.cgs && Chunks::count(n) <= 512 && per <= RES<C> ? (int)per : 0;
+    const size_t dyn = (size_t)BW * a.res * CHUNK * sizeof(C);
+    cudaFuncSetAttribute(k_tick<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BW * RES<C> * CHUNK * sizeof(C)));
+    cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_tick<C>, dim3(grid), dim3(BT), args, dyn, c->st);
     c->launches += 2;
     return check_cuda(c, e, "tick launch");
 }

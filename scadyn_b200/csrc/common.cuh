@@ -114,34 +114,40 @@ template <> SCD_HD cf as_c<cf>(cf a) { return a; }
 template <> SCD_HD cf as_c<cf>(cd a) { return make_float2((float)a.x, (float)a.y); }
 
 // Grid-wide barrier for kernels launched with cudaLaunchCooperativeKernel
-// (all CTAs co-resident).  The spin is bounded: after `limit` polls the CTA
-// records a timeout in *err and continues, so a broken launch ends with an
-// error status instead of a hung GPU.
+// (all CTAs co-resident).  A CTA's writes are released by its arrival and
+// acquired by one fence after the wait; polls are relaxed loads.  The spin is
+// bounded: after `limit` polls the CTA records a timeout in *err and
+// continues, so a broken launch ends with an error status instead of a hung
+// GPU.
 struct GridBarrier {
     unsigned int count;
     unsigned int gen;
 };
 
+__device__ __forceinline__ unsigned int ld_relaxed(const unsigned int *p) {
+    unsigned int v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void grid_barrier(GridBarrier *b, unsigned int nblocks, int *err,
                                              long long limit = (1LL << 24)) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned int *vgen = &b->gen;
-        unsigned int g = *vgen;
-        __threadfence();
-        unsigned int arrived = atomicAdd(&b->count, 1u);
+        const unsigned int g = ld_relaxed(&b->gen);
+        unsigned int arrived;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;\n" : "=r"(arrived) : "l"(&b->count) : "memory");
         if (arrived == nblocks - 1) {
-            atomicExch(&b->count, 0u);
-            __threadfence();
-            atomicAdd(&b->gen, 1u);
+            asm volatile("st.relaxed.gpu.global.u32 [%0], 0;\n" ::"l"(&b->count) : "memory");
+            asm volatile("red.add.release.gpu.global.u32 [%0], 1;\n" ::"l"(&b->gen) : "memory");
         } else {
             long long it = 0;
-            while (*vgen == g) {
+            while (ld_relaxed(&b->gen) == g) {
                 if (++it > limit) { atomicExch(err, 1); break; }
-                __nanosleep(64);
+                if (it > 64) __nanosleep(32);
             }
         }
-        __threadfence();
+        asm volatile("fence.acq_rel.gpu;\n" ::: "memory");
     }
     __syncthreads();
 }
