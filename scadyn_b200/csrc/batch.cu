@@ -54,7 +54,6 @@ struct TickArgs {
     cd *H;          // [slot][(m+1) m]
     cd *cs, *sn, *g, *y;   // [slot][m+1]
     C *x, *rhs, *w; // [slot][n]
-    double *red;    // [2][grid][NSMAX*4]
     double *cpart;  // [slot][nch][4] chunk partials
     double *rnorm;  // [slot][nch] chunk partials of ||w||^2 (resident Gram-Schmidt)
     int res;        // resident Gram-Schmidt: items per warp, 0 = off
@@ -1036,7 +1035,7 @@ struct ResidArgs {
     int ns;
     const cd *b64, *w64;   // rhs and A x, FP64
     cf *rhs32, *x32;       // inner right-hand side (r / rho) and initial guess (0)
-    double *red;
+    double *part;          // [slot][nch][4] chunk partials of ||r||^2, ||b||^2
     GridBarrier *bar;
     int *err;
     long long n;
@@ -1045,86 +1044,97 @@ struct ResidArgs {
 };
 
 // r = b - A x in FP64; stop when ||r||/||b|| < tol, else hand r/||r|| to an
-// inner complex64 solve with a zero initial guess
+// inner complex64 solve with a zero initial guess.  (slot, chunk) items over
+// the tick's chunks, one barrier; every CTA decides from the slots' state as
+// it was before the barrier (CTA 0 writes the new state while slower CTAs
+// still decide).  Summing one slot after another over the whole grid took
+// 75 us for 32 slots of 18,432 unknowns; the items take SCD_R1.
 __global__ void __launch_bounds__(BT) k_resid(ResidArgs a) {
-    __shared__ double bsh[64];
-    __shared__ double tot[NSMAX][4];
-    __shared__ int smode[NSMAX];
+    __shared__ double tot[NSMAX][2], sb64[NSMAX];
+    __shared__ int smode[NSMAX], sout[NSMAX], srpos[NSMAX];
     const long long n = a.n;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const long long q0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    for (int s = threadIdx.x; s < a.ns; s += blockDim.x) smode[s] = a.slots[s].mode;
+    const Chunks ch(n);
+    const int lane = ch.lane, items = a.ns * ch.nch;
+    constexpr int U = 4;
+    for (int s = threadIdx.x; s < a.ns; s += blockDim.x) {
+        smode[s] = a.slots[s].mode;
+        sout[s] = a.slots[s].outer;
+        sb64[s] = a.slots[s].b64;
+        srpos[s] = max(a.slots[s].rpos, 0);
+    }
     __syncthreads();
-    for (int s = 0; s < a.ns; ++s) {
+    for (int it = ch.gw; it < items; it += ch.nw) {
+        const int s = it / ch.nch, c = it - s * ch.nch;
         if (smode[s] != SLOT_RESID) continue;
+        const long long qa = c * ch.L, qb = min(n, qa + ch.L);
+        const cd *bs = a.b64 + (size_t)s * n, *ws = a.w64 + (size_t)srpos[s] * n;
         double v[2] = {0, 0};
-        const cd *bs = a.b64 + (size_t)s * n, *ws = a.w64 + (size_t)max(a.slots[s].rpos, 0) * n;
-        for (long long q = q0; q < n; q += stride) {
-            const cd b = bs[q], r = csub(b, ws[q]);
-            v[0] += cabs2(r);
-            v[1] += cabs2(b);
+        for (long long q = qa + lane; q < qb; q += 32 * U) {
+            cd b[U], w[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                b[u] = w[u] = cmk(0, 0);
+                if (q + 32 * u < qb) { b[u] = bs[q + 32 * u]; w[u] = ws[q + 32 * u]; }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                v[0] += cabs2(csub(b[u], w[u]));
+                v[1] += cabs2(b[u]);
+            }
         }
-        block_sum<2>(v, bsh);
-        if (threadIdx.x == 0) {
-            double *p = a.red + (size_t)blockIdx.x * (NSMAX * 4) + s * 4;
-            p[0] = v[0];
-            p[1] = v[1];
-        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+        if (lane == 0) *reinterpret_cast<double2 *>(a.part + ((size_t)s * ch.nch + c) * 4) = cmk(v[0], v[1]);
     }
     grid_barrier(a.bar, gridDim.x, a.err);
-    {
-        const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        for (int s = wp; s < a.ns; s += nw) {
-            double acc[2] = {0, 0};
-            for (int b = lane; b < (int)gridDim.x; b += 32) {
-                const double *p = a.red + (size_t)b * (NSMAX * 4) + s * 4;
-                acc[0] += __ldcg(p);
-                acc[1] += __ldcg(p + 1);
-            }
-            for (int q = 0; q < 2; ++q)
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-            if (lane == 0) { tot[s][0] = acc[0]; tot[s][1] = acc[1]; }
-        }
-        __syncthreads();
-    }
-    for (int s = 0; s < a.ns; ++s) {
+    for (int s = threadIdx.x >> 5; s < a.ns; s += BW) {
         if (smode[s] != SLOT_RESID) continue;
+        double t[2];
+        lane_partials<2>(a.part + (size_t)s * ch.nch * 4, 4, ch.nch, lane, t);
+        if (lane == 0) { tot[s][0] = t[0]; tot[s][1] = t[1]; }
+    }
+    __syncthreads();
+    auto bnorm = [&](int s) { return sout[s] == 0 ? sqrt(tot[s][1]) : sb64[s]; };
+    auto relres = [&](int s) { const double bn = bnorm(s); return bn > 0.0 ? sqrt(tot[s][0]) / bn : 0.0; };
+    auto stops = [&](int s) { return !(relres(s) >= a.tol) || sout[s] >= a.max_outer; };   // NaN stops too
+    for (int it = ch.gw; it < items; it += ch.nw) {
+        const int s = it / ch.nch, c = it - s * ch.nch;
+        if (smode[s] != SLOT_RESID || stops(s)) continue;
         const double rho = sqrt(tot[s][0]);
-        const double bn = a.slots[s].outer == 0 ? sqrt(tot[s][1]) : a.slots[s].b64;
-        const double rel = bn > 0.0 ? rho / bn : 0.0;
-        const bool stop = !(rel >= a.tol) || a.slots[s].outer >= a.max_outer;   // NaN stops too
-        if (!stop) {
-            const cd *bs = a.b64 + (size_t)s * n, *ws = a.w64 + (size_t)max(a.slots[s].rpos, 0) * n;
-            cf *rs = a.rhs32 + (size_t)s * n, *xs = a.x32 + (size_t)s * n;
-            for (long long q = q0; q < n; q += stride) {
-                const cd r = csub(bs[q], ws[q]);
-                rs[q] = make_float2((float)(r.x / rho), (float)(r.y / rho));
-                xs[q] = make_float2(0.f, 0.f);
-            }
+        const long long qa = c * ch.L, qb = min(n, qa + ch.L);
+        const cd *bs = a.b64 + (size_t)s * n, *ws = a.w64 + (size_t)srpos[s] * n;
+        cf *rs = a.rhs32 + (size_t)s * n, *xs = a.x32 + (size_t)s * n;
+        for (long long q = qa + lane; q < qb; q += 32) {
+            const cd r = csub(bs[q], ws[q]);
+            rs[q] = make_float2((float)(r.x / rho), (float)(r.y / rho));
+            xs[q] = make_float2(0.f, 0.f);
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            Slot &sl = a.slots[s];
-            if (sl.outer == 0) sl.b64 = bn;
-            sl.relres = rel;
-            sl.upd = 0;
-            if (stop) {
-                sl.mode = SLOT_DONE;
-                sl.conv = rel < a.tol;
-                sl.error = rel;
-                if (!(rel == rel)) sl.status = SCD_NAN;
-            } else {
-                sl.rho = rho;
-                sl.outer += 1;
-                sl.mode = SLOT_START;
-                sl.zero_x = 1;
-                sl.cycle = 0;
-                sl.step = 0;
-                sl.conv = 0;
-                sl.finish = 0;
-            }
-            if (*a.err) { sl.status = SCD_TIMEOUT; sl.mode = SLOT_DONE; }
+    }
+    if (blockIdx.x == 0 && threadIdx.x < a.ns && smode[threadIdx.x] == SLOT_RESID) {
+        const int s = threadIdx.x;
+        const double rel = relres(s);
+        Slot &sl = a.slots[s];
+        if (sout[s] == 0) sl.b64 = bnorm(s);
+        sl.relres = rel;
+        sl.upd = 0;
+        if (stops(s)) {
+            sl.mode = SLOT_DONE;
+            sl.conv = rel < a.tol;
+            sl.error = rel;
+            if (!(rel == rel)) sl.status = SCD_NAN;
+        } else {
+            sl.rho = sqrt(tot[s][0]);
+            sl.outer += 1;
+            sl.mode = SLOT_START;
+            sl.zero_x = 1;
+            sl.cycle = 0;
+            sl.step = 0;
+            sl.conv = 0;
+            sl.finish = 0;
         }
+        if (*a.err) { sl.status = SCD_TIMEOUT; sl.mode = SLOT_DONE; }
     }
 }
 
@@ -1139,7 +1149,6 @@ struct BatchBuffers {
     cd *x64 = nullptr, *b64 = nullptr, *Xin64 = nullptr, *W64 = nullptr;   // mixed: FP64 outer vectors
     Slot *slots = nullptr;
     Slot *h_slots = nullptr;
-    double *red = nullptr;
     double *cpart = nullptr, *ctot = nullptr, *rnorm = nullptr;
     double *cpm = nullptr, *ctm = nullptr;   // classical Gram-Schmidt reductions (opt-in)
     int *ccnt = nullptr;
@@ -1149,7 +1158,7 @@ struct BatchBuffers {
 
 static void free_bb(BatchBuffers &b) {
     void *p[] = {b.V, b.H, b.cs, b.sn, b.g, b.y, b.x, b.rhs, b.Xin, b.W, b.x64, b.b64, b.Xin64, b.W64,
-                 b.slots, b.red, b.cpart, b.ctot, b.ccnt, b.cpm, b.ctm, b.rnorm};
+                 b.slots, b.cpart, b.ctot, b.ccnt, b.cpm, b.ctm, b.rnorm};
     for (void *q : p) if (q) cudaFree(q);
     if (b.h_slots) cudaFreeHost(b.h_slots);
     b = BatchBuffers();
@@ -1219,7 +1228,6 @@ int batch_prepare(scd_ctx *c, int ns, int m, int mixed, BatchBuffers &b) {
     per_sm = std::min(per_sm, 2);
     b.grid = per_sm * c->nsm;
     b.grid_f = std::max(1, std::min(per_f, SCD_TICK_MINB)) * c->nsm;
-    if ((rc = al((void **)&b.red, sizeof(double) * 2 * (size_t)b.grid * NSMAX * 4, "partials"))) return rc;
     b.ns = ns;
     b.m = m;
     b.n = n;
@@ -1262,7 +1270,7 @@ static int launch_tick(scd_ctx *c, BatchBuffers &bb, int ns, int nact, int m, in
                        const std::vector<scd_ctx *> &ops, const std::vector<int> &cnt) {
     TickArgs<C> a;
     a.slots = bb.slots; a.ns = ns; a.V = (C *)bb.V; a.H = bb.H; a.cs = bb.cs; a.sn = bb.sn; a.g = bb.g; a.y = bb.y;
-    a.x = (C *)bb.x; a.rhs = (C *)bb.rhs; a.w = (C *)bb.W; a.red = bb.red; a.bar = c->d_bar; a.err = c->d_err;
+    a.x = (C *)bb.x; a.rhs = (C *)bb.rhs; a.w = (C *)bb.W; a.bar = c->d_bar; a.err = c->d_err;
     a.rnorm = bb.rnorm;
     a.cpart = bb.cpart; a.ctot = bb.ctot; a.ccnt = bb.ccnt; a.qctr = bb.ccnt + NSMAX;
     a.n = c->n; a.m = m; a.max_cycles = cycles; a.tol = tol; a.mixed = mixed;
@@ -1421,10 +1429,11 @@ int batch_run(scd_ctx *c, ColumnSource &src, double tol, int m, int cycles, int 
                 multi_matvec<cd>(c, ops, (const cd *)bb.Xin64, bb.W64, cnt_r);
                 ResidArgs ra;
                 ra.slots = bb.slots; ra.ns = ns; ra.b64 = bb.b64; ra.w64 = bb.W64; ra.rhs32 = (cf *)bb.rhs;
-                ra.x32 = (cf *)bb.x; ra.red = bb.red; ra.bar = c->d_bar; ra.err = c->d_err; ra.n = n; ra.tol = tol;
+                ra.x32 = (cf *)bb.x; ra.part = bb.cpart; ra.bar = c->d_bar; ra.err = c->d_err; ra.n = n; ra.tol = tol;
                 ra.max_outer = max_outer;
                 void *args[] = {&ra};
-                cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_resid, dim3(bb.grid), dim3(BT), args, 0, c->st);
+                const int rgrid = (int)std::min<long long>(bb.grid, ((long long)ns * Chunks::count(n) + BW - 1) / BW);
+                cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_resid, dim3(rgrid), dim3(BT), args, 0, c->st);
                 c->launches += 3 + (upd ? 1 : 0);
                 if ((rc = check_cuda(c, e, "residual launch"))) return rc;
             }
