@@ -275,6 +275,19 @@ static int upload_layout(scd_ctx *c, std::vector<NearTile> &tiles, long long off
     CK(cudaMemcpyAsync(c->d_pslot_base, c->pslot_base.data(), sizeof(long long) * (ng + 1), cudaMemcpyHostToDevice, c->st), "slots");
     if (ng) CK(cudaMemcpyAsync(c->d_pslot_cnt, c->pslot_cnt.data(), sizeof(int) * ng, cudaMemcpyHostToDevice, c->st), "slots");
     CK(cudaMemcpyAsync(c->d_grp_tile, c->grp_tile.data(), sizeof(int) * (ng + 1), cudaMemcpyHostToDevice, c->st), "group tiles");
+    // groups by the work of their tiles, in sixteenths of the largest (equal
+    // ones stay in spatial order, for the x segments they share)
+    std::vector<long long> work(ng, 0);
+    for (const NearTile &t : tiles) work[t.g1] += (long long)t.n1 * t.n2;
+    const long long most = ng ? std::max<long long>(1, *std::max_element(work.begin(), work.end())) : 1;
+    std::vector<int> order(ng);
+    for (int g = 0; g < ng; ++g) { order[g] = g; work[g] = 16 * work[g] / most; }
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return work[x] > work[y]; });
+    if ((rc = dalloc(c, &c->d_grp_order, std::max(ng, 1), "group order"))) return rc;
+    if (ng) {
+        CK(cudaMemcpyAsync(c->d_grp_order, order.data(), sizeof(int) * ng, cudaMemcpyHostToDevice, c->st), "group order");
+        CK(cudaStreamSynchronize(c->st), "group order");   // `order` is a local
+    }
     c->ntiles = nt;
     c->part_len = c->pslot_base[ng];
     c->tiles_h.swap(tiles);
@@ -449,7 +462,7 @@ int scd_destroy(scd_ctx *c) {
     if (!c) return SCD_OK;
     cudaSetDevice(c->dev);
     if (c->st) cudaStreamSynchronize(c->st);
-    void *ptrs[] = {c->d_perm, c->d_cube_off, c->d_grp_off, c->d_grp_cube, c->d_grp_tile, c->d_kerr, c->d_P, c->d_Fo, c->d_tdata, c->d_tiles, c->d_pslot_base,
+    void *ptrs[] = {c->d_perm, c->d_cube_off, c->d_grp_off, c->d_grp_cube, c->d_grp_tile, c->d_grp_order, c->d_kerr, c->d_P, c->d_Fo, c->d_tdata, c->d_tiles, c->d_pslot_base,
                     c->d_pslot_cnt, c->d_tc, c->d_tvol, c->d_eps, c->d_bpart, c->d_W, c->d_R, c->d_nzpart, c->d_x,
                     c->d_y, c->d_io, c->d_rhs,
                     c->d_bar, c->d_err, c->d_tw[0], c->d_tw[1], c->d_tw[2], c->f_P, c->f_Fo,

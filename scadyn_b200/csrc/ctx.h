@@ -119,6 +119,7 @@ struct scd_ctx {
     std::vector<int> pslot_cnt;          // per group, number of slots
     std::vector<int> grp_tile;           // ngroups + 1: first tile whose g1 is the group
     int *d_grp_tile = nullptr;
+    int *d_grp_order = nullptr;          // groups by their tiles' work, most first
     int *d_kerr = nullptr;               // near-zone kernel error word (bounded waits)
     long long *d_pslot_base = nullptr;
     int *d_pslot_cnt = nullptr;
@@ -259,5 +260,6 @@ int ensure_work(scd_ctx *c, int nrhs);
 void release_work(scd_ctx *c);
 int near_status(scd_ctx *c);
 // columns of the interleaved matvec input for nrhs right-hand sides: passes
-// of 16, at least 2 (16-byte rows for complex64)
-inline int xt_columns(int nrhs) { return std::max(2, (nrhs + 15) / 16 * 16); }   // SCD_TIMEOUT if a near-zone pipeline wait ran out (and clears it)
+// of 16 in rows of 18 (the FP64 near zone's bank spread), at least 2 (16-byte
+// rows for complex64)
+inline int xt_columns(int nrhs) { return std::max(2, (nrhs + 15) / 16 * 18); }   // SCD_TIMEOUT if a near-zone pipeline wait ran out (and clears it)

@@ -524,16 +524,12 @@ k_fft_x_inv(const Cx *__restrict__ W, Cx *__restrict__ R, const Cx *__restrict__
 // The x segments come from xT, the right-hand sides interleaved per unknown
 // (k_xpose), so a group's x is one contiguous run x[3j+b][r].  Consumer
 // warps release a tile on its slot's "empty" barrier; there is no CTA-wide
-// barrier in the tile loop, so row and column warps run independently.  Warps [0, HT) hold row items (quad q, block row
-// i): a 3 x U register tile of row sums for right-hand sides Uq..Uq+U-1.
-// Warps [HT, 2HT) hold column items (q, block column j).  Lanes run over i
-// (resp. j), so with the odd plane stride both sides read the tile without
-// bank conflicts, and x is a broadcast.
+// barrier in the tile loop.
 //
-// Every sum runs in one canonical order -- row sums: tiles in order, then
-// j = 0..n2-1, then b = 0..2; column sums: i = 0..n1-1, then a = 0..2 --
-// for any number of right-hand sides and any U, so a column's result does
-// not depend on the batch it is solved in.
+// Every sum runs in one canonical order for any number of right-hand sides,
+// so a column's result does not depend on the batch it is solved in: in FP64
+// see k_near_dmma below; in complex64 row sums over tiles in order, then j =
+// 0..n2-1, then b = 0..2, column sums over i = 0..n1-1, then a = 0..2.
 constexpr int NZ_QMAX = 4;             // quads of right-hand sides per pass
 constexpr int NZ_SLOTS = 8;                 // tiles in flight at most (mbarrier pairs)
 constexpr int NZ_META = 272;                // bytes of barriers, ring offsets and the stop flag
@@ -541,14 +537,17 @@ constexpr size_t NZ_SMEM_2CTA = 113 * 1024; // dynamic shared memory per CTA tha
 constexpr size_t NZ_SMEM_4CTA = 56 * 1024;  // ... four CTAs
 // With one right-hand side a tile's sums are short dependent chains, so the
 // kernel is latency-bound per tile: four CTAs per SM (registers and ring
-// bounded to fit) keep four tiles in progress.  With register tiles of four
-// right-hand sides the compiler is left free (two CTAs fit).
+// bounded to fit) keep four tiles in progress; 43,248 tets in FP64 take 276 us
+// so, 319 with three CTAs whose rings hold two tiles.  With register tiles of
+// four right-hand sides the compiler is left free (two CTAs fit).
 template <int U> constexpr int NZ_MIN_CTAS = U == 1 ? 4 : 1;
+template <int NS> constexpr int N1_THREADS = 32 * ((2 * SCD_GROUP_MAX * NS + 31) / 32) + 32;
 constexpr size_t NZ_SMEM_MAX = 227 * 1024;
 constexpr int NZ_MAX_THREADS = 2 * 32 * ((SCD_GROUP_MAX * NZ_QMAX + 31) / 32) + 32;
 
 struct NearPass {
     const NearTile *tiles;
+    const int *grp_order;    // groups, most work first (a short last wave)
     const int *grp_tile, *grp_off;
     const long long *pslot_base;
     const void *data;
@@ -590,59 +589,132 @@ __device__ __forceinline__ void load_xu(uint32_t addr, C (&xu)[U]) {
     }
 }
 
-// partial sums p = 0..NS-1 -> p0 + p1 (NS = 2): NP partials in the lane, or
-// one per lane over L adjacent lanes (lane 0 of each pair gets the total;
-// every lane of the warp must call it)
-template <typename C> __device__ __forceinline__ C shfl_down_c(C v, int d, int width) {
-    v.x = __shfl_down_sync(0xffffffffu, v.x, d, width);
-    v.y = __shfl_down_sync(0xffffffffu, v.y, d, width);
-    return v;
-}
-template <typename C, int U, int NP, int L>
-__device__ __forceinline__ void combine_split(const C (&p)[NP][3][U], C (&tot)[3][U]) {
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if constexpr (NP == 2) {
-                tot[q][u] = cadd(p[0][q][u], p[1][q][u]);
-            } else if constexpr (L == 2) {
-                tot[q][u] = cadd(p[0][q][u], shfl_down_c(p[0][q][u], 1, 2));
-            } else {
-                tot[q][u] = p[0][q][u];
-            }
-        }
-}
-
-// NS (1 or 2) splits every row and column sum into NS partial sums over the
-// j (row) or i (column) residues mod NS, added in order at the end: with one
-// right-hand side (U = 1) NS lanes share a row or column, one partial each;
-// with U = 4 one lane keeps all NS partials.  Either way the sums are formed
-// in the same order, so a column stays bit-identical alone and in a batch.
-template <typename ST, typename C, int U, int NS>
-__global__ void __launch_bounds__(NZ_MAX_THREADS, NZ_MIN_CTAS<U>) k_near_groups(NearPass a) {
-    static_assert(NS == 1 || NS == 2, "split");
-    constexpr int L = U == 1 ? NS : 1;     // lanes per row or column
-    constexpr int NP = NS / L;             // partial sums per lane
-    extern __shared__ __align__(128) unsigned char nz_sh[];
-    uint64_t *full = reinterpret_cast<uint64_t *>(nz_sh);
-    uint64_t *empty = full + NZ_SLOTS;
+// What the near-zone kernels share: the barriers and the ring at the front of
+// dynamic shared memory, and the producer that fills the ring.
+struct NearFrame {
+    uint64_t *full, *empty;
     // per slot, written by the producer before the slot's arrive: ring offset,
     // n2 and column partial slot of the tile (consumers read no tile table)
-    int *toff = reinterpret_cast<int *>(nz_sh + 16 * NZ_SLOTS);
-    int *tn2 = toff + NZ_SLOTS;
-    long long *tcol = reinterpret_cast<long long *>(nz_sh + 24 * NZ_SLOTS);
+    int *toff, *tn2;
+    long long *tcol;
     // raised by the first wait that gives up: the producer issues no more
     // copies, the consumers skip the remaining tiles (still arriving on their
     // barriers), and the kernel returns with a.err set
-    volatile int *stop = reinterpret_cast<volatile int *>(nz_sh + 32 * NZ_SLOTS);
-    C *const X1 = reinterpret_cast<C *>(nz_sh + NZ_META);                 // x(g)
-    unsigned char *const ring = nz_sh + NZ_META + a.x1_bytes;
+    volatile int *stop;
+    unsigned char *x1, *ring;
+    __device__ NearFrame(unsigned char *sh, uint32_t x1_bytes) {
+        full = reinterpret_cast<uint64_t *>(sh);
+        empty = full + NZ_SLOTS;
+        toff = reinterpret_cast<int *>(sh + 16 * NZ_SLOTS);
+        tn2 = toff + NZ_SLOTS;
+        tcol = reinterpret_cast<long long *>(sh + 24 * NZ_SLOTS);
+        stop = reinterpret_cast<volatile int *>(sh + 32 * NZ_SLOTS);
+        x1 = sh + NZ_META;
+        ring = sh + NZ_META + x1_bytes;
+    }
+    // one thread of the CTA, before a __syncthreads
+    __device__ void init(int consumer_warps) const {
+        for (int k = 0; k < NZ_SLOTS; ++k) {
+            mbar_init(&full[k], 1);              // the producer's arrive (with the tile's bytes)
+            mbar_init(&empty[k], consumer_warps);
+        }
+        *stop = 0;
+        mbar_fence_init();
+    }
+};
+
+// The producer thread: tiles t0..t1-1 of group rows [s1, s1 + n1), once per
+// pass of PS right-hand sides, each with its x segment (and the group's own x
+// beside the first).  Ring accounting: `used` bytes are reserved by the
+// `count` tiles in flight (a tile that wraps also reserves the unused end of
+// the ring); tiles are released in order, oldest first.
+template <typename ST, typename C>
+__device__ __forceinline__ void near_produce(const NearPass &a, const NearFrame &f, int t0, int t1, int s1, int n1, int PS) {
     const ST *data = static_cast<const ST *>(a.data);
     const C *xT = static_cast<const C *>(a.xT);
+    const int RG = a.rg_stride;     // xT row length
+    const uint32_t R = a.ring_bytes;
+    uint32_t head = 0, used = 0;
+    uint32_t resv[NZ_SLOTS] = {};
+    int oldest = 0, count = 0, ord = 0;
+    int last[NZ_SLOTS];                  // latest tile issued into each slot
+    for (int k = 0; k < NZ_SLOTS; ++k) last[k] = -1;
+    bool halt = false;
+    auto release_oldest = [&]() {
+        const int k = oldest % NZ_SLOTS;
+        if (!mbar_wait_or(&f.empty[k], (uint32_t)((oldest / NZ_SLOTS) & 1), a.err, f.stop)) halt = true;
+        used -= resv[k];
+        ++oldest;
+        --count;
+    };
+    for (int r0 = 0; r0 < a.nrhs && !halt; r0 += PS) {
+        const C *xp = xT + (long long)(r0 / PS) * a.n * RG;
+        while (count > 0 && !halt) release_oldest();   // x1 is rewritten: the previous pass must be done
+        for (int t = t0; t < t1 && !halt; ++t, ++ord) {
+            const NearTile &tl = a.tiles[t];
+            const uint32_t mb = (uint32_t)(tile_elems(tl.n1, tl.n2) * (long long)sizeof(ST));
+            const uint32_t xb = (uint32_t)(3 * tl.n2 * RG * sizeof(C));
+            const uint32_t x1b = t == t0 ? (uint32_t)(3 * n1 * RG * sizeof(C)) : 0u;
+            const uint32_t S = mb + xb;
+            bool fit = head + S <= R;
+            uint32_t res = fit ? S : (R - head) + S;
+            while (count > 0 && !halt && (count == NZ_SLOTS || used + res > R)) release_oldest();
+            if (halt || *f.stop) { halt = true; break; }
+            if (count == 0) { head = 0; used = 0; fit = true; res = S; }
+            const uint32_t st = fit ? head : 0u;
+            const int k = ord % NZ_SLOTS;
+            f.toff[k] = (int)st;
+            f.tn2[k] = tl.n2;
+            f.tcol[k] = tl.col_off;
+            mbar_expect_tx(&f.full[k], S + x1b);
+            bulk_g2s(f.ring + st, data + tl.data_off, mb, &f.full[k]);
+            bulk_g2s(f.ring + st + mb, xp + 3LL * tl.s2 * RG, xb, &f.full[k]);
+            if (x1b) bulk_g2s(f.x1, xp + 3LL * s1 * RG, x1b, &f.full[k]);
+            head = st + S;
+            used += res;
+            resv[k] = res;
+            last[k] = ord;
+            ++count;
+        }
+    }
+    if (halt) {
+        // a wait gave up: tell the consumers, then let every copy still
+        // landing in the ring finish before the CTA exits
+        *f.stop = 1;
+        for (int k = 0; k < NZ_SLOTS; ++k)
+            if (last[k] >= 0) mbar_wait(&f.full[k], (uint32_t)((last[k] / NZ_SLOTS) & 1), a.err);
+    }
+}
+
+// a consumer warp waits for tile `ord`; false (and the slot released) if the
+// pipeline has stopped -- the warp skips or computes as one
+__device__ __forceinline__ bool near_wait_tile(const NearPass &a, const NearFrame &f, int ord, int lane) {
+    const int k = ord % NZ_SLOTS;
+    bool ok = !*f.stop && mbar_wait_or(&f.full[k], (uint32_t)((ord / NZ_SLOTS) & 1), a.err, f.stop);
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) {
+        *f.stop = 1;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&f.empty[k]);
+    }
+    return ok;
+}
+
+// The complex64 matvec on the CUDA cores (complex128 storage, or on request).
+// Warps [0, HT) hold row items (quad q, block row i): a 3 x U register tile of
+// row sums for right-hand sides Uq..Uq+U-1.  Warps [HT, 2HT) hold column items
+// (q, block column j).  Lanes run over i (resp. j), so with the odd plane
+// stride both sides read the tile without bank conflicts, and x is a
+// broadcast.
+template <typename ST, int U>
+__global__ void __launch_bounds__(NZ_MAX_THREADS, NZ_MIN_CTAS<U>) k_near_groups(NearPass a) {
+    typedef cf C;
+    extern __shared__ __align__(128) unsigned char nz_sh[];
+    const NearFrame f(nz_sh, a.x1_bytes);
+    C *const X1 = reinterpret_cast<C *>(f.x1);                 // x(g)
     C *part = static_cast<C *>(a.part);
 
-    const int g = blockIdx.x;
+    const int g = a.grp_order[blockIdx.x];
     const int t0 = a.grp_tile[g], t1 = a.grp_tile[g + 1];
     const int s1 = a.grp_off[g], n1 = a.grp_off[g + 1] - s1;
     const int ld1 = n1 | 1;
@@ -652,108 +724,32 @@ __global__ void __launch_bounds__(NZ_MAX_THREADS, NZ_MIN_CTAS<U>) k_near_groups(
     const int ncw = 2 * HT / 32;                 // consumer warps
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < NZ_SLOTS; ++k) {
-            mbar_init(&full[k], 1);              // the producer's arrive (with the tile's bytes)
-            mbar_init(&empty[k], ncw);
-        }
-        *stop = 0;
-        mbar_fence_init();
-    }
+    if (threadIdx.x == 0) f.init(ncw);
     __syncthreads();
-
     if (warp == ncw) {
-        // ------------------------------------------------------ producer
-        // ring accounting: `used` bytes are reserved by the `count` tiles in
-        // flight (a tile that wraps also reserves the unused end of the ring);
-        // tiles are released in order, oldest first
-        if (lane == 0) {
-            const uint32_t R = a.ring_bytes;
-            uint32_t head = 0, used = 0;
-            uint32_t resv[NZ_SLOTS] = {};
-            int oldest = 0, count = 0, ord = 0;
-            int last[NZ_SLOTS];                  // latest tile issued into each slot
-            for (int k = 0; k < NZ_SLOTS; ++k) last[k] = -1;
-            bool halt = false;
-            auto release_oldest = [&]() {
-                const int k = oldest % NZ_SLOTS;
-                if (!mbar_wait_or(&empty[k], (uint32_t)((oldest / NZ_SLOTS) & 1), a.err, stop)) halt = true;
-                used -= resv[k];
-                ++oldest;
-                --count;
-            };
-            for (int r0 = 0; r0 < a.nrhs && !halt; r0 += PS) {
-                const C *xp = xT + (long long)(r0 / PS) * a.n * RG;
-                while (count > 0 && !halt) release_oldest();   // X1 is rewritten: the previous pass must be done
-                for (int t = t0; t < t1 && !halt; ++t, ++ord) {
-                    const NearTile &tl = a.tiles[t];
-                    const uint32_t mb = (uint32_t)(tile_elems(tl.n1, tl.n2) * (long long)sizeof(ST));
-                    const uint32_t xb = (uint32_t)(3 * tl.n2 * RG * sizeof(C));
-                    const uint32_t x1b = t == t0 ? (uint32_t)(3 * n1 * RG * sizeof(C)) : 0u;
-                    const uint32_t S = mb + xb;
-                    bool fit = head + S <= R;
-                    uint32_t res = fit ? S : (R - head) + S;
-                    while (count > 0 && !halt && (count == NZ_SLOTS || used + res > R)) release_oldest();
-                    if (halt || *stop) { halt = true; break; }
-                    if (count == 0) { head = 0; used = 0; fit = true; res = S; }
-                    const uint32_t st = fit ? head : 0u;
-                    const int k = ord % NZ_SLOTS;
-                    toff[k] = (int)st;
-                    tn2[k] = tl.n2;
-                    tcol[k] = tl.col_off;
-                    mbar_expect_tx(&full[k], S + x1b);
-                    bulk_g2s(ring + st, data + tl.data_off, mb, &full[k]);
-                    bulk_g2s(ring + st + mb, xp + 3LL * tl.s2 * RG, xb, &full[k]);
-                    if (x1b) bulk_g2s(X1, xp + 3LL * s1 * RG, x1b, &full[k]);
-                    head = st + S;
-                    used += res;
-                    resv[k] = res;
-                    last[k] = ord;
-                    ++count;
-                }
-            }
-            if (halt) {
-                // a wait gave up: tell the consumers, then let every copy
-                // still landing in the ring finish before the CTA exits
-                *stop = 1;
-                for (int k = 0; k < NZ_SLOTS; ++k)
-                    if (last[k] >= 0) mbar_wait(&full[k], (uint32_t)((last[k] / NZ_SLOTS) & 1), a.err);
-            }
-        }
+        if (lane == 0) near_produce<ST, C>(a, f, t0, t1, s1, n1, PS);
         return;
     }
 
     // ---------------------------------------------------------- consumers
     const bool rowside = warp < HT / 32;
     const int it = rowside ? threadIdx.x : threadIdx.x - HT;
-    const bool row_item = rowside && it < n1 * a.nq * L;
-    const int rq = row_item ? it / (n1 * L) : 0;
-    const int ri = row_item ? (it - rq * n1 * L) / L : 0, hl = row_item ? (it - rq * n1 * L) % L : 0;
+    const bool row_item = rowside && it < n1 * a.nq;
+    const int rq = row_item ? it / n1 : 0, ri = row_item ? it - rq * n1 : 0;
     int ord = 0;
     for (int r0 = 0; r0 < a.nrhs; r0 += PS) {
         const int rg = min(PS, a.nrhs - r0);
-        C accs[NP][3][U];
+        C acc[3][U];
 #pragma unroll
-        for (int p = 0; p < NP; ++p)
+        for (int q = 0; q < 3; ++q)
 #pragma unroll
-            for (int q = 0; q < 3; ++q)
-#pragma unroll
-                for (int u = 0; u < U; ++u) accs[p][q][u] = czero<C>();
-        C (&acc)[3][U] = accs[0];
+            for (int u = 0; u < U; ++u) acc[q][u] = czero<C>();
         for (int t = t0; t < t1; ++t, ++ord) {
             const int kslot = ord % NZ_SLOTS;
-            bool ok = !*stop && mbar_wait_or(&full[kslot], (uint32_t)((ord / NZ_SLOTS) & 1), a.err, stop);
-            ok = __all_sync(0xffffffffu, ok);   // the warp skips or computes as one (shuffles below)
-            if (!ok) {
-                *stop = 1;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&empty[kslot]);
-                continue;
-            }
-            const int n2 = tn2[kslot];
-            const int tof = toff[kslot];
-            const long long tcoff = tcol[kslot];
-            const uint32_t M = smem_addr(ring + tof);
+            if (!near_wait_tile(a, f, ord, lane)) continue;
+            const int n2 = f.tn2[kslot];
+            const long long tcoff = f.tcol[kslot];
+            const uint32_t M = smem_addr(f.ring + f.toff[kslot]);
             const uint32_t X2 = M + (uint32_t)(tile_elems(n1, n2) * (long long)sizeof(ST));
             constexpr uint32_t SB = sizeof(ST), CB = sizeof(C);
             const uint32_t mrow = SB * ld1, xrow = CB * RG;   // bytes between planes / x rows
@@ -761,36 +757,17 @@ __global__ void __launch_bounds__(NZ_MAX_THREADS, NZ_MIN_CTAS<U>) k_near_groups(
                 if (row_item) {
                     uint32_t mp = M + SB * ri;            // plane (9j + 3b), lane i
                     uint32_t xp = X2 + CB * U * rq;       // x row 3j + b
-                    // one j: the three b-planes into partial pp
-                    auto row_j = [&](C (&pp)[3][U]) {
-#pragma unroll
-                        for (int b = 0; b < 3; ++b) {
-                            C xu[U];
-                            load_xu<C, U>(xp, xu);
-                            const C mm[3] = {as_c<C>(lds_c(mp, ST{})), as_c<C>(lds_c(mp + mrow, ST{})),
-                                             as_c<C>(lds_c(mp + 2 * mrow, ST{}))};
-                            mac3<C, U>(pp, mm, xu);
-                            mp += 3 * mrow;
-                            xp += xrow;
-                        }
-                    };
-                    if constexpr (NP == 1) {
-                        // lane hl takes j = hl, hl + L, ...
-                        mp += hl * 9 * mrow;
-                        xp += hl * 3 * xrow;
-                        for (int j = hl; j < n2; j += L) {
-                            row_j(acc);
-                            mp += (L - 1) * 9 * mrow;
-                            xp += (L - 1) * 3 * xrow;
-                        }
-                    } else {
-                        for (int j = 0; j < n2; j += 2) {
-                            row_j(accs[0]);
-                            if (j + 1 < n2) row_j(accs[1]);
-                        }
+                    for (int j = 0; j < 3 * n2; ++j) {
+                        C xu[U];
+                        load_xu<C, U>(xp, xu);
+                        const C mm[3] = {as_c<C>(lds_c(mp, ST{})), as_c<C>(lds_c(mp + mrow, ST{})),
+                                         as_c<C>(lds_c(mp + 2 * mrow, ST{}))};
+                        mac3<C, U>(acc, mm, xu);
+                        mp += 3 * mrow;
+                        xp += xrow;
                     }
                 }
-            } else if (NS == 1 && tcoff >= 0 && it < n2 * a.nq) {
+            } else if (tcoff >= 0 && it < n2 * a.nq) {
                 const int q = it / n2, j = it - q * n2;
                 C cacc[3][U];
 #pragma unroll
@@ -821,74 +798,11 @@ __global__ void __launch_bounds__(NZ_MAX_THREADS, NZ_MIN_CTAS<U>) k_near_groups(
                         pc[2] = cacc[2][u];
                     }
                 }
-            } else if (NS > 1 && tcoff >= 0) {
-                // split column sums: partial p over i = p, p + NS, ...; the
-                // lanes of a column are adjacent (all lanes join the shuffle)
-                const bool col_item = it < n2 * a.nq * L;
-                const int q = col_item ? it / (n2 * L) : 0;
-                const int j = col_item ? (it - q * n2 * L) / L : 0, cl = col_item ? (it - q * n2 * L) % L : 0;
-                C cps[NP][3][U];
-#pragma unroll
-                for (int p = 0; p < NP; ++p)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b)
-#pragma unroll
-                        for (int u = 0; u < U; ++u) cps[p][b][u] = czero<C>();
-                if (col_item) {
-                    const uint32_t mj = M + SB * 9 * j * ld1;
-                    const uint32_t x0 = smem_addr(X1) + CB * U * q;   // x row 3i + a
-                    auto col_i = [&](int i, C (&pp)[3][U]) {
-                        uint32_t xp = x0 + 3 * i * xrow;
-#pragma unroll
-                        for (int aa = 0; aa < 3; ++aa) {
-                            C xu[U];
-                            load_xu<C, U>(xp, xu);
-                            const uint32_t mp = mj + aa * mrow + SB * i;
-                            const C mm[3] = {as_c<C>(lds_c(mp, ST{})), as_c<C>(lds_c(mp + 3 * mrow, ST{})),
-                                             as_c<C>(lds_c(mp + 6 * mrow, ST{}))};
-                            mac3<C, U>(pp, mm, xu);
-                            xp += xrow;
-                        }
-                    };
-                    if constexpr (NP == 1) {
-                        for (int i = cl; i < n1; i += L) col_i(i, cps[0]);
-                    } else {
-                        for (int i = 0; i < n1; i += 2) {
-                            col_i(i, cps[0]);
-                            if (i + 1 < n1) col_i(i + 1, cps[1]);
-                        }
-                    }
-                }
-                C ctot[3][U];
-                combine_split<C, U, NP, L>(cps, ctot);
-                if (col_item && cl == 0) {
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const int r = U * q + u;
-                        if (r < rg && !(a.skip && a.skip[r0 + r])) {
-                            C *pc = part + (r0 + r) * a.part_len + tcoff + 3 * j;
-                            pc[0] = ctot[0][u];
-                            pc[1] = ctot[1][u];
-                            pc[2] = ctot[2][u];
-                        }
-                    }
-                }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[kslot]);
+            if (lane == 0) mbar_arrive(&f.empty[kslot]);
         }
-        if constexpr (NS > 1) {
-            if (rowside) {
-                // all row-side lanes take part in the combination (shuffles)
-                C tot[3][U];
-                combine_split<C, U, NP, L>(accs, tot);
-#pragma unroll
-                for (int q = 0; q < 3; ++q)
-#pragma unroll
-                    for (int u = 0; u < U; ++u) acc[q][u] = tot[q][u];
-            }
-        }
-        if (row_item && hl == 0) {
+        if (row_item) {
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int r = U * rq + u;
@@ -900,6 +814,291 @@ __global__ void __launch_bounds__(NZ_MAX_THREADS, NZ_MIN_CTAS<U>) k_near_groups(
                 }
             }
         }
+    }
+}
+
+// ---- FP64
+// Both FP64 kernels form a sum over unknowns k in blocks of four: per block
+// the real part adds Ar(k) xr(k) for the four k in order, then -Ai(k) xi(k);
+// the imaginary part Ar(k) xi(k), then Ai(k) xr(k).  That is what two
+// m8n8k4 DMMAs per part compute (each output is a chain of four fused
+// multiply-adds in k order, checked bit for bit over 128,000 random sums), so
+// one right-hand side on the FMA units and many on the tensor cores give a
+// column the same bits.  NS = 2 sums even and odd blocks of a tile separately,
+// then adds the two.  A row sum adds its tiles' sums in order; k past the end
+// contributes fma(0, 0, s).
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// Two or more right-hand sides, 8 NT of them per pass (their rows of xT are
+// 8 NT + 2 values apart: a quarter-warp's reads of four k and two
+// right-hand sides then fall in distinct banks).  Consumer warp w forms the
+// row sums of unknowns 8w .. 8w + 7 of the group, kept in registers across
+// the tiles, and the column sums of unknowns 8w .. 8w + 7 of each tile's g2:
+// one element read and converted per lane feeds 4 NT DMMAs.  Bound by the
+// FP64 tensor pipe (36 TFLOP/s measured; it is active 64-70 % of the time):
+// 16 right-hand sides of a 12,864-tet sphere take 331 us (585 with register
+// tiles of FMAs), 16 of 3,000 tets 130 (172).
+constexpr int ND_WARPS = (3 * SCD_GROUP_MAX + 7) / 8;   // consumer warps, then the producer
+template <int NT> constexpr int ND_PS = 8 * NT;
+template <int NT> constexpr int ND_RG = 8 * NT + 2;
+
+// a lane's operands of one block: its element and NT values of x, zero past the end
+template <typename ST, int NT> struct DmmaOperands {
+    ST m;
+    cd x[NT];
+    __device__ __forceinline__ void load(uint32_t ma, uint32_t xa, bool in, int nt) {
+        m = in ? lds_c(ma, ST{}) : ST{};
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+            if (t < nt) x[t] = in ? lds_c(xa + 128 * t, cd{}) : cmk(0, 0);
+    }
+};
+template <typename ST, int NT>
+__device__ __forceinline__ void dmma_block(double (&re)[NT][2], double (&im)[NT][2], const DmmaOperands<ST, NT> &o, int nt) {
+    const cd m = as_c<cd>(o.m);
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+        if (t < nt) { dmma(re[t], m.x, o.x[t].x); dmma(im[t], m.x, o.x[t].y); }
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+        if (t < nt) { dmma(re[t], -m.y, o.x[t].y); dmma(im[t], m.y, o.x[t].x); }
+}
+// a tile's sums over K unknowns in blocks of four, the next block's operands
+// read before the present one's DMMAs; at(kk) is the lane's element address
+// for its unknown kk of a block
+template <typename ST, int NT, int NS, typename At>
+__device__ __forceinline__ void dmma_sum(double (&re)[NS][NT][2], double (&im)[NS][NT][2], uint32_t xa, int K, int k4, int nt, At at) {
+#pragma unroll
+    for (int p = 0; p < NS; ++p)
+#pragma unroll
+        for (int t = 0; t < NT; ++t) re[p][t][0] = re[p][t][1] = im[p][t][0] = im[p][t][1] = 0.0;
+    constexpr uint32_t XB = 16 * 4 * ND_RG<NT>;                                // x rows of a block
+    DmmaOperands<ST, NT> cur, nxt;
+    cur.load(at(k4), xa, k4 < K, nt);
+    for (int k = 0; k < K; k += 4 * NS) {
+#pragma unroll
+        for (int p = 0; p < NS; ++p) {
+            const int kp = k + 4 * p;
+            if (p > 0 && kp >= K) break;
+            xa += XB;
+            const int kk = kp + 4 + k4;
+            nxt.load(at(kk), xa, kk < K, nt);
+            dmma_block<ST, NT>(re[p], im[p], cur, nt);
+            cur = nxt;
+        }
+    }
+    if constexpr (NS == 2)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                re[0][t][e] = SCD_ADD(re[0][t][e], re[1][t][e]);
+                im[0][t][e] = SCD_ADD(im[0][t][e], im[1][t][e]);
+            }
+}
+template <int NT>
+__device__ __forceinline__ void dmma_store(cd *part, const NearPass &a, int r0, int rg, long long at, const double (&re)[NT][2],
+                                           const double (&im)[NT][2], int lane) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int r = 8 * t + 2 * (lane & 3) + e;
+            if (r < rg && !(a.skip && a.skip[r0 + r])) part[(r0 + r) * a.part_len + at] = cmk(re[t][e], im[t][e]);
+        }
+}
+
+template <typename ST, int NT, int NS>
+__global__ void __launch_bounds__(32 * ND_WARPS + 32, 2) k_near_dmma(NearPass a) {
+    extern __shared__ __align__(128) unsigned char nz_sh[];
+    const NearFrame f(nz_sh, a.x1_bytes);
+    cd *part = static_cast<cd *>(a.part);
+    const int g = a.grp_order[blockIdx.x];
+    const int t0 = a.grp_tile[g], t1 = a.grp_tile[g + 1];
+    const int s1 = a.grp_off[g], n1 = a.grp_off[g + 1] - s1;
+    const int ld1 = n1 | 1, K1 = 3 * n1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) f.init(ND_WARPS);
+    __syncthreads();
+    if (warp == ND_WARPS) {
+        if (lane == 0) near_produce<ST, cd>(a, f, t0, t1, s1, n1, ND_PS<NT>);
+        return;
+    }
+    constexpr uint32_t SB = sizeof(ST);
+    const int m8 = 8 * warp + (lane >> 2), k4 = lane & 3;
+    const int row = min(m8, K1 - 1);
+    const uint32_t row_at = SB * ((row % 3) * ld1 + row / 3);                  // element (row, 0) of a tile
+    const uint32_t x_at = 16 * (k4 * ND_RG<NT> + (lane >> 2));
+    int ord = 0;
+    for (int r0 = 0; r0 < a.nrhs; r0 += ND_PS<NT>) {
+        const int rg = min(ND_PS<NT>, a.nrhs - r0), nt = (rg + 7) / 8;
+        double rre[NT][2], rim[NT][2], re[NS][NT][2], im[NS][NT][2];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) rre[t][0] = rre[t][1] = rim[t][0] = rim[t][1] = 0.0;
+        for (int t = t0; t < t1; ++t, ++ord) {
+            if (!near_wait_tile(a, f, ord, lane)) continue;
+            const int kslot = ord % NZ_SLOTS;
+            const int n2 = f.tn2[kslot], K2 = 3 * n2;
+            const long long tcoff = f.tcol[kslot];
+            const uint32_t M = smem_addr(f.ring + f.toff[kslot]);
+            const uint32_t X2 = M + (uint32_t)(tile_elems(n1, n2) * (long long)sizeof(ST));
+            if (8 * warp < K1) {
+                dmma_sum<ST, NT, NS>(re, im, X2 + x_at, K2, k4, nt, [&](int kk) { return M + row_at + SB * 3 * ld1 * kk; });
+#pragma unroll
+                for (int q = 0; q < NT; ++q)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        rre[q][e] = SCD_ADD(rre[q][e], re[0][q][e]);
+                        rim[q][e] = SCD_ADD(rim[q][e], im[0][q][e]);
+                    }
+            }
+            if (tcoff >= 0 && 8 * warp < K2) {
+                const uint32_t mc = M + SB * 3 * min(m8, K2 - 1) * ld1;
+                int aa = k4 % 3, i = k4 / 3;              // row kk = 3i + aa, in steps of four
+                dmma_sum<ST, NT, NS>(re, im, smem_addr(f.x1) + x_at, K1, k4, nt, [&](int) {
+                    const uint32_t at = mc + SB * (aa * ld1 + i);
+                    ++i;
+                    if (++aa == 3) { aa = 0; ++i; }
+                    return at;
+                });
+                if (m8 < K2) dmma_store<NT>(part, a, r0, rg, tcoff + m8, re[0], im[0], lane);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&f.empty[kslot]);
+        }
+        if (m8 < K1) dmma_store<NT>(part, a, r0, rg, a.pslot_base[g] + m8, rre, rim, lane);
+    }
+}
+
+// One right-hand side: NS adjacent lanes form the three row sums of one tet of
+// the group, or the three column sums of one tet of g2, lane p the blocks p,
+// p + NS, ...: per block 12 elements and 4 values of x are read together for
+// 48 FMAs.  Row and column items run the same code on other addresses and
+// follow one another over the lanes, so that a tile of 20 x 20 tets fills 80
+// of 96 lanes (40 + 40 of 64 + 64 with a side to each warp): the conversions
+// of the stored complex64 elements, each made once for its row and once for
+// its column, are what the kernel is bound by.  150,720 tets take 723 us,
+// 4.1 TB/s of tiles (788 with a side to each warp), 43,248 take 276 (323),
+// 1,680 take 45 (54).
+template <typename ST> struct OneBlock {
+    ST m[4][3];
+    cd x[4];
+    // element d of unknown q at ma[q] + d * md
+    __device__ __forceinline__ void load(const uint32_t (&ma)[4], uint32_t md, uint32_t xa, int nk) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const bool in = q < nk;
+            x[q] = in ? lds_c(xa + 16 * q, cd{}) : cmk(0, 0);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) m[q][d] = in ? lds_c(ma[q] + d * md, ST{}) : ST{};
+        }
+    }
+    __device__ __forceinline__ void add(cd (&acc)[3]) const {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const cd v = as_c<cd>(m[q][d]);
+                acc[d].x = SCD_FMA(v.x, x[q].x, acc[d].x);
+                acc[d].y = SCD_FMA(v.x, x[q].y, acc[d].y);
+            }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const cd v = as_c<cd>(m[q][d]);
+                acc[d].x = SCD_FMA(-v.y, x[q].y, acc[d].x);
+                acc[d].y = SCD_FMA(v.y, x[q].x, acc[d].y);
+            }
+    }
+};
+// the NS lanes' sums added (every lane of the warp calls it)
+template <int NS>
+__device__ __forceinline__ void one_combine(cd (&acc)[3]) {
+    if constexpr (NS == 2)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const cd o = make_double2(__shfl_xor_sync(0xffffffffu, acc[d].x, 1), __shfl_xor_sync(0xffffffffu, acc[d].y, 1));
+            acc[d] = cadd(acc[d], o);
+        }
+}
+
+template <typename ST, int NS>
+__global__ void __launch_bounds__(N1_THREADS<NS>, 4) k_near_one(NearPass a) {
+    extern __shared__ __align__(128) unsigned char nz_sh[];
+    const NearFrame f(nz_sh, a.x1_bytes);
+    cd *part = static_cast<cd *>(a.part);
+    const int g = a.grp_order[blockIdx.x];
+    const int t0 = a.grp_tile[g], t1 = a.grp_tile[g + 1];
+    const int s1 = a.grp_off[g], n1 = a.grp_off[g + 1] - s1;
+    const int ld1 = n1 | 1, ncw = a.half / 32;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) f.init(ncw);
+    __syncthreads();
+    if (warp == ncw) {
+        if (lane == 0) near_produce<ST, cd>(a, f, t0, t1, s1, n1, 1);
+        return;
+    }
+    constexpr uint32_t SB = sizeof(ST);
+    const bool on = !(a.skip && a.skip[0]);
+    const int item = threadIdx.x / NS, p = threadIdx.x - NS * item;   // row tets, then column tets; partial
+    const bool row = item < n1;
+    const int col = item - n1;
+    const uint32_t plane = SB * ld1;
+    // element (d, k = 3i + aa) of the item: from one k to the next `inc`, from
+    // aa = 2 to the next i `wrap`; d planes md apart
+    const uint32_t md = row ? plane : 3 * plane;
+    const uint32_t inc = row ? 3 * plane : plane, wrap = row ? 3 * plane : SB - 2 * plane;
+    const uint32_t first = row ? SB * item + 12 * p * plane : 9 * col * plane + ((4 * p) % 3) * plane + SB * ((4 * p) / 3);
+    cd sum[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)};
+    for (int t = t0, ord = 0; t < t1; ++t, ++ord) {
+        if (!near_wait_tile(a, f, ord, lane)) continue;
+        const int kslot = ord % NZ_SLOTS;
+        const int n2 = f.tn2[kslot];
+        const long long tcoff = f.tcol[kslot];
+        const uint32_t M = smem_addr(f.ring + f.toff[kslot]);
+        const uint32_t X2 = M + (uint32_t)(tile_elems(n1, n2) * (long long)sizeof(ST));
+        cd acc[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)};
+        const bool cols = !row && tcoff >= 0 && col < n2;
+        const int K = row ? 3 * n2 : cols ? 3 * n1 : 0;
+        uint32_t ma = M + first, xa = (row ? X2 : smem_addr(f.x1)) + 64 * p;
+        int aa = (4 * p) % 3;
+        OneBlock<ST> o;
+        for (int k = 4 * p; k < K; k += 4 * NS) {
+            uint32_t m4[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                m4[q] = ma;
+                ma += aa == 2 ? wrap : inc;
+                aa = aa == 2 ? 0 : aa + 1;
+            }
+            o.load(m4, md, xa, K - k);
+            o.add(acc);
+            if constexpr (NS == 2) {       // the other lane's block
+                ma += 3 * inc + (wrap - inc) + (aa == 2 ? wrap : inc);
+                aa = aa == 2 ? 0 : aa + 1;
+            }
+            xa += 64 * NS;
+        }
+        __syncwarp();
+        one_combine<NS>(acc);
+        if (row) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) sum[d] = cadd(sum[d], acc[d]);
+        } else if (cols && p == 0 && on) {
+            cd *pc = part + tcoff + 3 * col;
+            pc[0] = acc[0]; pc[1] = acc[1]; pc[2] = acc[2];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&f.empty[kslot]);
+    }
+    if (row && p == 0 && on) {
+        cd *pr = part + a.pslot_base[g] + 3 * item;
+        pr[0] = sum[0]; pr[1] = sum[1]; pr[2] = sum[2];
     }
 }
 
@@ -1241,23 +1440,23 @@ void fft_chain_t(scd_ctx *c, const C *x, int nrhs, const int *done) {
     c->launches += tl ? 4 : 6;
 }
 
-template <typename ST, typename C, int U, int NS>
-void near_launch(scd_ctx *c, const ST *data, const C *x, int nrhs, const int *done) {
-    NearPass a;
-    a.tiles = c->d_tiles; a.grp_tile = c->d_grp_tile; a.grp_off = c->d_grp_off; a.pslot_base = c->d_pslot_base;
+// One near-zone launch: `passes` of PS right-hand sides whose rows of xT are
+// rg values apart, ncw consumer warps per CTA, shared memory for `budget`
+// bytes per CTA where a tile with its x fits it.
+template <typename ST, typename C, typename K>
+void near_launch(scd_ctx *c, K kernel, const ST *data, const C *x, int nrhs, int PS, int rg, int threads, size_t budget,
+                 NearPass a, const int *done) {
+    a.tiles = c->d_tiles; a.grp_order = c->d_grp_order; a.grp_tile = c->d_grp_tile; a.grp_off = c->d_grp_off; a.pslot_base = c->d_pslot_base;
     a.data = data; a.xT = Res<C>::xT(c); a.n = c->n; a.part = Res<C>::part(c); a.part_len = c->part_len;
     a.skip = done; a.nrhs = nrhs;
     a.err = c->d_kerr;
-    const int nq = U == 1 ? 1 : std::min(NZ_QMAX, (nrhs + U - 1) / U);
-    a.nq = nq;
-    a.half = 32 * ((c->max_per_group * a.nq * (U == 1 ? NS : 1) + 31) / 32);   // lanes per side
     // xT rows are whole 16-byte units (bulk-copy granularity)
-    a.rg_stride = nq * U;
+    a.rg_stride = rg;
     while ((a.rg_stride * sizeof(C)) % 16) ++a.rg_stride;
     a.x1_bytes = (uint32_t)(3 * c->max_per_group * a.rg_stride * sizeof(C));
-    // the ring fills what two CTAs per SM leave, and must hold the largest tile with its x
+    // the ring fills the budget, and must hold the largest tile with its x
     const size_t max_tile = (size_t)c->max_tile_store * sizeof(ST) + a.x1_bytes;
-    size_t ring = ((U == 1 ? NZ_SMEM_4CTA : NZ_SMEM_2CTA) - NZ_META - a.x1_bytes) / 16 * 16;
+    size_t ring = (budget - NZ_META - a.x1_bytes) / 16 * 16;
     if (ring < max_tile) ring = std::min((NZ_SMEM_MAX - NZ_META - a.x1_bytes) / 16 * 16, (max_tile + 15) / 16 * 16 * 2);
     if (ring < max_tile) {
         // cannot happen with groups of at most SCD_GROUP_MAX slots; reported
@@ -1266,34 +1465,52 @@ void near_launch(scd_ctx *c, const ST *data, const C *x, int nrhs, const int *do
         return;
     }
     a.ring_bytes = (uint32_t)ring;
-    {
-        const int npass = (nrhs + nq * U - 1) / (nq * U);
-        dim3 g((unsigned)((c->n + 255) / 256), npass);
-        k_xpose<C><<<g, 256, 0, c->st>>>(x, c->n, c->n, nrhs, nq * U, a.rg_stride, Res<C>::xT(c));
-        c->launches += 1;
-    }
+    const dim3 g((unsigned)((c->n + 255) / 256), (nrhs + PS - 1) / PS);
+    k_xpose<C><<<g, 256, 0, c->st>>>(x, c->n, c->n, nrhs, PS, a.rg_stride, Res<C>::xT(c));
+    c->launches += 1;
     const size_t sh = NZ_META + a.x1_bytes + a.ring_bytes;
-    cudaFuncSetAttribute(k_near_groups<ST, C, U, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     if (c->timing) cudaEventRecord(c->ev[6], c->st);
-    k_near_groups<ST, C, U, NS><<<c->ngroups, 2 * a.half + 32, sh, c->st>>>(a);
+    kernel<<<c->ngroups, threads, sh, c->st>>>(a);
     if (c->timing) cudaEventRecord(c->ev[7], c->st);
 }
 
-template <typename ST, typename C>
-void near_dispatch(scd_ctx *c, const ST *data, const C *x, int nrhs, const int *done) {
-    // near_split 2 (the default): two partial sums per row and column (two
-    // lanes each at one right-hand side, both in one lane at four) for the
-    // FP64 matvec, the same arithmetic per sum at U = 1 and U = 4, so a column
-    // keeps its bits alone and in a batch; the complex64 matvec of the mixed
-    // form keeps one sum per lane (its U = 4 kernel would lose occupancy to
-    // the second set of accumulators)
-    if (c->near_split == 2 && std::is_same<C, cd>::value) {
-        if (nrhs == 1) near_launch<ST, C, 1, 2>(c, data, x, nrhs, done);
-        else near_launch<ST, C, 4, 2>(c, data, x, nrhs, done);
-    } else {
-        if (nrhs == 1) near_launch<ST, C, 1, 1>(c, data, x, nrhs, done);
-        else near_launch<ST, C, 4, 1>(c, data, x, nrhs, done);
-    }
+template <typename ST, int U>
+void near_cf(scd_ctx *c, const ST *data, const cf *x, int nrhs, const int *done) {
+    NearPass a{};
+    a.nq = U == 1 ? 1 : std::min(NZ_QMAX, (nrhs + U - 1) / U);
+    a.half = 32 * ((c->max_per_group * a.nq + 31) / 32);   // lanes per side
+    near_launch<ST, cf>(c, k_near_groups<ST, U>, data, x, nrhs, a.nq * U, a.nq * U, 2 * a.half + 32,
+                        U == 1 ? NZ_SMEM_4CTA : NZ_SMEM_2CTA, a, done);
+}
+
+template <typename ST, int NS>
+void near_cd(scd_ctx *c, const ST *data, const cd *x, int nrhs, const int *done) {
+    NearPass a{};
+    a.nq = 1;
+    a.half = 32 * ((2 * NS * c->max_per_group + 31) / 32);   // consumer lanes of the one-column kernel
+    // one right-hand side on the FMA units takes 276 us at 43,248 tets; the
+    // DMMAs, padded to 8 columns, could not take less than 336 (12.1 GFLOP at
+    // 36 TFLOP/s), which they share among two or more
+    if (nrhs == 1)
+        near_launch<ST, cd>(c, k_near_one<ST, NS>, data, x, 1, 1, 1, a.half + 32, NZ_SMEM_4CTA, a, done);
+    else if (nrhs <= 8)
+        near_launch<ST, cd>(c, k_near_dmma<ST, 1, NS>, data, x, nrhs, ND_PS<1>, ND_RG<1>, 32 * ND_WARPS + 32, NZ_SMEM_2CTA, a, done);
+    else
+        near_launch<ST, cd>(c, k_near_dmma<ST, 2, NS>, data, x, nrhs, ND_PS<2>, ND_RG<2>, 32 * ND_WARPS + 32, NZ_SMEM_2CTA, a, done);
+}
+
+template <typename ST>
+void near_dispatch(scd_ctx *c, const ST *data, const cf *x, int nrhs, const int *done) {
+    if (nrhs == 1) near_cf<ST, 1>(c, data, x, nrhs, done);
+    else near_cf<ST, 4>(c, data, x, nrhs, done);
+}
+// near_split 2 (the default): two partial sums per row and column sum, in
+// every FP64 kernel, so a column keeps its bits alone and in a batch
+template <typename ST>
+void near_dispatch(scd_ctx *c, const ST *data, const cd *x, int nrhs, const int *done) {
+    if (c->near_split == 2) near_cd<ST, 2>(c, data, x, nrhs, done);
+    else near_cd<ST, 1>(c, data, x, nrhs, done);
 }
 
 template <typename C>
@@ -1305,8 +1522,8 @@ void near_t(scd_ctx *c, const C *x, int nrhs, const int *done) {
             return;
         }
     }
-    if (c->near_prec == SCD_STORE_C64) near_dispatch<cf, C>(c, (const cf *)c->d_tdata, x, nrhs, done);
-    else near_dispatch<cd, C>(c, (const cd *)c->d_tdata, x, nrhs, done);
+    if (c->near_prec == SCD_STORE_C64) near_dispatch<cf>(c, (const cf *)c->d_tdata, x, nrhs, done);
+    else near_dispatch<cd>(c, (const cd *)c->d_tdata, x, nrhs, done);
     c->launches += 1;
 }
 
