@@ -887,12 +887,12 @@ def sweep_bench(nw, nmax_cap):
 
 def fft_len(v, smooth):
     """Padded FFT length the library picks for 2N = v (power of two, or the
-    shorter of 80, 96, 192 with 5-smooth lengths enabled)."""
+    shorter of 40, 48, 80, 96, 112, 192 with the default lengths)."""
     p2 = 8
     while p2 < v:
         p2 *= 2
     if smooth:
-        for p in (80, 96, 192):
+        for p in (40, 48, 80, 96, 112, 192):
             if v <= p < p2:
                 return p
     return p2

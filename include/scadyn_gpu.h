@@ -80,14 +80,14 @@ typedef struct scd_grid_desc {
 /* scd_grid_desc.fft_passes */
 #define SCD_FFT_PASSES_DEFAULT  0   /* SCD_FFT_PASSES_FUSED_YZ where the lengths and shared memory allow */
 #define SCD_FFT_PASSES_FUSED_YZ 1   /* one kernel per (x column, grid) transforms y, z, x Fg, z^-1, y^-1 in
-                                       shared memory (y and z lengths 64, 80, 96, 128 or 192) */
+                                       shared memory (every length but 8, 256 and 512) */
 #define SCD_FFT_PASSES_THREE    2   /* separate y forward, z (forward, x Fg, inverse), y inverse passes */
 
 /* scd_grid_desc.fft_lengths.  Every choice is an exact linear convolution:
  * the input occupies N <= P/2 samples of each axis. */
 #define SCD_FFT_DEFAULT         0   /* SCD_FFT_SMOOTH */
 #define SCD_FFT_POW2            1   /* smallest power of two >= 2N */
-#define SCD_FFT_SMOOTH          2   /* smallest of the powers of two and 80, 96, 192 that is >= 2N */
+#define SCD_FFT_SMOOTH          2   /* smallest of the powers of two and 40, 48, 80, 96, 112, 192 that is >= 2N */
 
 /* scd_grid_desc.near_kernel: the near-zone SpMV of the complex64 matvec of the
  * mixed-precision inner solves (the FP64 matvec always runs on the CUDA cores) */

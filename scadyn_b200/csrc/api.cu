@@ -48,11 +48,11 @@ static int next_pow2(int v) {
 
 // FFT length of an axis with N nodes: the smallest power of two >= 2N, or
 // (the default) the smallest length >= 2N among the powers of two and the
-// 5-smooth lengths with register transforms (80, 96, 192)
+// 7-smooth lengths with register transforms (40, 48, 80, 96, 112, 192)
 static int fft_len(int v, bool smooth) {
     const int p2 = next_pow2(v);
     if (!smooth) return p2;
-    for (int p : {80, 96, 192})
+    for (int p : {40, 48, 80, 96, 112, 192})
         if (p >= v && p < p2) return p;
     return p2;
 }

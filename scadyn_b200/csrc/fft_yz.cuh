@@ -1,13 +1,12 @@
 // The y and z passes of the pruned FFT convolution fused into one kernel,
 // one CTA per (x column, grid): the (y, z) plane of an x-transformed grid is
-// held in shared memory and transformed along y (length PY, zero padded from
-// Ny), then along z (length PZ, zero padded from Nz) in chunks of KC lines,
-// multiplied by the Green spectrum, transformed back along z and y, and its
-// Ny x Nz corner is written back in place.  Replaces the three passes y
-// forward, z (forward, x Fg, inverse), y inverse (FFT3d_2 / IFFT3d_2,
-// src/possu.f90:140-289, with the product of src/gmres_module.f90:104...):
-// the plane crosses HBM once each way instead of six times, and the z lines
-// are never strided in global memory.
+// transformed along y (length PY, zero padded from Ny) into shared memory,
+// then along z (length PZ, zero padded from Nz), multiplied by the Green
+// spectrum, transformed back along z and y, and its Ny x Nz corner is written
+// back in place.  Replaces the three passes y forward, z (forward, x Fg,
+// inverse), y inverse (FFT3d_2 / IFFT3d_2, src/possu.f90:140-289, with the
+// product of src/gmres_module.f90:104...): the plane crosses HBM once each way
+// instead of six times, and the z lines are never strided in global memory.
 //
 // Global layout of an x-transformed grid (rg = 4 r + g): Wt[rg][x][z][y],
 // x < Px, z < Nz, y < Ny (y fastest), written by the x forward pass and read
@@ -16,51 +15,38 @@
 // Fyz[(fx Hy + fy) Hz + fz], H = P/2 + 1.
 //
 // Shared memory (elements of C): twiddles twy[PY], twz[PZ]; the plane
-// A[NzR][LSY] (row z holds the y line, padded index pidx); the chunk
-// B[KC][LSZ] (row l holds the z line of ky = ky0 + l).  NzR = Nz rounded up
-// to a multiple of 8, so that a warp's lines are either all real or all
-// padding rows (the line transforms are warp-synchronous).
+// A[Nz][LSY], whose column c = (p + PER b) T + t of row z holds ky = t PER + p
+// + N1 b (so that a line's threads store consecutive columns); one exchange
+// buffer per warp.  Lines are transformed in registers (fft_line.cuh): a y
+// line goes from global memory to the plane, a z line from a column of the
+// plane through the Green product and back, a y line from the plane to global
+// memory, each with one exchange per transform.  A z line reads and writes its
+// own column only, so the CTA synchronises twice in all.
 //
-// Line transforms are the register transforms of fft_reg.cuh (P = 64, 128,
-// 8 threads per line) and fft_mixed.cuh (P = 80, 96 with 4 threads, 192 with
-// 8).  The phases below are host-callable so that a host program can run the
-// whole pass thread by thread and check it (tests/fft_yz_check.cu).
+// Bound by shared memory and instruction issue about equally.  Before, the
+// lines lived in shared memory between their phases (14 accesses an element
+// where 5 remain) and only 64, 80, 96, 128 and 192 had a transform, so that a
+// 22-node axis ran at 64 instead of 48.  32 complex64 right-hand sides: grid
+// 22 x 20 x 18 156 -> 51 us, 46 x 40 x 28 585 -> 294; 16 in FP64, 24 x 24 x 24
+// 242 -> 83; one in FP64, 64 x 54 x 40 126 -> 73.
+//
+// The phases are host-callable so that a host program can run the whole pass
+// line by line and check it (tests/fft_yz_check.cu).
 #pragma once
+#include <algorithm>
+
 #include "common.cuh"
-#include "fft_mixed.cuh"
-#include "fft_reg.cuh"
+#include "fft_line.cuh"
 
-constexpr int YZ_THREADS = 256;
-
-// Line stride in shared memory: at least the padded line (pidx range), and
-// such that the lines a half-warp transforms together fall in disjoint
-// 8-byte bank pairs: with 8 threads per line a half-warp holds 2 lines, each
-// touching 8 consecutive pairs per access, so the stride is 8 mod 16 pairs;
-// with 4 threads it holds 4 lines of 4 pairs, so 4 or 12 mod 16.
-constexpr int yz_line_stride(int P, int tpl) {
-    int L = P + (P >> 4) + 1;
-    while (tpl == 8 ? (L % 16 != 8) : (L % 16 != 4 && L % 16 != 12)) ++L;
-    return L;
-}
+constexpr int YZ_THREADS = 256;   // most threads of a CTA
 
 template <int P> struct YzLine {
-    static constexpr bool REG = P == 64 || P == 128;
-    static constexpr bool MIX = P == 80 || P == 96 || P == 192;
-    static constexpr bool OK = REG || MIX;
-    static constexpr int TPL = REG ? 8 : (P % 64 == 0 ? 8 : 4);   // threads per line
-    static constexpr int LS = yz_line_stride(P, TPL);               // line stride
-    static constexpr int LINES = YZ_THREADS / TPL;                  // lines per round
+    static constexpr bool OK = half_len(P);
+    static constexpr int TPL = HalfLine<P>::T;
+    // plane row stride: 4 mod 8, so that four threads of four lines fall in
+    // distinct banks along the rows (y) and across them (z)
+    static constexpr int LS = (P + 7) / 8 * 8 + 4;
 };
-
-// Chunk copies between the plane's columns and the z lines run over 4 x 4
-// tiles (4 consecutive lines ky by 4 consecutive z per half-warp): the plane
-// side reads 4 runs of 4 contiguous elements, the chunk side writes 4 runs of
-// 4, instead of 16 elements one line stride apart on one side.
-SCD_HD void yz_tile4(int e, int nl, int &l, int &z) {
-    const int w = e & 15, blk = e >> 4, nbl = nl >> 2;
-    l = ((blk % nbl) << 2) + (w & 3);
-    z = ((blk / nbl) << 2) + (w >> 2);
-}
 
 struct YzDims {
     int Nx, Ny, Nz, NzR;   // grid nodes, Nz rounded up to a multiple of 8
@@ -71,172 +57,239 @@ struct YzDims {
 SCD_HD int yz_fold(int u, int P) { return u <= P - u ? u : P - u; }
 SCD_HD int yz_round8(int n) { return (n + 7) & ~7; }
 
-// shared-memory elements of one CTA
+// exchange elements of a warp
+template <int PY, int PZ> constexpr int yz_ex() {
+    return HalfLine<PY>::EW > HalfLine<PZ>::EW ? HalfLine<PY>::EW : HalfLine<PZ>::EW;
+}
+// shared-memory elements of a CTA of `threads` for planes of nz rows
 template <int PY, int PZ>
-SCD_HD long long yz_smem_elems(int NzR) {
-    return (long long)PY + PZ + (long long)NzR * YzLine<PY>::LS + (long long)YzLine<PZ>::LINES * YzLine<PZ>::LS;
+SCD_HD long long yz_smem_elems(int nz, int threads = YZ_THREADS) {
+    return (long long)PY + PZ + (long long)nz * YzLine<PY>::LS + (long long)(threads / 32) * yz_ex<PY, PZ>();
 }
 
-// plane load: A[z][y] = Wp[z Ny + y] for z < Nz, y < Ny, zero elsewhere
-// (the y padding and the rows Nz..NzR-1)
+// ky of plane column c
+template <int PY> SCD_HD int yz_ky(int c) {
+    using H = HalfLine<PY>;
+    const int t = c % H::T, q = c / H::T;
+    return t * H::PER + q % H::PER + H::N1 * (q / H::PER);
+}
+
+// thread t of the y line of row z: global row -> x
 template <int PY, typename C>
-SCD_HD void yz_load(int tid, C *A, const C *Wp, const YzDims &D) {
-    constexpr int LSY = YzLine<PY>::LS;
-    for (int e = tid; e < D.NzR * PY; e += YZ_THREADS) {
-        const int z = e / PY, y = e - z * PY;
-        A[z * LSY + pidx(y)] = (z < D.Nz && y < D.Ny) ? Wp[(long long)z * D.Ny + y] : czero<C>();
-    }
+SCD_HD void yz_y_load(C (&x)[HalfLine<PY>::M], const C *Wp, int z, int t, bool live, const YzDims &D) {
+    using H = HalfLine<PY>;
+    ct_for<H::M>([&](auto k) {
+        const int y = t + H::T * k;
+        x[k] = live && y < D.Ny ? Wp[(long long)z * D.Ny + y] : czero<C>();
+    });
 }
-
-// plane store: Wp[z Ny + y] = A[z][y] for z < Nz, y < Ny
 template <int PY, typename C>
-SCD_HD void yz_store(int tid, const C *A, C *Wp, const YzDims &D) {
-    constexpr int LSY = YzLine<PY>::LS;
-    const int n = D.Nz * D.Ny;
-    for (int e = tid; e < n; e += YZ_THREADS) {
-        const int z = e / D.Ny, y = e - z * D.Ny;
-        Wp[e] = A[z * LSY + pidx(y)];
-    }
+SCD_HD void yz_y_put(const C (&u)[HalfLine<PY>::PER][HalfLine<PY>::T], C *A, int z, int t) {
+    using H = HalfLine<PY>;
+    ct_for<H::PER>([&](auto p) {
+        ct_for<H::T>([&](auto b) { A[z * YzLine<PY>::LS + (p + H::PER * b) * H::T + t] = u[p][b]; });
+    });
 }
-
-// chunk load: B[l][z] = A[z][ky0 + l] for z < Nz and ky0 + l < PY, zero
-// elsewhere (the z padding and lines past PY)
+template <int PY, typename C>
+SCD_HD void yz_y_get(C (&u)[HalfLine<PY>::PER][HalfLine<PY>::T], const C *A, int z, int t, bool live) {
+    using H = HalfLine<PY>;
+    ct_for<H::PER>([&](auto p) {
+        ct_for<H::T>([&](auto b) { u[p][b] = live ? A[z * YzLine<PY>::LS + (p + H::PER * b) * H::T + t] : czero<C>(); });
+    });
+}
+template <int PY, typename C>
+SCD_HD void yz_y_store(const C (&x)[HalfLine<PY>::M], C *Wp, int z, int t, const YzDims &D) {
+    using H = HalfLine<PY>;
+    ct_for<H::M>([&](auto k) {
+        const int y = t + H::T * k;
+        if (y < D.Ny) Wp[(long long)z * D.Ny + y] = x[k];
+    });
+}
+// thread t of the z line of plane column c
 template <int PY, int PZ, typename C>
-SCD_HD void yz_zload(int tid, const C *A, C *B, int ky0, const YzDims &D) {
-    constexpr int LSY = YzLine<PY>::LS, LSZ = YzLine<PZ>::LS, KC = YzLine<PZ>::LINES;
-    static_assert(KC % 4 == 0 && PZ % 4 == 0, "4 x 4 tiles");
-    for (int e = tid; e < KC * PZ; e += YZ_THREADS) {
-        int l, z;
-        yz_tile4(e, KC, l, z);
-        const int ky = ky0 + l;
-        B[l * LSZ + pidx(z)] = (z < D.Nz && ky < PY) ? A[z * LSY + pidx(ky)] : czero<C>();
-    }
+SCD_HD void yz_z_load(C (&x)[HalfLine<PZ>::M], const C *A, int c, int t, bool live, const YzDims &D) {
+    using H = HalfLine<PZ>;
+    ct_for<H::M>([&](auto k) {
+        const int z = t + H::T * k;
+        x[k] = live && z < D.Nz ? A[z * YzLine<PY>::LS + c] : czero<C>();
+    });
 }
-
-// chunk store: A[z][ky0 + l] = B[l][z] for z < Nz and ky0 + l < PY
 template <int PY, int PZ, typename C>
-SCD_HD void yz_zstore(int tid, C *A, const C *B, int ky0, const YzDims &D) {
-    constexpr int LSY = YzLine<PY>::LS, LSZ = YzLine<PZ>::LS, KC = YzLine<PZ>::LINES;
-    const int n = KC * ((D.Nz + 3) & ~3);
-    for (int e = tid; e < n; e += YZ_THREADS) {
-        int l, z;
-        yz_tile4(e, KC, l, z);
-        const int ky = ky0 + l;
-        if (ky < PY && z < D.Nz) A[z * LSY + pidx(ky)] = B[l * LSZ + pidx(z)];
-    }
+SCD_HD void yz_z_store(const C (&x)[HalfLine<PZ>::M], C *A, int c, int t, const YzDims &D) {
+    using H = HalfLine<PZ>;
+    ct_for<H::M>([&](auto k) {
+        const int z = t + H::T * k;
+        if (z < D.Nz) A[z * YzLine<PY>::LS + c] = x[k];
+    });
 }
-
-// the Green product of a chunk: B[l][kz] *= Fyz(fx, fold(ky), fold(kz)),
-// each line by its own TZ threads (thread t of line l = tid / TZ takes kz = t,
-// t + TZ, ...), so that the line's transforms before and after it need only
-// a warp synchronisation (a warp holds whole lines)
-template <int PY, int PZ, typename C>
-SCD_HD void yz_green(int tid, C *B, const C *Fyz, int fx, int ky0, const YzDims &D) {
-    constexpr int LSZ = YzLine<PZ>::LS, TZ = YzLine<PZ>::TPL;
-    const int l = tid / TZ, t = tid - l * TZ, ky = ky0 + l;
-    if (ky >= PY) return;
-    const C *Fr = Fyz + ((long long)fx * D.Hy + yz_fold(ky, PY)) * D.Hz;
-    for (int kz = t; kz < PZ; kz += TZ) B[l * LSZ + pidx(kz)] = cmul(Fr[yz_fold(kz, PZ)], B[l * LSZ + pidx(kz)]);
+// the Green values of thread t's part of a z line, Fr = the line's octant row
+template <int PZ, typename C>
+SCD_HD void yz_green_load(C (&f)[HalfLine<PZ>::PER][HalfLine<PZ>::T], const C *Fr, int t) {
+    using H = HalfLine<PZ>;
+    ct_for<H::PER>([&](auto p) { ct_for<H::T>([&](auto b) { f[p][b] = Fr[yz_fold(t * H::PER + p + H::N1 * b, PZ)]; }); });
 }
-
-// one line transform run on the host: every thread of the line, phase by
-// phase, as the warp does
-template <int P, bool INV, typename C>
-void yz_line_host(C *s, const C *tw) {
-    if constexpr (YzLine<P>::REG) {
-        constexpr int PER = RegFft<P>::PER;
-        C v[8][P / 8];
-        for (int t = 0; t < 8; ++t) regfft_A<P, INV>(s, tw, t, v[t]);
-        for (int t = 0; t < 8; ++t) regfft_A_store<P>(s, t, v[t]);
-        C u[8][PER][8];
-        for (int t = 0; t < 8; ++t) regfft_B<P, INV>(s, tw, t, u[t]);
-        for (int t = 0; t < 8; ++t) regfft_B_store<P>(s, t, u[t]);
-    } else {
-        constexpr int T = YzLine<P>::TPL, PER = MixFft<P, T>::PER;
-        C v[T][P / T];
-        for (int t = 0; t < T; ++t) mixfft_A<P, T, INV>(s, tw, t, v[t]);
-        for (int t = 0; t < T; ++t) mixfft_A_store<P, T>(s, t, v[t]);
-        C u[T][PER][T];
-        for (int t = 0; t < T; ++t) mixfft_B<P, T, INV>(s, tw, t, u[t]);
-        for (int t = 0; t < T; ++t) mixfft_B_store<P, T>(s, t, u[t]);
-    }
+template <int PZ, typename C>
+SCD_HD void yz_green_mul(C (&u)[HalfLine<PZ>::PER][HalfLine<PZ>::T], const C (&f)[HalfLine<PZ>::PER][HalfLine<PZ>::T]) {
+    using H = HalfLine<PZ>;
+    ct_for<H::PER>([&](auto p) { ct_for<H::T>([&](auto b) { u[p][b] = cmul(f[p][b], u[p][b]); }); });
 }
 
 // the whole fused pass of one plane on the host (x column x, grid rg): the
-// same phases, in the kernel's order, with the CTA's threads run in turn
+// same steps, line after line, the threads of a line in turn
 template <int PY, int PZ, typename C>
 void yz_plane_host(C *Wp, const C *Fyz, const C *twy, const C *twz, int x, const YzDims &D, C *smem) {
-    constexpr int LSY = YzLine<PY>::LS, LSZ = YzLine<PZ>::LS, KC = YzLine<PZ>::LINES;
-    C *A = smem + PY + PZ, *B = A + (long long)D.NzR * LSY;
-    for (int t = 0; t < YZ_THREADS; ++t) yz_load<PY>(t, A, Wp, D);
-    for (int l = 0; l < D.NzR; ++l) yz_line_host<PY, false>(A + l * LSY, twy);
-    const int fx = yz_fold(x, D.Px);
-    for (int ky0 = 0; ky0 < PY; ky0 += KC) {
-        for (int t = 0; t < YZ_THREADS; ++t) yz_zload<PY, PZ>(t, A, B, ky0, D);
-        for (int l = 0; l < KC; ++l) yz_line_host<PZ, false>(B + l * LSZ, twz);
-        for (int t = 0; t < YZ_THREADS; ++t) yz_green<PY, PZ>(t, B, Fyz, fx, ky0, D);
-        for (int l = 0; l < KC; ++l) yz_line_host<PZ, true>(B + l * LSZ, twz);
-        for (int t = 0; t < YZ_THREADS; ++t) yz_zstore<PY, PZ>(t, A, B, ky0, D);
+    using HY = HalfLine<PY>;
+    using HZ = HalfLine<PZ>;
+    C *A = smem + PY + PZ, *E = A + (long long)D.Nz * YzLine<PY>::LS;
+    for (int z = 0; z < D.Nz; ++z) {
+        C *e = E + (z % HY::LW) * HY::ES;
+        for (int t = 0; t < HY::T; ++t) {
+            C v[HY::M];
+            yz_y_load<PY>(v, Wp, z, t, true, D);
+            half_fwd_a<PY>(v, e, twy, t);
+        }
+        for (int t = 0; t < HY::T; ++t) {
+            C u[HY::PER][HY::T];
+            half_fwd_b<PY>(e, u, t);
+            yz_y_put<PY>(u, A, z, t);
+        }
     }
-    for (int l = 0; l < D.NzR; ++l) yz_line_host<PY, true>(A + l * LSY, twy);
-    for (int t = 0; t < YZ_THREADS; ++t) yz_store<PY>(t, A, Wp, D);
+    const int fx = yz_fold(x, D.Px);
+    for (int c = 0; c < PY; ++c) {
+        C *e = E + (c % HZ::LW) * HZ::ES;
+        static C u[HZ::T][HZ::PER][HZ::T];
+        for (int t = 0; t < HZ::T; ++t) {
+            C v[HZ::M];
+            yz_z_load<PY, PZ>(v, A, c, t, true, D);
+            half_fwd_a<PZ>(v, e, twz, t);
+        }
+        for (int t = 0; t < HZ::T; ++t) {
+            C f[HZ::PER][HZ::T];
+            half_fwd_b<PZ>(e, u[t], t);
+            yz_green_load<PZ>(f, Fyz + ((long long)fx * D.Hy + yz_fold(yz_ky<PY>(c), PY)) * D.Hz, t);
+            yz_green_mul<PZ>(u[t], f);
+        }
+        for (int t = 0; t < HZ::T; ++t) half_inv_b<PZ>(u[t], e, t);
+        for (int t = 0; t < HZ::T; ++t) {
+            C v[HZ::M];
+            half_inv_a<PZ>(e, twz, v, t);
+            yz_z_store<PY, PZ>(v, A, c, t, D);
+        }
+    }
+    for (int z = 0; z < D.Nz; ++z) {
+        C *e = E + (z % HY::LW) * HY::ES;
+        for (int t = 0; t < HY::T; ++t) {
+            C u[HY::PER][HY::T];
+            yz_y_get<PY>(u, A, z, t, true);
+            half_inv_b<PY>(u, e, t);
+        }
+        for (int t = 0; t < HY::T; ++t) {
+            C v[HY::M];
+            half_inv_a<PY>(e, twy, v, t);
+            yz_y_store<PY>(v, Wp, z, t, D);
+        }
+    }
 }
+
+// one launch of the fused pass (fft_yz_*.cu): nrg grids
+template <typename C> struct YzLaunch {
+    C *W;
+    const C *Fyz, *twy, *twz;
+    YzDims D;
+    const int *done;
+    int nrg;
+    cudaStream_t st;
+};
+template <int PY, typename C> void yz_launch(const YzLaunch<C> &l, int Pz);
 
 #ifdef __CUDACC__
-template <int P, bool INV, typename C>
-__device__ __forceinline__ void yz_line_dev(C *s, const C *tw, int t) {
-    if constexpr (YzLine<P>::REG) fft_line_reg<P, INV, C>(s, tw, t);
-    else fft_line_mixed<P, YzLine<P>::TPL, INV, C>(s, tw, t);
-}
-
-// the NzR y lines of the plane, LINES per round; a warp's lines are all
-// below NzR or all above it (NzR and the lines per warp are multiples of
-// 8 and 4), so the warp-synchronous transform is never split
-template <int PY, bool INV, typename C>
-__device__ __forceinline__ void yz_ylines_dev(C *A, const C *tw, int NzR) {
-    constexpr int TPL = YzLine<PY>::TPL, LS = YzLine<PY>::LS, LINES = YzLine<PY>::LINES;
-    const int tid = threadIdx.x;
-    for (int l0 = 0; l0 < NzR; l0 += LINES) {
-        const int l = l0 + tid / TPL;
-        if (l < NzR) yz_line_dev<PY, INV, C>(A + l * LS, tw, tid % TPL);
-    }
-}
-
 // one CTA per (x, rg): grid (Px, 4 nrhs); dynamic shared memory
-// yz_smem_elems<PY, PZ>(NzR) elements of C
+// yz_smem_elems<PY, PZ>(Nz, threads) elements of C
 template <int PY, int PZ, typename C>
-__global__ void __launch_bounds__(YZ_THREADS)
+__global__ void __launch_bounds__(YZ_THREADS, sizeof(C) == 8 ? 2 : 1)
 k_fft_yz(C *__restrict__ Wt, const C *__restrict__ Fyz, const C *__restrict__ twy_g, const C *__restrict__ twz_g,
          YzDims D, const int *done) {
     const int x = blockIdx.x, rg = blockIdx.y;
     if (done && done[rg >> 2]) return;
-    constexpr int LSY = YzLine<PY>::LS, LSZ = YzLine<PZ>::LS, KC = YzLine<PZ>::LINES, TZ = YzLine<PZ>::TPL;
+    using HY = HalfLine<PY>;
+    using HZ = HalfLine<PZ>;
     extern __shared__ __align__(16) unsigned char yz_raw[];
-    C *twy = reinterpret_cast<C *>(yz_raw), *twz = twy + PY, *A = twz + PZ, *B = A + D.NzR * LSY;
-    const int tid = threadIdx.x;
-    for (int i = tid; i < PY; i += YZ_THREADS) twy[i] = twy_g[i];
-    for (int i = tid; i < PZ; i += YZ_THREADS) twz[i] = twz_g[i];
+    C *twy = reinterpret_cast<C *>(yz_raw), *twz = twy + PY, *A = twz + PZ;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    C *E = A + D.Nz * YzLine<PY>::LS + warp * yz_ex<PY, PZ>();
+    for (int i = threadIdx.x; i < PY; i += blockDim.x) twy[i] = twy_g[i];
+    for (int i = threadIdx.x; i < PZ; i += blockDim.x) twz[i] = twz_g[i];
     C *Wp = Wt + ((long long)rg * D.Px + x) * D.Nz * D.Ny;
-    yz_load<PY>(tid, A, Wp, D);
+    const int ty = half_t<PY>(lane), ly = half_l<PY>(lane), tz = half_t<PZ>(lane), lz = half_l<PZ>(lane);
     __syncthreads();
-    yz_ylines_dev<PY, false>(A, twy, D.NzR);
-    __syncthreads();
-    const int fx = yz_fold(x, D.Px);
-    for (int ky0 = 0; ky0 < PY; ky0 += KC) {
-        yz_zload<PY, PZ>(tid, A, B, ky0, D);
-        __syncthreads();
-        yz_line_dev<PZ, false, C>(B + (tid / TZ) * LSZ, twz, tid % TZ);
-        __syncwarp();   // a warp holds whole lines (YZ_THREADS / TZ lines, 32 / TZ per warp)
-        yz_green<PY, PZ>(tid, B, Fyz, fx, ky0, D);
+    for (int z0 = warp * HY::LW; z0 < D.Nz; z0 += nw * HY::LW) {
+        const int z = z0 + ly;
+        const bool live = z < D.Nz;
+        C *e = E + ly * HY::ES;
+        {
+            C v[HY::M];
+            yz_y_load<PY>(v, Wp, z, ty, live, D);
+            half_fwd_a<PY>(v, e, twy, ty);
+        }
         __syncwarp();
-        yz_line_dev<PZ, true, C>(B + (tid / TZ) * LSZ, twz, tid % TZ);
-        __syncthreads();
-        yz_zstore<PY, PZ>(tid, A, B, ky0, D);
-        __syncthreads();
+        C u[HY::PER][HY::T];
+        half_fwd_b<PY>(e, u, ty);
+        if (live) yz_y_put<PY>(u, A, z, ty);
+        __syncwarp();
     }
-    yz_ylines_dev<PY, true>(A, twy, D.NzR);
     __syncthreads();
-    yz_store<PY>(tid, A, Wp, D);
+    const C *Fx = Fyz + (long long)yz_fold(x, D.Px) * D.Hy * D.Hz;
+    for (int c0 = warp * HZ::LW; c0 < PY; c0 += nw * HZ::LW) {
+        const bool live = c0 + lz < PY;
+        const int c = min(c0 + lz, PY - 1);
+        C *e = E + lz * HZ::ES;
+        {
+            C v[HZ::M];
+            yz_z_load<PY, PZ>(v, A, c, tz, live, D);
+            half_fwd_a<PZ>(v, e, twz, tz);
+        }
+        C u[HZ::PER][HZ::T], f[HZ::PER][HZ::T];
+        yz_green_load<PZ>(f, Fx + yz_fold(yz_ky<PY>(c), PY) * D.Hz, tz);
+        __syncwarp();
+        half_fwd_b<PZ>(e, u, tz);
+        yz_green_mul<PZ>(u, f);
+        __syncwarp();
+        half_inv_b<PZ>(u, e, tz);
+        __syncwarp();
+        C v[HZ::M];
+        half_inv_a<PZ>(e, twz, v, tz);
+        if (live) yz_z_store<PY, PZ>(v, A, c, tz, D);
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int z0 = warp * HY::LW; z0 < D.Nz; z0 += nw * HY::LW) {
+        const int z = z0 + ly;
+        const bool live = z < D.Nz;
+        C *e = E + ly * HY::ES;
+        {
+            C u[HY::PER][HY::T];
+            yz_y_get<PY>(u, A, z, ty, live);
+            half_inv_b<PY>(u, e, ty);
+        }
+        __syncwarp();
+        C v[HY::M];
+        half_inv_a<PY>(e, twy, v, ty);
+        if (live) yz_y_store<PY>(v, Wp, z, ty, D);
+        __syncwarp();
+    }
+}
+
+// Threads of a CTA: the count (128 or 256) that keeps more warps on an SM for
+// the plane's size, 128 if both do (its lines fill the warps better on small
+// planes).
+template <int PY, int PZ, typename C>
+void yz_launch_t(const YzLaunch<C> &l) {
+    auto bytes = [&](int threads) { return sizeof(C) * (size_t)yz_smem_elems<PY, PZ>(l.D.Nz, threads); };
+    auto warps = [&](int threads) { return (int)std::min<size_t>((size_t)227 * 1024 / (bytes(threads) + 1024), 512 / threads) * threads; };
+    const int threads = warps(256) > warps(128) ? 256 : 128;
+    const size_t sh = bytes(threads);
+    cudaFuncSetAttribute(k_fft_yz<PY, PZ, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+    k_fft_yz<PY, PZ, C><<<dim3(l.D.Px, l.nrg), threads, sh, l.st>>>(l.W, l.Fyz, l.twy, l.twz, l.D, l.done);
 }
 
 // Fyz[(fx Hy + fy) Hz + fz] = Fo[(fz Hy + fy) Hx + fx]

@@ -15,7 +15,6 @@
 #include <type_traits>
 
 #include "ctx.h"
-#include "fft_mixed.cuh"
 #include "fft_reg.cuh"
 #include "fft_yz.cuh"
 #include "linear_basis.h"
@@ -277,37 +276,14 @@ __device__ __forceinline__ void fft_line(C *s, const C *tw, int t) {
     }
 }
 
-// Line FFT of the passes: register-resident 8-thread transform for P = 64
-// and 128 (fft_reg.cuh), register-resident mixed-radix transform with 4 or 8
-// threads for the 5-smooth lengths below (fft_mixed.cuh), shared-memory
-// radix-4 Stockham for other powers of two.
-// (N1 = P / threads <= 24 keeps the FP64 transforms within the register file)
-template <int P> constexpr bool fft_mixed_len() { return P == 80 || P == 96 || P == 192; }
-// lines per CTA halved until the line buffers fit 44 KB of static shared memory
-constexpr int fft_fit_lpb(int lpb, int ls, int es) { return (lpb > 1 && lpb * ls * es > 44 * 1024) ? fft_fit_lpb(lpb / 2, ls, es) : lpb; }
+// Lines per CTA of the shared-memory radix-4 transform, for the powers of two
+// without a half-full line transform (fft_line.cuh): 8, 256 and 512.
 template <int P, typename Cx> struct FftCfg {
-    static constexpr bool REG = P == 64 || P == 128;
-    static constexpr bool MIX = !REG && fft_mixed_len<P>();
     static constexpr int LS = P + (P >> 4) + 1;              // padded line stride (bank spread)
-    static constexpr int TPL = REG ? 8 : MIX ? (P % 64 == 0 ? 8 : 4) : P / 4;   // threads per line
-    static constexpr int LPB = REG ? (sizeof(Cx) == 16 ? 16 : 32)
-                               : MIX ? fft_fit_lpb(256 / TPL / (sizeof(Cx) == 16 ? 2 : 1), LS, (int)sizeof(Cx))
-                                     : ((256 / TPL) > 0 ? 256 / TPL : 1);   // lines per CTA
+    static constexpr int TPL = P / 4;                        // threads per line
+    static constexpr int LPB = 256 / TPL > 0 ? 256 / TPL : 1;
     static constexpr int THREADS = TPL * LPB;
 };
-
-template <int P, bool INV, typename Cx>
-__device__ __forceinline__ void fft_line_any(Cx *s, const Cx *tw, int t) {
-    if constexpr (FftCfg<P, Cx>::REG) {
-        fft_line_reg<P, INV, Cx>(s, tw, t);
-        __syncthreads();   // the passes' next loops read every line of the CTA
-    } else if constexpr (FftCfg<P, Cx>::MIX) {
-        fft_line_mixed<P, FftCfg<P, Cx>::TPL, INV, Cx>(s, tw, t);
-        __syncthreads();
-    } else {
-        fft_line<P, INV, Cx>(s, tw, t);
-    }
-}
 
 struct GridDims {
     int Nx, Ny, Nz, Px, Py, Pz, Hx, Hy, Hz, ncx, ncy, ncz, ncubes;
@@ -369,7 +345,7 @@ k_fft_x_fwd(const Cx *__restrict__ bpart, Cx *__restrict__ W, const Cx *__restri
     }
     __syncthreads();
     const int l = threadIdx.x / Cf::TPL, t = threadIdx.x - l * Cf::TPL;
-    fft_line_any<P, false, Cx>(sh + l * Cf::LS, tw, t);
+    fft_line<P, false, Cx>(sh + l * Cf::LS, tw, t);
     if constexpr (TL) {
         Cx *Wr = W + (long long)rg * P * nlines;
         for (int e = threadIdx.x; e < Cf::LPB * P; e += blockDim.x) {
@@ -386,6 +362,186 @@ k_fft_x_fwd(const Cx *__restrict__ bpart, Cx *__restrict__ W, const Cx *__restri
             }
         }
     }
+}
+
+// The passes for the lengths of fft_line.cuh, 128 threads (64 where four warps'
+// exchange buffers exceed static shared memory), lines in registers; the
+// three-pass chain forms its lines as the fused pass does (the same bits).  X
+// forward: thread t of line (y, z) assembles its nodes x = t + T k < Nx from
+// the box partial sums -- the up to four boxes of (y, z) once per line, the
+// one or two of x per node, in node_value's order -- and writes the layouts of
+// k_fft_x_fwd.  Bound by the latency of the box reads: 32
+// complex64 right-hand sides of a 46 x 40 x 28 grid take 107 us (166 with each
+// node's boxes found by itself and lines in shared memory).
+template <int P, typename Cx>
+constexpr int XP_THREADS = (P + 4 * HalfLine<P>::EW) * sizeof(Cx) <= 48 * 1024 ? 128 : 64;
+template <int P, typename Cx, bool TL>
+__global__ void __launch_bounds__(XP_THREADS<P, Cx>)
+k_fft_x_fwd_line(const Cx *__restrict__ bpart, Cx *__restrict__ W, const Cx *__restrict__ twg, GridDims G, const int *done) {
+    if (done && done[blockIdx.y >> 2]) return;
+    using H = HalfLine<P>;
+    __shared__ Cx tw[P], ex[(XP_THREADS<P, Cx> / 32) * H::EW];
+    const int rg = blockIdx.y, g = rg & 3, r = rg >> 2, nlines = G.Ny * G.Nz;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = half_t<P>(lane), l = half_l<P>(lane);
+    for (int i = threadIdx.x; i < P; i += XP_THREADS<P, Cx>) tw[i] = twg[i];
+    const int line = (blockIdx.x * (XP_THREADS<P, Cx> / 32) + warp) * H::LW + l;
+    const bool live = line < nlines;
+    const int y = live ? line % G.Ny : 0, z = live ? line / G.Ny : 0;
+    const Cx *bp = bpart + (long long)r * G.ncubes * 108 + g * 27;
+    // offsets of the (y, z) boxes' node rows, z the slower: box b of an axis
+    // holds node b 2 + a; even nodes also belong to box b - 1 as its node 2
+    int row[4];
+    bool in[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int dz = q >> 1, dy = q & 1, bz = (z >> 1) - dz, by = (y >> 1) - dy;
+        const int az = dz ? 2 : z & 1, ay = dy ? 2 : y & 1;
+        in[q] = live && bz >= 0 && bz < G.ncz && by >= 0 && by < G.ncy && !(dz && (z & 1)) && !(dy && (y & 1));
+        row[q] = in[q] ? G.ncx * (by + G.ncy * bz) * 108 + 3 * ay + 9 * az : 0;
+    }
+    __syncthreads();
+    Cx *e = ex + warp * H::EW + l * H::ES;
+    {
+        Cx v[H::M];
+        ct_for<H::M>([&](auto k) {
+            const int x = t + H::T * k, b = x >> 1;
+            const bool lo = x < G.Nx && b < G.ncx, hi = x < G.Nx && !(x & 1) && b >= 1 && b - 1 < G.ncx;
+            Cx s = czero<Cx>();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (in[q] && lo) s = cadd(s, bp[row[q] + 108 * b + (x & 1)]);
+                if (in[q] && hi) s = cadd(s, bp[row[q] + 108 * (b - 1) + 2]);
+            }
+            v[k] = s;
+        });
+        half_fwd_a<P>(v, e, tw, t);
+    }
+    __syncwarp();
+    Cx u[H::PER][H::T];
+    half_fwd_b<P>(e, u, t);
+    Cx *Wr = TL ? W + (long long)rg * P * nlines + line : W + ((long long)rg * G.Nz + z) * G.Py * P + (long long)y * P;
+    const long long step = TL ? nlines : 1;
+    if (live)
+        ct_for<H::PER>([&](auto p) {
+            ct_for<H::T>([&](auto b) { Wr[(t * H::PER + p + H::N1 * b) * step] = u[p][b]; });
+        });
+}
+// inverse: R[(rg)][(z*Ny + y)*Nx + x], x < Nx
+template <int P, typename Cx, bool TL>
+__global__ void __launch_bounds__(XP_THREADS<P, Cx>)
+k_fft_x_inv_line(const Cx *__restrict__ W, Cx *__restrict__ R, const Cx *__restrict__ twg, GridDims G, const int *done) {
+    if (done && done[blockIdx.y >> 2]) return;
+    using H = HalfLine<P>;
+    __shared__ Cx tw[P], ex[(XP_THREADS<P, Cx> / 32) * H::EW];
+    const int rg = blockIdx.y, nlines = G.Ny * G.Nz;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = half_t<P>(lane), l = half_l<P>(lane);
+    for (int i = threadIdx.x; i < P; i += XP_THREADS<P, Cx>) tw[i] = twg[i];
+    const int line = (blockIdx.x * (XP_THREADS<P, Cx> / 32) + warp) * H::LW + l;
+    const bool live = line < nlines;
+    Cx *e = ex + warp * H::EW + l * H::ES;
+    {
+        Cx u[H::PER][H::T];
+        const int y = line % G.Ny, z = line / G.Ny;
+        const Cx *Wr = TL ? W + (long long)rg * P * nlines + line : W + ((long long)rg * G.Nz + z) * G.Py * P + (long long)y * P;
+        const long long step = TL ? nlines : 1;
+        ct_for<H::PER>([&](auto p) {
+            ct_for<H::T>([&](auto b) { u[p][b] = live ? Wr[(t * H::PER + p + H::N1 * b) * step] : czero<Cx>(); });
+        });
+        half_inv_b<P>(u, e, t);
+    }
+    __syncthreads();
+    Cx v[H::M];
+    half_inv_a<P>(e, tw, v, t);
+    Cx *Rr = R + ((long long)rg * nlines + line) * G.Nx;
+    if (live)
+        ct_for<H::M>([&](auto k) {
+            const int x = t + H::T * k;
+            if (x < G.Nx) Rr[x] = v[k];
+        });
+}
+
+// y and z passes of the three-pass chain on W[rg][z][y][x], lines of
+// consecutive x.  A line is read whole before it is written.
+template <int P, bool INV, typename Cx>
+__global__ void __launch_bounds__(XP_THREADS<P, Cx>)
+k_fft_y_line(Cx *__restrict__ W, const Cx *__restrict__ twg, GridDims G, const int *done) {
+    if (done && done[blockIdx.y >> 2]) return;
+    using H = HalfLine<P>;
+    __shared__ Cx tw[P], ex[(XP_THREADS<P, Cx> / 32) * H::EW];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = half_t<P>(lane), l = half_l<P>(lane);
+    for (int i = threadIdx.x; i < P; i += XP_THREADS<P, Cx>) tw[i] = twg[i];
+    const int line = (blockIdx.x * (XP_THREADS<P, Cx> / 32) + warp) * H::LW + l;
+    const bool live = line < G.Px * G.Nz;
+    const int z = live ? line / G.Px : 0, x = live ? line - z * G.Px : 0;
+    Cx *Wr = W + (((long long)blockIdx.y * G.Nz + z) * P) * G.Px + x;
+    Cx *e = ex + warp * H::EW + l * H::ES;
+    __syncthreads();
+    if constexpr (!INV) {
+        Cx v[H::M], u[H::PER][H::T];
+        ct_for<H::M>([&](auto k) {
+            const int y = t + H::T * k;
+            v[k] = live && y < G.Ny ? Wr[(long long)y * G.Px] : czero<Cx>();
+        });
+        half_fwd_a<P>(v, e, tw, t);
+        __syncwarp();
+        half_fwd_b<P>(e, u, t);
+        if (live)
+            ct_for<H::PER>([&](auto p) {
+                ct_for<H::T>([&](auto b) { Wr[(long long)(t * H::PER + p + H::N1 * b) * G.Px] = u[p][b]; });
+            });
+    } else {
+        Cx v[H::M], u[H::PER][H::T];
+        ct_for<H::PER>([&](auto p) {
+            ct_for<H::T>([&](auto b) { u[p][b] = live ? Wr[(long long)(t * H::PER + p + H::N1 * b) * G.Px] : czero<Cx>(); });
+        });
+        half_inv_b<P>(u, e, t);
+        __syncwarp();
+        half_inv_a<P>(e, tw, v, t);
+        if (live)
+            ct_for<H::M>([&](auto k) {
+                const int y = t + H::T * k;
+                if (y < G.Ny) Wr[(long long)y * G.Px] = v[k];
+            });
+    }
+}
+template <int P, typename Cx>
+__global__ void __launch_bounds__(XP_THREADS<P, Cx>)
+k_fft_z_line(Cx *__restrict__ W, const Cx *__restrict__ Fo, const Cx *__restrict__ twg, GridDims G, const int *done) {
+    if (done && done[blockIdx.y >> 2]) return;
+    using H = HalfLine<P>;
+    __shared__ Cx tw[P], ex[(XP_THREADS<P, Cx> / 32) * H::EW];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = half_t<P>(lane), l = half_l<P>(lane);
+    for (int i = threadIdx.x; i < P; i += XP_THREADS<P, Cx>) tw[i] = twg[i];
+    const int line = (blockIdx.x * (XP_THREADS<P, Cx> / 32) + warp) * H::LW + l;
+    const bool live = line < G.Px * G.Py;
+    const int y = live ? line / G.Px : 0, x = live ? line - y * G.Px : 0;
+    const long long plane = (long long)G.Px * G.Py;
+    Cx *Wr = W + (long long)blockIdx.y * plane * G.Nz + (long long)y * G.Px + x;
+    const Cx *Fr = Fo + (long long)fold(y, G.Py) * G.Hx + fold(x, G.Px);
+    Cx *e = ex + warp * H::EW + l * H::ES;
+    Cx v[H::M], u[H::PER][H::T];
+    __syncthreads();
+    ct_for<H::M>([&](auto k) {
+        const int z = t + H::T * k;
+        v[k] = live && z < G.Nz ? Wr[z * plane] : czero<Cx>();
+    });
+    half_fwd_a<P>(v, e, tw, t);
+    __syncwarp();
+    half_fwd_b<P>(e, u, t);
+    ct_for<H::PER>([&](auto p) {
+        ct_for<H::T>([&](auto b) {
+            u[p][b] = cmul(__ldg(&Fr[(long long)fold(t * H::PER + p + H::N1 * b, P) * G.Hy * G.Hx]), u[p][b]);
+        });
+    });
+    __syncwarp();
+    half_inv_b<P>(u, e, t);
+    __syncwarp();
+    half_inv_a<P>(e, tw, v, t);
+    if (live)
+        ct_for<H::M>([&](auto k) {
+            const int z = t + H::T * k;
+            if (z < G.Nz) Wr[z * plane] = v[k];
+        });
 }
 
 // Y pass: lines (x < Px, z < Nz); forward reads y < Ny and writes y < Py,
@@ -412,7 +568,7 @@ k_fft_y(Cx *__restrict__ W, const Cx *__restrict__ twg, GridDims G, const int *d
     }
     __syncthreads();
     const int l = threadIdx.x / Cf::TPL, t = threadIdx.x - l * Cf::TPL;
-    fft_line_any<P, INV, Cx>(sh + l * Cf::LS, tw, t);
+    fft_line<P, INV, Cx>(sh + l * Cf::LS, tw, t);
     for (int e = threadIdx.x; e < Cf::LPB * P; e += blockDim.x) {
         const int y = e / Cf::LPB, ll = e - y * Cf::LPB, x = x0 + ll;
         if (y < nout && x < G.Px) Wr[(long long)y * G.Px + x] = sh[ll * Cf::LS + pidx(y)];
@@ -442,7 +598,7 @@ k_fft_z(Cx *__restrict__ W, const Cx *__restrict__ Fo, const Cx *__restrict__ tw
     }
     __syncthreads();
     const int l = threadIdx.x / Cf::TPL, t = threadIdx.x - l * Cf::TPL;
-    fft_line_any<P, false, Cx>(sh + l * Cf::LS, tw, t);
+    fft_line<P, false, Cx>(sh + l * Cf::LS, tw, t);
     const int fy = fold(y, G.Py);
     // consecutive threads take consecutive lines (x), so the octant reads of
     // one z plane are contiguous
@@ -454,7 +610,7 @@ k_fft_z(Cx *__restrict__ W, const Cx *__restrict__ Fo, const Cx *__restrict__ tw
         }
     }
     __syncthreads();
-    fft_line_any<P, true, Cx>(sh + l * Cf::LS, tw, t);
+    fft_line<P, true, Cx>(sh + l * Cf::LS, tw, t);
     for (int e = threadIdx.x; e < Cf::LPB * P; e += blockDim.x) {
         const int z = e / Cf::LPB, ll = e - z * Cf::LPB, x = x0 + ll;
         if (z < G.Nz && x < G.Px) Wr[(long long)z * plane + x] = sh[ll * Cf::LS + pidx(z)];
@@ -495,7 +651,7 @@ k_fft_x_inv(const Cx *__restrict__ W, Cx *__restrict__ R, const Cx *__restrict__
     }
     __syncthreads();
     const int l = threadIdx.x / Cf::TPL, t = threadIdx.x - l * Cf::TPL;
-    fft_line_any<P, true, Cx>(sh + l * Cf::LS, tw, t);
+    fft_line<P, true, Cx>(sh + l * Cf::LS, tw, t);
     Cx *Rr = R + (long long)rg * G.Nx * G.Ny * G.Nz;
     for (int e = threadIdx.x; e < Cf::LPB * P; e += blockDim.x) {
         const int ll = e / P, x = e - ll * P, line = line0 + ll;
@@ -1259,88 +1415,97 @@ template <> struct Res<cf> {
     static cf *xT(scd_ctx *c) { return c->f_xT; }
 };
 
+// CTAs of a line kernel over n lines
+template <int P, typename C> dim3 line_grid(int n, int nrg) {
+    constexpr int per = XP_THREADS<P, C> / 32 * HalfLine<P>::LW;
+    return dim3((n + per - 1) / per, nrg);
+}
 template <int P, typename C>
 void fft_x_fwd_t(scd_ctx *c, const GridDims &G, int nrg, const int *done, const C *tw, bool tl) {
-    using Cf = FftCfg<P, C>;
-    dim3 grid((G.Ny * G.Nz + Cf::LPB - 1) / Cf::LPB, nrg);
-    if (tl) k_fft_x_fwd<P, C, true><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::bpart(c), Res<C>::W(c), tw, G, done);
-    else k_fft_x_fwd<P, C, false><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::bpart(c), Res<C>::W(c), tw, G, done);
+    if constexpr (half_len(P)) {
+        const dim3 grid = line_grid<P, C>(G.Ny * G.Nz, nrg);
+        if (tl) k_fft_x_fwd_line<P, C, true><<<grid, XP_THREADS<P, C>, 0, c->st>>>(Res<C>::bpart(c), Res<C>::W(c), tw, G, done);
+        else k_fft_x_fwd_line<P, C, false><<<grid, XP_THREADS<P, C>, 0, c->st>>>(Res<C>::bpart(c), Res<C>::W(c), tw, G, done);
+    } else {
+        using Cf = FftCfg<P, C>;
+        dim3 grid((G.Ny * G.Nz + Cf::LPB - 1) / Cf::LPB, nrg);
+        if (tl) k_fft_x_fwd<P, C, true><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::bpart(c), Res<C>::W(c), tw, G, done);
+        else k_fft_x_fwd<P, C, false><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::bpart(c), Res<C>::W(c), tw, G, done);
+    }
 }
 template <int P, bool INV, typename C>
 void fft_y_t(scd_ctx *c, const GridDims &G, int nrg, const int *done, const C *tw) {
-    using Cf = FftCfg<P, C>;
-    dim3 grid(((G.Px + Cf::LPB - 1) / Cf::LPB) * G.Nz, nrg);
-    k_fft_y<P, INV, C><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::W(c), tw, G, done);
+    if constexpr (half_len(P)) {
+        k_fft_y_line<P, INV, C><<<line_grid<P, C>(G.Px * G.Nz, nrg), XP_THREADS<P, C>, 0, c->st>>>(Res<C>::W(c), tw, G, done);
+    } else {
+        using Cf = FftCfg<P, C>;
+        dim3 grid(((G.Px + Cf::LPB - 1) / Cf::LPB) * G.Nz, nrg);
+        k_fft_y<P, INV, C><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::W(c), tw, G, done);
+    }
 }
 template <int P, typename C>
 void fft_z_t(scd_ctx *c, const GridDims &G, int nrg, const int *done, const C *tw) {
-    using Cf = FftCfg<P, C>;
-    dim3 grid(((G.Px + Cf::LPB - 1) / Cf::LPB) * G.Py, nrg);
-    k_fft_z<P, C><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::W(c), Res<C>::Fo(c), tw, G, done);
+    if constexpr (half_len(P)) {
+        k_fft_z_line<P, C><<<line_grid<P, C>(G.Px * G.Py, nrg), XP_THREADS<P, C>, 0, c->st>>>(Res<C>::W(c), Res<C>::Fo(c), tw, G, done);
+    } else {
+        using Cf = FftCfg<P, C>;
+        dim3 grid(((G.Px + Cf::LPB - 1) / Cf::LPB) * G.Py, nrg);
+        k_fft_z<P, C><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::W(c), Res<C>::Fo(c), tw, G, done);
+    }
 }
 template <int P, typename C>
 void fft_x_inv_t(scd_ctx *c, const GridDims &G, int nrg, const int *done, const C *tw, bool tl) {
-    using Cf = FftCfg<P, C>;
-    dim3 grid((G.Ny * G.Nz + Cf::LPB - 1) / Cf::LPB, nrg);
-    if (tl) k_fft_x_inv<P, C, true><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::W(c), Res<C>::R(c), tw, G, done);
-    else k_fft_x_inv<P, C, false><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::W(c), Res<C>::R(c), tw, G, done);
-}
-
-// the fused y-z pass (fft_yz.cuh) for one (PY, PZ) pair
-template <int PY, int PZ, typename C>
-void fft_yz_t(scd_ctx *c, const GridDims &G, int nrg, const int *done) {
-    if constexpr (YzLine<PY>::OK && YzLine<PZ>::OK) {
-        YzDims D;
-        D.Nx = G.Nx; D.Ny = G.Ny; D.Nz = G.Nz; D.NzR = yz_round8(G.Nz);
-        D.Px = G.Px; D.Hx = G.Hx; D.Hy = G.Hy; D.Hz = G.Hz;
-        const size_t sh = sizeof(C) * (size_t)yz_smem_elems<PY, PZ>(D.NzR);
-        cudaFuncSetAttribute(k_fft_yz<PY, PZ, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-        k_fft_yz<PY, PZ, C><<<dim3(G.Px, nrg), YZ_THREADS, sh, c->st>>>(Res<C>::W(c), Res<C>::Fyz(c), Res<C>::tw(c, 1),
-                                                                       Res<C>::tw(c, 2), D, done);
+    if constexpr (half_len(P)) {
+        const dim3 grid = line_grid<P, C>(G.Ny * G.Nz, nrg);
+        if (tl) k_fft_x_inv_line<P, C, true><<<grid, XP_THREADS<P, C>, 0, c->st>>>(Res<C>::W(c), Res<C>::R(c), tw, G, done);
+        else k_fft_x_inv_line<P, C, false><<<grid, XP_THREADS<P, C>, 0, c->st>>>(Res<C>::W(c), Res<C>::R(c), tw, G, done);
+    } else {
+        using Cf = FftCfg<P, C>;
+        dim3 grid((G.Ny * G.Nz + Cf::LPB - 1) / Cf::LPB, nrg);
+        if (tl) k_fft_x_inv<P, C, true><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::W(c), Res<C>::R(c), tw, G, done);
+        else k_fft_x_inv<P, C, false><<<grid, Cf::THREADS, 0, c->st>>>(Res<C>::W(c), Res<C>::R(c), tw, G, done);
     }
 }
 
-template <int PY, typename C>
-void fft_yz_pz(scd_ctx *c, const GridDims &G, int nrg, const int *done) {
-    switch (G.Pz) {
-        case 64: fft_yz_t<PY, 64, C>(c, G, nrg, done); break;
-        case 80: fft_yz_t<PY, 80, C>(c, G, nrg, done); break;
-        case 96: fft_yz_t<PY, 96, C>(c, G, nrg, done); break;
-        case 128: fft_yz_t<PY, 128, C>(c, G, nrg, done); break;
-        case 192: fft_yz_t<PY, 192, C>(c, G, nrg, done); break;
-        default: break;
-    }
-}
-
+// the fused y-z pass (fft_yz.cuh)
 template <typename C>
 void fft_yz(scd_ctx *c, const GridDims &G, int nrg, const int *done) {
+    YzLaunch<C> l;
+    l.W = Res<C>::W(c); l.Fyz = Res<C>::Fyz(c); l.twy = Res<C>::tw(c, 1); l.twz = Res<C>::tw(c, 2);
+    l.D.Nx = G.Nx; l.D.Ny = G.Ny; l.D.Nz = G.Nz; l.D.NzR = yz_round8(G.Nz);
+    l.D.Px = G.Px; l.D.Hx = G.Hx; l.D.Hy = G.Hy; l.D.Hz = G.Hz;
+    l.done = done; l.nrg = nrg; l.st = c->st;
     switch (G.Py) {
-        case 64: fft_yz_pz<64, C>(c, G, nrg, done); break;
-        case 80: fft_yz_pz<80, C>(c, G, nrg, done); break;
-        case 96: fft_yz_pz<96, C>(c, G, nrg, done); break;
-        case 128: fft_yz_pz<128, C>(c, G, nrg, done); break;
-        case 192: fft_yz_pz<192, C>(c, G, nrg, done); break;
+        case 16: yz_launch<16>(l, G.Pz); break;
+        case 32: yz_launch<32>(l, G.Pz); break;
+        case 40: yz_launch<40>(l, G.Pz); break;
+        case 48: yz_launch<48>(l, G.Pz); break;
+        case 64: yz_launch<64>(l, G.Pz); break;
+        case 80: yz_launch<80>(l, G.Pz); break;
+        case 96: yz_launch<96>(l, G.Pz); break;
+        case 112: yz_launch<112>(l, G.Pz); break;
+        case 128: yz_launch<128>(l, G.Pz); break;
+        case 192: yz_launch<192>(l, G.Pz); break;
         default: break;
     }
 }
 
-constexpr bool yz_len_ok(int P) { return P == 64 || P == 80 || P == 96 || P == 128 || P == 192; }
-
-// shared-memory bytes of the fused y-z pass for the context's lengths
+// least shared memory of the fused y-z pass for the context's lengths (CTAs of
+// 128 threads): the sum of fft_yz.cuh's yz_smem_elems
 template <typename C>
 size_t yz_smem_bytes(const scd_ctx *c) {
-    const int NzR = yz_round8(c->Nz);
-    auto tpl = [](int P) { return (P == 64 || P == 128 || P % 64 == 0) ? 8 : 4; };
-    auto lines = [&](int P) { return YZ_THREADS / tpl(P); };
-    auto ls = [&](int P) { return yz_line_stride(P, tpl(P)); };
-    return sizeof(C) * (size_t)(c->Py + c->Pz + (long long)NzR * ls(c->Py) + (long long)lines(c->Pz) * ls(c->Pz));
+    auto ex = [](int P) {
+        const int T = P == 40 ? 2 : P % 64 == 0 ? 8 : 4;
+        return 32 / T * (T * half_row(P / T, T) + 1);
+    };
+    return sizeof(C) * ((size_t)c->Py + c->Pz + (size_t)c->Nz * ((c->Py + 7) / 8 * 8 + 4) + 4 * (size_t)std::max(ex(c->Py), ex(c->Pz)));
 }
 
 // whether the complex64 (or FP64) chain takes the fused y-z pass: both lengths
 // have warp-synchronous line transforms and the CTA fits shared memory
 template <typename C>
 bool use_yz(const scd_ctx *c) {
-    if (!c->yz_on || !yz_len_ok(c->Py) || !yz_len_ok(c->Pz)) return false;
+    if (!c->yz_on || !half_len(c->Py) || !half_len(c->Pz)) return false;
     return yz_smem_bytes<C>(c) <= (size_t)(227 * 1024);
 }
 
@@ -1389,7 +1554,10 @@ int rhs_span(const scd_ctx *c, int tuned, int nrhs, int items, int unit, int per
         case 32: CALL(32); break;                    \
         case 64: CALL(64); break;                    \
         case 128: CALL(128); break;                  \
+        case 40: CALL(40); break;                    \
+        case 48: CALL(48); break;                    \
         case 80: CALL(80); break;                    \
+        case 112: CALL(112); break;                  \
         case 96: CALL(96); break;                    \
         case 192: CALL(192); break;                  \
         case 256: CALL(256); break;                  \
