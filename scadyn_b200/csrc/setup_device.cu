@@ -23,6 +23,7 @@
 #include "ctx.h"
 #include "geom.cuh"
 #include "lin_setup.cuh"
+#include "near_pair.cuh"
 
 namespace {
 
@@ -62,228 +63,25 @@ __device__ __forceinline__ void face_of(const V3 *t, int f, V3 *tri) {
 // Gr (src/common.f90:271-279): exp(ikR) / (4 pi R)
 __device__ __forceinline__ cd green(V3 rf, V3 rp, double k) { return green_hd(rf, rp, k); }
 
-// analytical_integration, src/singularity_subtraction.f90:15-108: the
-// integrals of 1/R and R over a triangle (Np = 2)
-__device__ void analytic_tri(const V3 *tri, V3 n, V3 r, double &K1, double &K2) {
-    const double w0 = vdot(vsub(r, tri[0]), n);
-    double tl[3], Il[3];
-    double Km1 = 0.0;
-    // edges l = 1..3: (l2, l1) = (3,2), (1,3), (2,1) in 1-based vertex ids
-    const int L2[3] = {2, 0, 1}, L1[3] = {1, 2, 0};
-    double sp[3], sm[3], rp[3], rm[3], r0[3];
-    for (int l = 0; l < 3; ++l) {
-        const V3 p2 = tri[L2[l]], p1 = tri[L1[l]];
-        const V3 slv = vsub(p2, p1);
-        const double ns = sqrt(vdot(slv, slv));
-        const V3 sl = V3{slv.x / ns, slv.y / ns, slv.z / ns};
-        const V3 ml = vcross(sl, n);
-        const V3 pl1mr = vsub(p1, r);
-        const double tl0 = vdot(pl1mr, ml);
-        const double ll = sqrt(vdot(slv, slv));
-        const double sml = vdot(pl1mr, sl), spl = sml + ll;
-        const V3 rmp2 = vsub(r, p2);
-        const double Rpl = sqrt(vdot(rmp2, rmp2)), Rml = sqrt(vdot(pl1mr, pl1mr));
-        const double R0l = sqrt(tl0 * tl0 + w0 * w0);
-        tl[l] = tl0;
-        double Km3;
-        if (fabs(w0) > 1.0e-10) {
-            const double Bl = atan((tl0 * spl) / (R0l * R0l + fabs(w0) * Rpl)) - atan((tl0 * sml) / (R0l * R0l + fabs(w0) * Rml));
-            Km3 = 1.0 / fabs(w0) * Bl;
-        } else {
-            Km3 = 0.0;
-        }
-        if ((Rml + sml) > (Rpl - spl)) Il[l] = log(fabs((Rpl + spl) / (Rml + sml)));
-        else Il[l] = log(fabs((Rml - sml) / (Rpl - spl)));
-        Km1 = Km1 + 1.0 / (-1.0 + 2.0) * (-1.0 * w0 * w0 * Km3 + tl0 * Il[l]);
-        sp[l] = spl; sm[l] = sml; rp[l] = Rpl; rm[l] = Rml; r0[l] = R0l;
+// quadrature accessor for the shared set-up arithmetic (near_pair.cuh, lin_setup.cuh)
+struct DevQ {
+    SCD_HD static double t5(int i, int c) {
+#ifdef __CUDA_ARCH__
+        return cQT5[i][c];
+#else
+        return hq().t5[i][c];
+#endif
     }
-    // n = 1: I_l = 1/2 (s+ R+ - s- R- + R0^2 I_l); K1 = 1/3 (w0^2 K_-1 + sum t I)
-    for (int l = 0; l < 3; ++l)
-        Il[l] = 1.0 / (1.0 + 1.0) * (sp[l] * rp[l] - sm[l] * rm[l] + 1.0 * r0[l] * r0[l] * Il[l]);
-    const double K1v = 1.0 / (1.0 + 2.0) * (1.0 * w0 * w0 * Km1 + (tl[0] * Il[0] + tl[1] * Il[1] + tl[2] * Il[2]));
-    K1 = Km1;
-    K2 = K1v;
-}
-
-// singularity_subtraction_int_V_G, src/singularity_subtraction.f90:112-189
-__device__ cd int_V_G(V3 rf, double k, const V3 *Pb, const double *wb, double sumw, const V3 *B) {
-    const double cut = 1.0e-10 * pow(sumw, F13_D);
-    const double c4 = 1.0 / (4 * PI);
-    cd intR = cmk(0, 0);
-    for (int i = 0; i < 24; ++i) {
-        const double RR = vdist(Pb[i], rf);
-        cd II;
-        if (RR < cut) II = cmk(0.0, k / (4.0 * PI));
-        else {
-            const double f = c4 * 1.0 * 1.0 / RR + c4 * (k * k) * (-0.5) * RR;
-            II = green(rf, Pb[i], k);
-            II.x -= f;
-        }
-        intR.x += II.x * wb[i];
-        intR.y += II.y * wb[i];
+    SCD_HD static double r5(int i, int c) {
+#ifdef __CUDA_ARCH__
+        return cQR5[i][c];
+#else
+        return hq().r5[i][c];
+#endif
     }
-    double i4a = 0.0, i4b = 0.0;
-    for (int f = 0; f < 4; ++f) {
-        V3 tri[3];
-        face_of(B, f, tri);
-        const V3 n = tri_normal(tri);
-        double K1, K2;
-        analytic_tri(tri, n, rf, K1, K2);
-        const double a1 = vdot(n, vsub(tri[0], rf));
-        i4a = i4a + a1 * K1 * 0.5;
-        i4b = i4b + a1 * K2 * 0.25;
-    }
-    const double f2 = c4 * 1.0 * i4a + c4 * (k * k) * (-0.5) * i4b;
-    return cmk(intR.x + f2, intR.y);
-}
-
-// singularity_subtraction_int_S_G, src/singularity_subtraction.f90:193-243
-__device__ cd int_S_G(V3 rf, const V3 *tri, V3 n, double k, const V3 *Pb, const double *wb, double sumw) {
-    const double cut = 1.0e-10 * sqrt(sumw);
-    const double c4 = 1.0 / (4 * PI);
-    cd intR = cmk(0, 0);
-    for (int i = 0; i < 7; ++i) {
-        const double R = vdist(Pb[i], rf);
-        cd II;
-        if (R < cut) II = cmk(0.0, k / (4 * PI));
-        else {
-            const double f = c4 * 1.0 * 1.0 / R + c4 * (k * k) * (-0.5) * R;
-            II = green(rf, Pb[i], k);
-            II.x -= f;
-        }
-        intR.x += II.x * wb[i];
-        intR.y += II.y * wb[i];
-    }
-    double K1, K2;
-    analytic_tri(tri, n, rf, K1, K2);
-    const double f2 = c4 * 1.0 * K1 + c4 * (k * k) * (-0.5) * K2;
-    return cmk(intR.x + f2, intR.y);
-}
-
-}  // namespace
-
-namespace {
-
-// ---------------------------------------------------------------- blocks
-// One near-zone block (src/precorrection.f90:183-254) for test tet t and
-// basis tet b (original numbering t <= b):
-//   blk = delta_tb I/(eps_t - 1) + (-k^2 (V_VG - corr) + (dV_dVG - corr2))/sqrt(vol_t vol_b)
-// where corr = S_t^T G S_b I and corr2(r,c) = P_r,t^T G P_c,b with the 27x27
-// grid Green matrix G of the two boxes (compute_pG, :21-46, precorrect_const,
-// :50-82).  gs/gx/gy/gz = G S_b, G Sx_b, G Sy_b, G Sz_b (27 each).
-struct TetGeo {
-    V3 v[4];
-    double vol;
 };
 
-__device__ void near_block(const TetGeo &T, const TetGeo &B, bool self, cd eps_t, double k,
-                           const cd *St, const cd *Sxt, const cd *Syt, const cd *Szt, long long ps,
-                           const cd *gs, const cd *gx, const cd *gy, const cd *gz, cd out[9]) {
-    // precorrection (linear in S; computed from G times basis projectors)
-    cd acorr = cmk(0, 0);
-    cd corr2[9];
-    for (int q = 0; q < 9; ++q) corr2[q] = cmk(0, 0);
-    for (int a = 0; a < 27; ++a) {
-        cfma(acorr, gs[a], St[a * ps]);
-        const cd pt[3] = {Sxt[a * ps], Syt[a * ps], Szt[a * ps]};
-        const cd gb[3] = {gx[a], gy[a], gz[a]};
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) cfma(corr2[r + 3 * c], gb[c], pt[r]);
-    }
-    const double sv = sqrt(T.vol * B.vol);
-    acorr = cscale(acorr, sv);
-    for (int q = 0; q < 9; ++q) corr2[q] = cscale(corr2[q], sv);
-
-    // order-5 points of the basis tet (linmap_tet, src/common.f90:1354-1377)
-    V3 Pb[24];
-    double wb[24], sumw = 0.0;
-    for (int i = 0; i < 24; ++i) {
-        const double N2 = cQT5[i][0], N3 = cQT5[i][1], N4 = cQT5[i][2], N1 = 1 - N2 - N3 - N4;
-        Pb[i] = V3{B.v[0].x * N1 + B.v[1].x * N2 + B.v[2].x * N3 + B.v[3].x * N4,
-                   B.v[0].y * N1 + B.v[1].y * N2 + B.v[2].y * N3 + B.v[3].y * N4,
-                   B.v[0].z * N1 + B.v[1].z * N2 + B.v[2].z * N3 + B.v[3].z * N4};
-        wb[i] = cQT5[i][3] * 6.0 * B.vol;
-        sumw += wb[i];
-    }
-    // integrate_V_V_G (src/precorrection.f90:729-760)
-    cd vvg = cmk(0, 0);
-    for (int i = 0; i < 24; ++i) {
-        const double N2 = cQT5[i][0], N3 = cQT5[i][1], N4 = cQT5[i][2], N1 = 1 - N2 - N3 - N4;
-        const V3 rf = V3{T.v[0].x * N1 + T.v[1].x * N2 + T.v[2].x * N3 + T.v[3].x * N4,
-                         T.v[0].y * N1 + T.v[1].y * N2 + T.v[2].y * N3 + T.v[3].y * N4,
-                         T.v[0].z * N1 + T.v[1].z * N2 + T.v[2].z * N3 + T.v[3].z * N4};
-        const double wt = cQT5[i][3] * 6.0 * T.vol;
-        const cd in = int_V_G(rf, k, Pb, wb, sumw, B.v);
-        vvg.x += in.x * wt;
-        vvg.y += in.y * wt;
-    }
-    // integrate_dV_dV_G (src/precorrection.f90:764-806)
-    cd dvv[9];
-    for (int q = 0; q < 9; ++q) dvv[q] = cmk(0, 0);
-    for (int ft = 0; ft < 4; ++ft) {
-        V3 ttri[3], ta, tb;
-        face_of(T.v, ft, ttri);
-        const V3 tn = tri_normal(ttri);
-        const double tw1 = tri_ww1(ttri, ta, tb);
-        for (int fb = 0; fb < 4; ++fb) {
-            V3 btri[3], ba, bb;
-            face_of(B.v, fb, btri);
-            const V3 bn = tri_normal(btri);
-            const double bw1 = tri_ww1(btri, ba, bb);
-            V3 Pbt[7];
-            double wbt[7], sw = 0.0;
-            for (int j = 0; j < 7; ++j) {
-                Pbt[j] = V3{btri[0].x + ba.x * cQR5[j][0] + bb.x * cQR5[j][1],
-                            btri[0].y + ba.y * cQR5[j][0] + bb.y * cQR5[j][1],
-                            btri[0].z + ba.z * cQR5[j][0] + bb.z * cQR5[j][1]};
-                wbt[j] = cQR5[j][2] * bw1;
-                sw += wbt[j];
-            }
-            cd acc = cmk(0, 0);
-            for (int i = 0; i < 7; ++i) {
-                const V3 rf = V3{ttri[0].x + ta.x * cQR5[i][0] + tb.x * cQR5[i][1],
-                                 ttri[0].y + ta.y * cQR5[i][0] + tb.y * cQR5[i][1],
-                                 ttri[0].z + ta.z * cQR5[i][0] + tb.z * cQR5[i][1]};
-                const double wt = cQR5[i][2] * tw1;
-                const cd in = int_S_G(rf, btri, bn, k, Pbt, wbt, sw);
-                acc.x += in.x * wt;
-                acc.y += in.y * wt;
-            }
-            const double tnv[3] = {tn.x, tn.y, tn.z}, bnv[3] = {bn.x, bn.y, bn.z};
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const double m = tnv[r] * bnv[c];
-                    dvv[r + 3 * c].x += m * acc.x;
-                    dvv[r + 3 * c].y += m * acc.y;
-                }
-        }
-    }
-    const double k2 = k * k, inv = 1.0 / sqrt(B.vol * T.vol);
-    const cd einv = cdiv(cmk(1.0, 0.0), cmk(eps_t.x - 1.0, eps_t.y));
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int q = r + 3 * c;
-            cd v = cmk(0, 0);
-            if (r == c) {
-                const cd d1 = csub(vvg, acorr);
-                v = cmk(-k2 * d1.x, -k2 * d1.y);
-            }
-            const cd d2 = csub(dvv[q], corr2[q]);
-            v = cmk(inv * (v.x + d2.x), inv * (v.y + d2.y));
-            if (self && r == c) v = cadd(v, einv);
-            out[q] = v;
-        }
-}
-
 // ------------------------------------------------------------- near kernel
-// One CTA per tile (c1 <= c2).  Shared: box-node Green matrix G(c1,c2) and
-// G (resp. G^T) times the basis projectors of every tet of the tile.
 struct NearArgs {
     const NearTile *tiles;
     const double *tc;        // slot-ordered vertex coords, 12 per slot
@@ -310,12 +108,6 @@ __device__ __forceinline__ long long box_node_id(const NearArgs &a, int cube, in
     return ((long long)z * a.Ny + y) * a.Nx + x;
 }
 
-__device__ __forceinline__ void load_tet(const NearArgs &a, int slot, TetGeo &t) {
-    const double *p = a.tc + 12LL * slot;
-    for (int v = 0; v < 4; ++v) t.v[v] = V3{p[3 * v], p[3 * v + 1], p[3 * v + 2]};
-    t.vol = a.vol[slot];
-}
-
 // block (i, j) of tile tl, from column-major blk (transposed when tr)
 __device__ __forceinline__ void store_block(const NearArgs &a, const NearTile &tl, int i, int j, const cd *blk, bool tr) {
     for (int r = 0; r < 3; ++r)
@@ -326,8 +118,6 @@ __device__ __forceinline__ void store_block(const NearArgs &a, const NearTile &t
             else ((cd *)a.data)[e] = v;
         }
 }
-
-constexpr int NEAR_THREADS = 128;
 
 // box-node Green matrix of a tile's two boxes and G (resp. G^T) times the
 // projectors of every basis function of the tile, in shared memory
@@ -363,54 +153,95 @@ __device__ void tile_green(const NearArgs &a, const NearTile &tl, cd *G, cd *GP1
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(NEAR_THREADS) k_near_build(NearArgs a) {
+// The blocks of up to NB_COLS tets of g2 against all of g1 (src/precorrection.f90:
+// 183-254), a thread per pair of tets, for test tet t and basis tet b
+// (original numbering t <= b):
+//   blk = delta_tb I/(eps_t - 1) + (-k^2 (V_VG - corr) + (dV_dVG - corr2))/sqrt(vol_t vol_b)
+// where corr = S_t^T G S_b I and corr2(r,c) = P_r,t^T G P_c,b with the 27x27
+// grid Green matrix G of the two boxes (compute_pG, :21-46, precorrect_const,
+// :50-82).  Shared: G, G times the projectors of the CTA's tets of g2 (with
+// the roles swapped corr2 is the transposed sum), and both sides' PairGeo.
+// Bound by the latency and issue of FP64 arithmetic (a third of the pipe's
+// rate), more than half of it in the Green function.  8,628 tets (sphere,
+// near zone of 20 tets per box) take 32 ms; 144 with the integrals evaluated
+// face by face and point by point, two CTAs of 128 threads per SM.
+constexpr int NB_COLS = 8;                           // most tets of g2 per CTA
+constexpr int NB_THREADS = 128;
+SCD_HD int nb_cols(int n1) { return n1 * NB_COLS <= NB_THREADS ? NB_COLS : NB_THREADS / n1; }
+constexpr size_t NB_SMEM = sizeof(double) * (18 * NB_THREADS + PG * (SCD_GROUP_MAX + NB_COLS)) + sizeof(cd) * NB_COLS * 108;
+static_assert(sizeof(double) * 18 * NB_THREADS >= sizeof(cd) * 27 * 27, "G shares the accumulators' place");
+__global__ void __launch_bounds__(NB_THREADS, 4) k_near_build(NearArgs a) {
     extern __shared__ cd shm[];
     const NearTile tl = a.tiles[blockIdx.x];
-    cd *G = shm;                                    // 27 x 27: G[i*27 + j] = Gr(node_c1(i), node_c2(j))
-    cd *GP1 = G + 27 * 27;                          // per tet of c1: G^T P (4 x 27)
-    cd *GP2 = GP1 + (size_t)tl.n1 * 108;            // per tet of c2: G P (4 x 27)
-    tile_green(a, tl, G, GP1, GP2);
+    const int j0 = blockIdx.y * nb_cols(tl.n1), nc = min(nb_cols(tl.n1), tl.n2 - j0);
+    if (nc <= 0) return;
+    cd *G = shm, *GP = shm + 9 * NB_THREADS;         // GP[jj][g][p] = sum_q G(p, q) P_g(q, j0 + jj)
+    double *acc = reinterpret_cast<double *>(shm);   // after GP is formed, over G
+    double *geo1 = reinterpret_cast<double *>(GP + NB_COLS * 108), *geo2 = geo1 + PG * SCD_GROUP_MAX;
     const long long TT = 27LL * a.T;
-    const int s1 = tl.s1, s2 = tl.s2;
-    const bool diag = tl.g1 == tl.g2;
-    const int npairs = tl.n1 * tl.n2;
-    for (int e = threadIdx.x; e < npairs; e += blockDim.x) {
-        const int i = e / tl.n2, j = e % tl.n2;
-        if (diag && j < i) continue;                // diagonal tile: each pair once
-        const int sa = s1 + i, sb = s2 + j;
-        const bool fwd = a.perm[sa] <= a.perm[sb];  // test = lower original index
-        const int st = fwd ? sa : sb, sbas = fwd ? sb : sa;
-        const cd *gp = fwd ? GP2 + (size_t)j * 108 : GP1 + (size_t)i * 108;
-        TetGeo Tt, Bt;
-        load_tet(a, st, Tt);
-        load_tet(a, sbas, Bt);
-        cd blk[9];
-        near_block(Tt, Bt, st == sbas, a.eps[st], a.k, a.P + st, a.P + TT + st, a.P + 2 * TT + st, a.P + 3 * TT + st,
-                   a.T, gp, gp + 27, gp + 54, gp + 81, blk);
-        store_block(a, tl, i, j, blk, !fwd);
-        if (diag && i != j) store_block(a, tl, j, i, blk, true);
+    for (int e = threadIdx.x; e < 27 * 27; e += NB_THREADS) {
+        const int i = e / 27, j = e % 27;
+        cd v = cmk(0, 0);
+        if (box_node_id(a, tl.c1, i) != box_node_id(a, tl.c2, j))
+            v = green(box_node(a, tl.c1, i), box_node(a, tl.c2, j), a.k);
+        G[e] = v;
     }
+    for (int e = threadIdx.x; e < 10 * (tl.n1 + nc); e += NB_THREADS) {
+        const int t = e / 10, item = e - 10 * t;
+        const int slot = t < tl.n1 ? tl.s1 + t : tl.s2 + j0 + (t - tl.n1);
+        pair_geo(t < tl.n1 ? geo1 + PG * t : geo2 + PG * (t - tl.n1), a.tc + 12LL * slot, a.vol[slot], item);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nc * 108; e += NB_THREADS) {
+        const int jj = e / 108, g = (e / 27) % 4, p = e % 27;
+        const cd *P = a.P + (size_t)g * TT + (tl.s2 + j0 + jj);
+        cd s = cmk(0, 0);
+        for (int q = 0; q < 27; ++q) cfma(s, G[p * 27 + q], P[(size_t)q * a.T]);
+        GP[e] = s;
+    }
+    __syncthreads();
+    const int jj = threadIdx.x / tl.n1, i = threadIdx.x - jj * tl.n1, j = j0 + jj;   // i along the lanes
+    const bool diag = tl.g1 == tl.g2;
+    if (jj >= nc || (diag && j < i)) return;         // diagonal tile: each pair once
+    const int sa = tl.s1 + i, sb = tl.s2 + j;
+    const bool fwd = a.perm[sa] <= a.perm[sb];       // test = lower original index
+    const double *T = fwd ? geo1 + PG * i : geo2 + PG * jj, *B = fwd ? geo2 + PG * jj : geo1 + PG * i;
+    cd vvg, blk[9];
+    pair_integrals<DevQ>(T, B, a.k, vvg, blk, acc + threadIdx.x, NB_THREADS);
+    const double sv = sqrt(T[PG_VOL] * B[PG_VOL]), inv = 1.0 / sv, k2 = a.k * a.k;
+    cd corr = cmk(0, 0), corr2[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) corr2[q] = cmk(0, 0);
+    const cd *gp = GP + jj * 108, *P = a.P + sa;
+    for (int p = 0; p < 27; ++p) {
+        cfma(corr, gp[p], P[(size_t)p * a.T]);
+        const cd pr[3] = {P[TT + (size_t)p * a.T], P[2 * TT + (size_t)p * a.T], P[3 * TT + (size_t)p * a.T]};
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) cfma(corr2[r + 3 * c], gp[27 * (c + 1) + p], pr[r]);
+    }
+    // corr2(r, c) couples axis r of slot sa to axis c of slot sb
+    const cd d1 = csub(vvg, cscale(corr, sv));
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const cd m = fwd ? corr2[r + 3 * c] : corr2[c + 3 * r];
+            const cd d2 = csub(blk[r + 3 * c], cscale(m, sv));
+            cd v = r == c ? cmk(-k2 * d1.x, -k2 * d1.y) : cmk(0, 0);
+            blk[r + 3 * c] = cmk(inv * (v.x + d2.x), inv * (v.y + d2.y));
+        }
+    if (sa == sb) {
+        const cd eps = a.eps[sa], einv = cdiv(cmk(1.0, 0.0), cmk(eps.x - 1.0, eps.y));
+#pragma unroll
+        for (int q = 0; q < 9; q += 4) blk[q] = cadd(blk[q], einv);
+    }
+    store_block(a, tl, i, j, blk, !fwd);
+    if (diag && i != j) store_block(a, tl, j, i, blk, true);
 }
 
 // ------------------------------------------------------- linear basis
-// quadrature accessor for the shared set-up arithmetic (lin_setup.cuh)
-struct DevQ {
-    SCD_HD static double t5(int i, int c) {
-#ifdef __CUDA_ARCH__
-        return cQT5[i][c];
-#else
-        return hq().t5[i][c];
-#endif
-    }
-    SCD_HD static double r5(int i, int c) {
-#ifdef __CUDA_ARCH__
-        return cQR5[i][c];
-#else
-        return hq().r5[i][c];
-#endif
-    }
-};
-
 __device__ __forceinline__ void store_elem(const NearArgs &a, const NearTile &tl, int i, int j, int el, cd v) {
     const long long e = tl.data_off + tile_at(tl.n1, i, j, el);
     if (a.c64) ((cf *)a.data)[e] = make_float2((float)v.x, (float)v.y);
@@ -924,9 +755,9 @@ int setup_nearzone_device(scd_ctx *c, int prec) {
             return rc;
         k_near_build_lin<<<c->ntiles, 32 * LIN_WARPS, sh, c->st>>>(a);
     } else {
-        const size_t sh = sizeof(cd) * (27 * 27 + (size_t)2 * c->max_per_group * 108);
-        if (sh > 48 * 1024) cudaFuncSetAttribute(k_near_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-        k_near_build<<<c->ntiles, NEAR_THREADS, sh, c->st>>>(a);
+        cudaFuncSetAttribute(k_near_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NB_SMEM);
+        if (c->ntiles > 0)
+            k_near_build<<<dim3(c->ntiles, (c->max_per_group + nb_cols(SCD_GROUP_MAX) - 1) / nb_cols(SCD_GROUP_MAX)), NB_THREADS, NB_SMEM, c->st>>>(a);
     }
     rc = check_cuda(c, cudaGetLastError(), "near-zone launch");
     if (!rc) rc = check_cuda(c, cudaStreamSynchronize(c->st), "near-zone build");
