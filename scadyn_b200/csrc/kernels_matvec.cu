@@ -22,13 +22,16 @@
 namespace {
 
 constexpr int WARPS_PER_CTA = 4;
-// resident CTAs per SM the complex64 interpolation kernel is compiled for
-// (its register cap): at C2 with 32 right-hand sides 0.75 ms with 3 (160
-// registers), 0.90 with 1 (174), 1.07 with 4 or 5 (spills)
+// resident CTAs per SM the complex64 interpolation of fewer than eight
+// right-hand sides is compiled for (its register cap)
 #ifndef SCD_GATHER_MINB
 #define SCD_GATHER_MINB 3
 #endif
 // interpolation warps per SM that the spans of right-hand sides aim at
+// ... and of eight or more (k_gather_cta)
+#ifndef SCD_GATHER_CTAS
+#define SCD_GATHER_CTAS 4
+#endif
 #ifndef SCD_GATHER_WARPS
 #define SCD_GATHER_WARPS 24
 #endif
@@ -1367,6 +1370,103 @@ k_gather(const C *__restrict__ Rg, const C *__restrict__ P, int T, const int *__
     }
 }
 
+// The same interpolation for eight or more right-hand sides, one CTA per
+// (group, span): the group's 108 projector rows are staged in shared memory by
+// asynchronous copies, and the four warps take SR right-hand sides each per
+// round, in k_gather's order of sums (the same bits).  Bound by the latency of
+// the slot and node reads: 32 complex64 right-hand sides of 60k tets take 238 us
+// (334 with a warp per group that reads the rows from L1 every round), 16 FP64
+// ones of 12,864 tets 57 (67); five CTAs per SM (96 registers) take 266.
+constexpr int GCB = 128;
+template <typename C, int SR> struct GatherShared {
+    C P[108][SCD_GROUP_MAX + 1];
+    C R[GCB / 32][SR][4][27];
+};
+template <typename C, int SR>
+__global__ void __launch_bounds__(GCB, sizeof(C) == 8 ? SCD_GATHER_CTAS : 2)
+k_gather_cta(const C *__restrict__ Rg, const C *__restrict__ P, int T, const int *__restrict__ grp_off,
+             const int *__restrict__ grp_cube, GridDims G, typename CReal<C>::type k2, const C *__restrict__ part,
+             long long part_len, const long long *__restrict__ pslot_base, const int *__restrict__ pslot_cnt,
+             C *__restrict__ y, long long ld, const int *skip, int nrhs, int rspan) {
+    extern __shared__ __align__(16) unsigned char ga_raw[];
+    GatherShared<C, SR> &sh = *reinterpret_cast<GatherShared<C, SR> *>(ga_raw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = blockIdx.x;
+    const int s0 = grp_off[gq], nc = grp_off[gq + 1] - s0, c = grp_cube[gq];
+    for (int row = threadIdx.x >> 4; row < 108; row += GCB / 16)
+        for (int t = threadIdx.x & 15; t < nc; t += 16)
+            cp_async_el<(int)sizeof(C)>(&sh.P[row][t], P + (size_t)row * T + s0 + t, true);
+    const int bx = c % G.ncx, by = (c / G.ncx) % G.ncy, bz = c / (G.ncx * G.ncy);
+    const long long NN = (long long)G.Nx * G.Ny * G.Nz;
+    const C *pr0 = part + pslot_base[gq] + 3 * lane;
+    const int nslot = pslot_cnt[gq];
+    const int a = lane % 3, b = (lane / 3) % 3, cc = lane / 9;
+    const long long node = ((long long)(2 * bz + cc) * G.Ny + (2 * by + b)) * G.Nx + (2 * bx + a);
+    const int rlo = blockIdx.y * rspan, rhi = min(nrhs, rlo + rspan);
+    const int nround = (rhi - rlo + GCB / 32 * SR - 1) / (GCB / 32 * SR);
+    for (int rd = 0; rd < nround; ++rd) {
+        const int r0 = rlo + (rd * (GCB / 32) + warp) * SR;
+        __syncwarp();
+        if (lane < 27)
+#pragma unroll
+            for (int q = 0; q < SR; ++q)
+                if (r0 + q < rhi)
+#pragma unroll
+                    for (int g = 0; g < 4; ++g)
+                        cp_async_el<(int)sizeof(C)>(&sh.R[warp][q][g][lane], Rg + ((long long)(r0 + q) * 4 + g) * NN + node, true);
+        cp_async_wait_all();
+        if (rd == 0) __syncthreads();
+        else __syncwarp();
+        if (lane >= nc || r0 >= rhi) continue;
+        C acc[SR][6];
+#pragma unroll
+        for (int q = 0; q < SR; ++q)
+#pragma unroll
+            for (int v = 0; v < 6; ++v) acc[q][v] = czero<C>();
+        for (int j = 0; j < 27; ++j) {
+            const C p0 = sh.P[j][lane], px = sh.P[27 + j][lane], py = sh.P[54 + j][lane], pz = sh.P[81 + j][lane];
+#pragma unroll
+            for (int q = 0; q < SR; ++q) {
+                cfma(acc[q][0], p0, sh.R[warp][q][0][j]);
+                cfma(acc[q][1], p0, sh.R[warp][q][1][j]);
+                cfma(acc[q][2], p0, sh.R[warp][q][2][j]);
+                const C r3 = sh.R[warp][q][3][j];
+                cfma(acc[q][3], px, r3);
+                cfma(acc[q][4], py, r3);
+                cfma(acc[q][5], pz, r3);
+            }
+        }
+        C far[SR][3], nz[SR][3];
+        bool on[SR];
+#pragma unroll
+        for (int q = 0; q < SR; ++q) {
+            on[q] = r0 + q < rhi && !(skip && skip[r0 + q]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                far[q][d] = csub_scaled(acc[q][3 + d], k2, acc[q][d]);
+                nz[q][d] = czero<C>();
+            }
+        }
+#pragma unroll 2
+        for (int t = 0; t < nslot; ++t) {
+            const C *pt = pr0 + (long long)t * 3 * nc;
+#pragma unroll
+            for (int q = 0; q < SR; ++q) {
+                if (!on[q]) continue;
+                const C *pq = pt + (r0 + q) * part_len;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) nz[q][d] = cadd(nz[q][d], pq[d]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < SR; ++q) {
+            if (!on[q]) continue;
+            C *yr = y + (r0 + q) * ld + 3LL * (s0 + lane);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) yr[d] = cadd(nz[q][d], far[q][d]);
+        }
+    }
+}
+
 __global__ void k_twiddles(cd *tw, int P) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < P) {
@@ -1535,8 +1635,8 @@ bool ensure_fyz(scd_ctx *c) {
 // CTAs; two waves of the interpolation's twelve warps).  A longer span reads
 // the projector rows fewer times, a shorter one keeps a small mesh from
 // leaving SMs idle: 32 complex64 right-hand sides of 6,144 tets (300 groups)
-// interpolate in 32 us with spans of 4, in 91 with one span of 32; at 60k
-// tets both take 335.
+// interpolated in 32 us with spans of 4 per warp, in 91 with one span of 32; at
+// 60k tets both took 335.
 int rhs_span(const scd_ctx *c, int tuned, int nrhs, int items, int unit, int per_sm) {
     int sp = tuned;
     if (sp <= 0) {
@@ -1702,7 +1802,15 @@ void gather_t(scd_ctx *c, C *y, int nrhs, const int *done) {
     if (c->ngroups == 0) return;
     typedef typename CReal<C>::type R;
     const R k2 = (R)(c->k * c->k);
-    if (nrhs >= 4) {
+    if (nrhs >= 8) {
+        constexpr int SR = 4;
+        const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, GCB / 32 * SR, SCD_GATHER_CTAS);
+        const int sh = (int)sizeof(GatherShared<C, SR>);
+        cudaFuncSetAttribute(k_gather_cta<C, SR>, cudaFuncAttributeMaxDynamicSharedMemorySize, sh);
+        k_gather_cta<C, SR><<<dim3((unsigned)c->ngroups, (nrhs + sp - 1) / sp), GCB, sh, c->st>>>(
+            Res<C>::R(c), Res<C>::P(c), c->T, c->d_grp_off, c->d_grp_cube, G, k2, Res<C>::part(c), c->part_len,
+            c->d_pslot_base, c->d_pslot_cnt, y, c->n, done, nrhs, sp);
+    } else if (nrhs >= 4) {
         const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, 4, SCD_GATHER_WARPS);
         k_gather<C, 4><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(
             Res<C>::R(c), Res<C>::P(c), c->T, c->d_grp_off, c->d_grp_cube, c->ngroups, G, k2, Res<C>::part(c),
