@@ -348,13 +348,13 @@ class Solver:
     # --- hot path
     def compute_Ax2(self, x):
         x = _c128(x)
-        Ax = np.zeros_like(x)
+        Ax = np.empty_like(x)
         self._chk(self.lib.scd_matvec(self.ctx, _p(x), _p(Ax)), "matvec")
         return Ax
 
     def gmres(self, rhs, tol=1e-5, m=50, cycles=4):
         rhs = _c128(rhs)
-        x = np.zeros_like(rhs)
+        x = np.empty_like(rhs)
         it = C.c_int32()
         rr = C.c_double()
         rc = self._chk(self.lib.scd_gmres(self.ctx, _p(rhs), _p(x), tol, m, cycles, C.byref(it), C.byref(rr)),
@@ -391,7 +391,7 @@ class Solver:
             ncol = nmat - col0
         Tc = np.zeros((ncol, nmat), np.complex128)
         iters = np.zeros(ncol, np.int32)
-        X = np.zeros((ncol, self.n), np.complex128) if want_x else None
+        X = np.empty((ncol, self.n), np.complex128) if want_x else None
         o = SolveOpts(tol, m, cycles, block, precision, inner_tol, max_outer, gram_schmidt)
         rc = self._chk(self.lib.scd_solve_columns(self.ctx, nmat, _p(mat), col0, ncol, _p(Tc), C.byref(o),
                                                   _p(iters), _p(X)),
