@@ -55,7 +55,7 @@ struct TickArgs {
     cd *cs, *sn, *g, *y;   // [slot][m+1]
     C *x, *rhs, *w; // [slot][n]
     double *cpart;  // [slot][nch][4] chunk partials
-    double *rnorm;  // [slot][nch] chunk partials of ||w||^2 (resident Gram-Schmidt)
+    double *rnorm;  // [slot][2][nch] chunk partials of ||w||^2 before and after (resident Gram-Schmidt)
     int res;        // resident Gram-Schmidt: items per warp, 0 = off
     double *ctot;   // [2][NSMAX][4] slot totals
     int *ccnt;      // [NSMAX] chunks published in the current reduction
@@ -516,12 +516,15 @@ __device__ void mgs_first(const TickArgs<C> &a, const Chunks &ch, const int *smo
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
         if (lane == 0) {
-            a.rnorm[(size_t)s * ch.nch + c] = v[0];
+            a.rnorm[(size_t)2 * s * ch.nch + c] = v[0];
             *reinterpret_cast<double2 *>(a.cpart + ((size_t)s * ch.nch + c) * 4) = cmk(v[1], v[2]);
         }
     }
 }
-// term k (1-based): partials of term k - 1 lie in pair (k - 1) & 1 of cpart
+// term k (1-based): partials of term k - 1 lie in pair (k - 1) & 1 of cpart.
+// The last term's ||w||^2 goes to rnorm: every CTA adds it after the last
+// barrier, and a CTA that is through may be writing the re-orthogonalisation's
+// partials to cpart while a slower one still reads
 template <typename C>
 __device__ void mgs_term(const TickArgs<C> &a, const Chunks &ch, int k, const int *smode, const int *sstep, const int *swpos,
                          C *wsh, C (&z)[CHUNK / 32]) {
@@ -567,7 +570,10 @@ __device__ void mgs_term(const TickArgs<C> &a, const Chunks &ch, int k, const in
         for (int h2 = 0; h2 < 2; ++h2)
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) u[h2] += __shfl_xor_sync(0xffffffffu, u[h2], o);
-        if (lane == 0) *reinterpret_cast<double2 *>(a.cpart + ((size_t)s * ch.nch + c) * 4 + 2 * (k & 1)) = cmk(u[0], u[1]);
+        if (lane == 0) {
+            if (more) *reinterpret_cast<double2 *>(a.cpart + ((size_t)s * ch.nch + c) * 4 + 2 * (k & 1)) = cmk(u[0], u[1]);
+            else a.rnorm[((size_t)2 * s + 1) * ch.nch + c] = u[0];
+        }
         if (j == 0)
 #pragma unroll
             for (int e = 0; e < CHUNK / 32; ++e) z[e] = zn[e];
@@ -742,8 +748,8 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
         for (int s = threadIdx.x >> 5; s < a.ns; s += BW) {
             if (smode[s] != SLOT_ARNOLDI) continue;
             double t[1], h[1];
-            lane_partials<1>(a.rnorm + (size_t)s * nch, 1, nch, lane, t);
-            lane_partials<1>(a.cpart + (size_t)s * nch * 4 + 2 * ((sstep[s] + 1) & 1), 4, nch, lane, h);
+            lane_partials<1>(a.rnorm + (size_t)2 * s * nch, 1, nch, lane, t);
+            lane_partials<1>(a.rnorm + ((size_t)2 * s + 1) * nch, 1, nch, lane, h);
             if (lane == 0) { snormav[s] = sqrt(t[0]); shn[s] = sqrt(h[0]); }
         }
         __syncthreads();
@@ -1201,7 +1207,7 @@ int batch_prepare(scd_ctx *c, int ns, int m, int mixed, BatchBuffers &b) {
     }
     if ((rc = al((void **)&b.slots, sizeof(Slot) * ns, "slots"))) return rc;
     if ((rc = al((void **)&b.cpart, sizeof(double) * (size_t)ns * nch * 4, "chunk partials"))) return rc;
-    if ((rc = al((void **)&b.rnorm, sizeof(double) * (size_t)ns * nch, "norm partials"))) return rc;
+    if ((rc = al((void **)&b.rnorm, sizeof(double) * (size_t)ns * 2 * nch, "norm partials"))) return rc;
     if ((rc = al((void **)&b.ctot, sizeof(double) * 2 * NSMAX * 4, "slot totals"))) return rc;
     if ((rc = al((void **)&b.ccnt, sizeof(int) * (NSMAX + QMAX), "chunk and work-queue counters"))) return rc;
     if (mixed && c->cgs_on) {
