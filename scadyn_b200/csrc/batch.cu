@@ -484,6 +484,7 @@ __device__ __forceinline__ void cgs_totals(const TickArgs<C> &a, const Chunks &c
 // The complex64 form, whose default is classical, has no registers to spare
 // for it.
 template <typename C> constexpr int RES = sizeof(C) == 16 ? 3 : 0;   // items per warp at most
+template <typename C> constexpr size_t TICK_SMEM = (size_t)BW * RES<C> * CHUNK * sizeof(C);
 template <typename C>
 __device__ void mgs_first(const TickArgs<C> &a, const Chunks &ch, const int *smode, const int *swpos, C *wsh, C (&z)[CHUNK / 32]) {
     const int lane = ch.lane;
@@ -1218,15 +1219,11 @@ int batch_prepare(scd_ctx *c, int ns, int m, int mixed, BatchBuffers &b) {
     if (cudaMallocHost((void **)&b.h_slots, sizeof(Slot) * ns) != cudaSuccess) return set_error(c, SCD_OOM, "pinned slots");
     int per_sm = 0, per_sm2 = 0;
     // with the most shared memory a tick asks for, so that the grid is resident in every variant
-    auto tick_ctas = [](const void *k, int res, size_t el) {
-        const size_t dyn = (size_t)BW * res * CHUNK * el;
-        int ctas = 0;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k, BT, dyn);
-        return ctas;
-    };
-    per_sm = tick_ctas((const void *)k_tick<cd>, RES<cd>, sizeof(cd));
-    const int per_f = tick_ctas((const void *)k_tick<cf>, RES<cf>, sizeof(cf));
+    smem_limit<TICK_SMEM<cd>>(k_tick<cd>);
+    smem_limit<TICK_SMEM<cf>>(k_tick<cf>);
+    int per_f = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tick<cd>, BT, TICK_SMEM<cd>);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_f, k_tick<cf>, BT, TICK_SMEM<cf>);
     per_sm = std::min(per_sm, per_f);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_resid, BT, 0);
     per_sm = std::min(per_sm, per_sm2);
@@ -1300,7 +1297,7 @@ static int launch_tick(scd_ctx *c, BatchBuffers &bb, int ns, int nact, int m, in
     const long long warps = (long long)grid * BW, per = (items + warps - 1) / warps;
     a.res = !a.cgs && Chunks::count(n) <= 512 && per <= RES<C> ? (int)per : 0;
     const size_t dyn = (size_t)BW * a.res * CHUNK * sizeof(C);
-    cudaFuncSetAttribute(k_tick<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BW * RES<C> * CHUNK * sizeof(C)));
+    smem_limit<TICK_SMEM<C>>(k_tick<C>);
     cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_tick<C>, dim3(grid), dim3(BT), args, dyn, c->st);
     c->launches += 2;
     return check_cuda(c, e, "tick launch");

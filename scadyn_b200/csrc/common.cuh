@@ -113,6 +113,30 @@ template <> SCD_HD cd as_c<cd>(cd a) { return a; }
 template <> SCD_HD cf as_c<cf>(cf a) { return a; }
 template <> SCD_HD cf as_c<cf>(cd a) { return make_float2((float)a.x, (float)a.y); }
 
+// Dynamic shared memory that launches of `kernel` may ask for.  The limit
+// belongs to the kernel and the device, so host threads with contexts of other
+// sizes share it: it is raised to one constant per kernel, never set to the
+// size of the launch at hand (another thread's larger launch, between its own
+// setting and its launch, would be refused).
+constexpr size_t SMEM_CTA = 227 * 1024;   // opt-in maximum per CTA, static shared memory included
+template <size_t BYTES, typename... A> inline cudaError_t smem_limit(void (*kernel)(A...)) {
+    static_assert(BYTES <= SMEM_CTA, "dynamic shared memory");
+    return cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BYTES);
+}
+// A launch with `smem` dynamic bytes of at most BYTES; the return is its own
+// (an error that was pending before it is not).
+template <size_t BYTES, typename... P, typename... A>
+inline cudaError_t launch_dyn(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    const cudaError_t e = smem_limit<BYTES>(kernel);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Grid-wide barrier for kernels launched with cudaLaunchCooperativeKernel
 // (all CTAs co-resident).  A CTA's writes are released by its arrival and
 // acquired by one fence after the wait; polls are relaxed loads.  The spin is

@@ -200,7 +200,7 @@ template <typename C> struct YzLaunch {
     int nrg;
     cudaStream_t st;
 };
-template <int PY, typename C> void yz_launch(const YzLaunch<C> &l, int Pz);
+template <int PY, typename C> cudaError_t yz_launch(const YzLaunch<C> &l, int Pz);
 
 #ifdef __CUDACC__
 // one CTA per (x, rg): grid (Px, 4 nrhs); dynamic shared memory
@@ -283,13 +283,12 @@ k_fft_yz(C *__restrict__ Wt, const C *__restrict__ Fyz, const C *__restrict__ tw
 // the plane's size, 128 if both do (its lines fill the warps better on small
 // planes).
 template <int PY, int PZ, typename C>
-void yz_launch_t(const YzLaunch<C> &l) {
+cudaError_t yz_launch_t(const YzLaunch<C> &l) {
     auto bytes = [&](int threads) { return sizeof(C) * (size_t)yz_smem_elems<PY, PZ>(l.D.Nz, threads); };
     auto warps = [&](int threads) { return (int)std::min<size_t>((size_t)227 * 1024 / (bytes(threads) + 1024), 512 / threads) * threads; };
     const int threads = warps(256) > warps(128) ? 256 : 128;
     const size_t sh = bytes(threads);
-    cudaFuncSetAttribute(k_fft_yz<PY, PZ, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
-    k_fft_yz<PY, PZ, C><<<dim3(l.D.Px, l.nrg), threads, sh, l.st>>>(l.W, l.Fyz, l.twy, l.twz, l.D, l.done);
+    return launch_dyn<SMEM_CTA>(k_fft_yz<PY, PZ, C>, dim3(l.D.Px, l.nrg), threads, sh, l.st, l.W, l.Fyz, l.twy, l.twz, l.D, l.done);
 }
 
 // Fyz[(fx Hy + fy) Hz + fz] = Fo[(fz Hy + fy) Hx + fx]

@@ -7,21 +7,21 @@
 
 #include "fft_yz.cuh"
 
-template <int PY, typename C> void yz_launch(const YzLaunch<C> &l, int Pz) {
+template <int PY, typename C> cudaError_t yz_launch(const YzLaunch<C> &l, int Pz) {
     switch (Pz) {
-        case 16: yz_launch_t<PY, 16>(l); break;
-        case 32: yz_launch_t<PY, 32>(l); break;
-        case 40: yz_launch_t<PY, 40>(l); break;
-        case 48: yz_launch_t<PY, 48>(l); break;
-        case 64: yz_launch_t<PY, 64>(l); break;
-        case 80: yz_launch_t<PY, 80>(l); break;
-        case 96: yz_launch_t<PY, 96>(l); break;
-        case 112: yz_launch_t<PY, 112>(l); break;
-        case 128: yz_launch_t<PY, 128>(l); break;
-        case 192: yz_launch_t<PY, 192>(l); break;
-        default: break;
+        case 16: return yz_launch_t<PY, 16>(l);
+        case 32: return yz_launch_t<PY, 32>(l);
+        case 40: return yz_launch_t<PY, 40>(l);
+        case 48: return yz_launch_t<PY, 48>(l);
+        case 64: return yz_launch_t<PY, 64>(l);
+        case 80: return yz_launch_t<PY, 80>(l);
+        case 96: return yz_launch_t<PY, 96>(l);
+        case 112: return yz_launch_t<PY, 112>(l);
+        case 128: return yz_launch_t<PY, 128>(l);
+        case 192: return yz_launch_t<PY, 192>(l);
+        default: return cudaErrorInvalidValue;
     }
 }
-#define SCD_YZ_INSTANCE(PY)                                    \
-    template void yz_launch<PY, cf>(const YzLaunch<cf> &, int); \
-    template void yz_launch<PY, cd>(const YzLaunch<cd> &, int);
+#define SCD_YZ_INSTANCE(PY)                                            \
+    template cudaError_t yz_launch<PY, cf>(const YzLaunch<cf> &, int); \
+    template cudaError_t yz_launch<PY, cd>(const YzLaunch<cd> &, int);

@@ -701,7 +701,7 @@ constexpr size_t NZ_SMEM_4CTA = 56 * 1024;  // ... four CTAs
 // four right-hand sides the compiler is left free (two CTAs fit).
 template <int U> constexpr int NZ_MIN_CTAS = U == 1 ? 4 : 1;
 template <int NS> constexpr int N1_THREADS = 32 * ((2 * SCD_GROUP_MAX * NS + 31) / 32) + 32;
-constexpr size_t NZ_SMEM_MAX = 227 * 1024;
+constexpr size_t NZ_SMEM_MAX = SMEM_CTA;
 constexpr int NZ_MAX_THREADS = 2 * 32 * ((SCD_GROUP_MAX * NZ_QMAX + 31) / 32) + 32;
 
 struct NearPass {
@@ -1606,7 +1606,7 @@ size_t yz_smem_bytes(const scd_ctx *c) {
 template <typename C>
 bool use_yz(const scd_ctx *c) {
     if (!c->yz_on || !half_len(c->Py) || !half_len(c->Pz)) return false;
-    return yz_smem_bytes<C>(c) <= (size_t)(227 * 1024);
+    return yz_smem_bytes<C>(c) <= SMEM_CTA;
 }
 
 // the transposed Green octant of the fused pass, built from Fo once per
@@ -1737,9 +1737,8 @@ void near_launch(scd_ctx *c, K kernel, const ST *data, const C *x, int nrhs, int
     k_xpose<C><<<g, 256, 0, c->st>>>(x, c->n, c->n, nrhs, PS, a.rg_stride, Res<C>::xT(c));
     c->launches += 1;
     const size_t sh = NZ_META + a.x1_bytes + a.ring_bytes;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     if (c->timing) cudaEventRecord(c->ev[6], c->st);
-    kernel<<<c->ngroups, threads, sh, c->st>>>(a);
+    launch_dyn<NZ_SMEM_MAX>(kernel, c->ngroups, threads, sh, c->st, a);
     if (c->timing) cudaEventRecord(c->ev[7], c->st);
 }
 
@@ -1805,11 +1804,11 @@ void gather_t(scd_ctx *c, C *y, int nrhs, const int *done) {
     if (nrhs >= 8) {
         constexpr int SR = 4;
         const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, GCB / 32 * SR, SCD_GATHER_CTAS);
-        const int sh = (int)sizeof(GatherShared<C, SR>);
-        cudaFuncSetAttribute(k_gather_cta<C, SR>, cudaFuncAttributeMaxDynamicSharedMemorySize, sh);
-        k_gather_cta<C, SR><<<dim3((unsigned)c->ngroups, (nrhs + sp - 1) / sp), GCB, sh, c->st>>>(
-            Res<C>::R(c), Res<C>::P(c), c->T, c->d_grp_off, c->d_grp_cube, G, k2, Res<C>::part(c), c->part_len,
-            c->d_pslot_base, c->d_pslot_cnt, y, c->n, done, nrhs, sp);
+        constexpr size_t sh = sizeof(GatherShared<C, SR>);
+        launch_dyn<sh>(
+            k_gather_cta<C, SR>, dim3((unsigned)c->ngroups, (nrhs + sp - 1) / sp), GCB, sh, c->st, Res<C>::R(c),
+            Res<C>::P(c), c->T, c->d_grp_off, c->d_grp_cube, G, k2, Res<C>::part(c), c->part_len, c->d_pslot_base,
+            c->d_pslot_cnt, y, c->n, done, nrhs, sp);
     } else if (nrhs >= 4) {
         const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, 4, SCD_GATHER_WARPS);
         k_gather<C, 4><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(

@@ -28,6 +28,7 @@ constexpr uint32_t NZM_META = 256;
 // CTA) must stay within the SM's 228 KB; 113 KB dynamic plus the kernel's
 // static bytes no longer did, and halved the resident CTAs
 constexpr size_t NZM_SMEM = 112 * 1024;
+constexpr size_t NZM_SMEM_MAX = SMEM_CTA - 256;   // less the kernel's static bytes
 constexpr size_t NZM_SMEM_WIDE = NzmSched<2>::CTAS == 2 ? NZM_SMEM : 224 * 1024;   // schedule 2
 
 struct NzmArgs {
@@ -547,7 +548,7 @@ int near_mma_prepare(scd_ctx *c) {
         const size_t fixed = 128 + NZM_META + x1 + c->nzm_slack;
         size_t ring = budget > fixed ? (budget - fixed) / 128 * 128 : 0;
         if (ring < max_slot) ring = (size_t)max_slot;   // one slot at least (then one CTA per SM)
-        if (fixed + ring > 227 * 1024) return set_error(c, SCD_BAD_ARG, "tensor-core near zone: a tile does not fit");
+        if (fixed + ring > NZM_SMEM_MAX) return set_error(c, SCD_BAD_ARG, "tensor-core near zone: a tile does not fit");
         c->nzm_x1[w] = x1;
         c->nzm_ring[w] = (uint32_t)ring;
     }
@@ -561,7 +562,6 @@ static void near_mma_pass(scd_ctx *c, const cf *x, int r0, int rg, const int *do
     constexpr int R = NzmSched<S>::R;
     const int w = R == NZM_RMAX ? 1 : 0;
     const size_t sh = 128 + NZM_META + c->nzm_x1[w] + c->nzm_ring[w] + c->nzm_slack;
-    cudaFuncSetAttribute(k_near_mma<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
     cudaMemsetAsync(c->d_xmax, 0, sizeof(unsigned int) * R, c->st);
     const unsigned gx = (unsigned)std::max<long long>(1, std::min<long long>((c->n + 2047) / 2048, c->nsm));
     k_xabsmax<<<dim3(gx, (unsigned)rg), 256, 0, c->st>>>(x, c->n, r0, rg, c->d_xmax);
@@ -573,7 +573,7 @@ static void near_mma_pass(scd_ctx *c, const cf *x, int r0, int rg, const int *do
     a.part = c->f_nzpart; a.part_len = c->part_len; a.skip = done; a.r0 = r0; a.rg = rg; a.xinv = c->d_xinv;
     a.x1_bytes = c->nzm_x1[w]; a.ring_bytes = c->nzm_ring[w]; a.slack_bytes = c->nzm_slack; a.err = c->d_kerr;
     if (c->timing) cudaEventRecord(c->ev[6], c->st);
-    k_near_mma<S><<<c->ngroups, NZM_THREADS, sh, c->st>>>(a);
+    launch_dyn<NZM_SMEM_MAX>(k_near_mma<S>, c->ngroups, NZM_THREADS, sh, c->st, a);
     if (c->timing) cudaEventRecord(c->ev[7], c->st);
     c->launches += 3;
 }

@@ -250,6 +250,7 @@ __device__ __forceinline__ void store_elem(const NearArgs &a, const NearTile &tl
 
 constexpr int LIN_WARPS = 4;
 constexpr int LIN_WARP_CD = LIN_POINTS * LIN_SCR + LIN_SMALL + 432;   // scratch, small sums, test projectors
+constexpr size_t lin_smem(int per_group) { return sizeof(cd) * (27 * 27 + (size_t)2 * per_group * 108 + (size_t)LIN_WARPS * LIN_WARP_CD); }
 
 // compute_near_zone_interactions_lin (src/precorrection.f90:268-371) on a
 // tile of pseudo-tets (4 consecutive slots per tet, whole tets per group):
@@ -749,13 +750,11 @@ int setup_nearzone_device(scd_ctx *c, int prec) {
     a.k = c->k; a.data = c->d_tdata; a.c64 = prec == SCD_STORE_C64;
     if (c->nb == 4) {
         // linear basis: 12x12 blocks per tet pair, written as pseudo-tet blocks
-        const size_t sh = sizeof(cd) * (27 * 27 + (size_t)2 * c->max_per_group * 108 + (size_t)LIN_WARPS * LIN_WARP_CD);
-        if ((rc = check_cuda(c, cudaFuncSetAttribute(k_near_build_lin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh),
-                             "near-zone shared memory")))
-            return rc;
+        const size_t sh = lin_smem(c->max_per_group);
+        if ((rc = check_cuda(c, smem_limit<lin_smem(SCD_GROUP_MAX)>(k_near_build_lin), "near-zone shared memory"))) return rc;
         k_near_build_lin<<<c->ntiles, 32 * LIN_WARPS, sh, c->st>>>(a);
     } else {
-        cudaFuncSetAttribute(k_near_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NB_SMEM);
+        if (c->ntiles > 0 && (rc = check_cuda(c, smem_limit<NB_SMEM>(k_near_build), "near-zone shared memory"))) return rc;
         if (c->ntiles > 0)
             k_near_build<<<dim3(c->ntiles, (c->max_per_group + nb_cols(SCD_GROUP_MAX) - 1) / nb_cols(SCD_GROUP_MAX)), NB_THREADS, NB_SMEM, c->st>>>(a);
     }
