@@ -108,8 +108,21 @@ void release_work(scd_ctx *c) {
     c->nzm_ready = false;
 }
 
+// a refused launch leaves its output as it was: the matvec's result is not one
+int launch_status(scd_ctx *c) {
+    if (c->launch_err == cudaSuccess) return SCD_OK;
+    const cudaError_t e = c->launch_err;
+    c->launch_err = cudaSuccess;
+    if (cudaPeekAtLastError() == e) cudaGetLastError();
+    return set_error(c, SCD_CUDA_ERROR, "matvec launch: %s", cudaGetErrorString(e));
+}
+
 // error word of the near-zone kernel: a bounded wait that ran out
 int near_status(scd_ctx *c) {
+    {
+        const int rc = launch_status(c);
+        if (rc) return rc;
+    }
     if (c->near_cfg_err) {
         c->near_cfg_err = 0;
         return set_error(c, SCD_BAD_ARG, "near-zone kernel not launched: a tile with its x segment exceeds the shared-memory ring");
@@ -587,6 +600,7 @@ int scd_set_nearzone(scd_ctx *c, int64_t B, const void *sp_mat, const int32_t *s
 }
 
 static int ready(scd_ctx *c) {
+    c->launch_err = cudaSuccess;
     if (!c->have_proj) return set_error(c, SCD_NOT_READY, "projectors not set");
     if (!c->have_green) return set_error(c, SCD_NOT_READY, "Green's function not set (or stale after a new wavenumber)");
     if (!c->have_near) return set_error(c, SCD_NOT_READY, "near zone not set");

@@ -1243,11 +1243,11 @@ int batch_prepare(scd_ctx *c, int ns, int m, int mixed, BatchBuffers &b) {
 // streams, forked from and joined back to c's stream, so the operators of a
 // sweep work concurrently.
 template <typename C>
-static void multi_matvec(scd_ctx *c, const std::vector<scd_ctx *> &ops, const C *in, C *out, const std::vector<int> &cnt) {
+static int multi_matvec(scd_ctx *c, const std::vector<scd_ctx *> &ops, const C *in, C *out, const std::vector<int> &cnt) {
     const long long n = c->n;
     if (ops.size() == 1) {
         if (cnt[0] > 0) run_matvec(ops[0], in, out, cnt[0], nullptr);
-        return;
+        return launch_status(c);
     }
     if (!c->ev_fork) cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
     cudaEventRecord(c->ev_fork, c->st);
@@ -1266,6 +1266,12 @@ static void multi_matvec(scd_ctx *c, const std::vector<scd_ctx *> &ops, const C 
         }
         off += cnt[w];
     }
+    int rc = SCD_OK;
+    for (scd_ctx *o : ops) {
+        const int r = launch_status(o);
+        if (r && !rc) rc = o == c ? r : set_error(c, r, "operator of the batch: %s", o->err.c_str());
+    }
+    return rc;
 }
 
 template <typename C>
@@ -1282,7 +1288,8 @@ static int launch_tick(scd_ctx *c, BatchBuffers &bb, int ns, int nact, int m, in
     const long long n = c->n;
     if (nact > 0) {
         k_stage<C><<<dim3(Chunks::count(n), ns), 256, 0, c->st>>>(bb.slots, ns, (C *)bb.V, (C *)bb.x, (C *)bb.Xin, n, m);
-        multi_matvec<C>(c, ops, (const C *)bb.Xin, (C *)bb.W, cnt);
+        const int rc = multi_matvec<C>(c, ops, (const C *)bb.Xin, (C *)bb.W, cnt);
+        if (rc) return rc;
     }
     NvtxRange r("arnoldi tick");
     void *args[] = {&a};
@@ -1429,7 +1436,7 @@ int batch_run(scd_ctx *c, ColumnSource &src, double tol, int m, int cycles, int 
             if (upd) k_outer_update<<<g2, 256, 0, c->st>>>(bb.slots, bb.x64, (const cf *)bb.x, n);
             if (resid) {
                 k_stage_resid<<<g2, 256, 0, c->st>>>(bb.slots, bb.x64, bb.Xin64, n);
-                multi_matvec<cd>(c, ops, (const cd *)bb.Xin64, bb.W64, cnt_r);
+                if ((rc = multi_matvec<cd>(c, ops, (const cd *)bb.Xin64, bb.W64, cnt_r))) return rc;
                 ResidArgs ra;
                 ra.slots = bb.slots; ra.ns = ns; ra.b64 = bb.b64; ra.w64 = bb.W64; ra.rhs32 = (cf *)bb.rhs;
                 ra.x32 = (cf *)bb.x; ra.part = bb.cpart; ra.bar = c->d_bar; ra.err = c->d_err; ra.n = n; ra.tol = tol;

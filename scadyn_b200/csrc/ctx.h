@@ -111,6 +111,7 @@ struct scd_ctx {
     long long max_tile_store = 0;        // largest tile_elems
     long long B_ref = 0;                 // blocks in the reference layout
     int near_split = 2;                  // partial sums per near-zone row/column sum (scd_grid_desc.near_split)
+    cudaError_t launch_err = cudaSuccess;   // of a matvec launch that was refused (launch_status)
     int near_cfg_err = 0;                // a near-zone launch was skipped: a tile outgrew the shared-memory ring
     // partial-sum slots per group: slot 0 holds the group's row sums over
     // all its tiles, slots 1.. the M^T x products of the tiles (g', g),
@@ -258,8 +259,9 @@ int set_error(scd_ctx *c, int code, const char *fmt, ...);
 int check_cuda(scd_ctx *c, cudaError_t e, const char *what);
 int ensure_work(scd_ctx *c, int nrhs);
 void release_work(scd_ctx *c);
-int near_status(scd_ctx *c);
+int launch_status(scd_ctx *c);   // SCD_CUDA_ERROR if a launch of a matvec was refused (and clears it)
+int near_status(scd_ctx *c);     // the same, and SCD_TIMEOUT if a near-zone pipeline wait ran out (and clears it)
 // columns of the interleaved matvec input for nrhs right-hand sides: passes
 // of 16 in rows of 18 (the FP64 near zone's bank spread), at least 2 (16-byte
 // rows for complex64)
-inline int xt_columns(int nrhs) { return std::max(2, (nrhs + 15) / 16 * 18); }   // SCD_TIMEOUT if a near-zone pipeline wait ran out (and clears it)
+inline int xt_columns(int nrhs) { return std::max(2, (nrhs + 15) / 16 * 18); }

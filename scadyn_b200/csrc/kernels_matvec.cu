@@ -1575,19 +1575,21 @@ void fft_yz(scd_ctx *c, const GridDims &G, int nrg, const int *done) {
     l.D.Nx = G.Nx; l.D.Ny = G.Ny; l.D.Nz = G.Nz; l.D.NzR = yz_round8(G.Nz);
     l.D.Px = G.Px; l.D.Hx = G.Hx; l.D.Hy = G.Hy; l.D.Hz = G.Hz;
     l.done = done; l.nrg = nrg; l.st = c->st;
+    cudaError_t e = cudaErrorInvalidValue;
     switch (G.Py) {
-        case 16: yz_launch<16>(l, G.Pz); break;
-        case 32: yz_launch<32>(l, G.Pz); break;
-        case 40: yz_launch<40>(l, G.Pz); break;
-        case 48: yz_launch<48>(l, G.Pz); break;
-        case 64: yz_launch<64>(l, G.Pz); break;
-        case 80: yz_launch<80>(l, G.Pz); break;
-        case 96: yz_launch<96>(l, G.Pz); break;
-        case 112: yz_launch<112>(l, G.Pz); break;
-        case 128: yz_launch<128>(l, G.Pz); break;
-        case 192: yz_launch<192>(l, G.Pz); break;
+        case 16: e = yz_launch<16>(l, G.Pz); break;
+        case 32: e = yz_launch<32>(l, G.Pz); break;
+        case 40: e = yz_launch<40>(l, G.Pz); break;
+        case 48: e = yz_launch<48>(l, G.Pz); break;
+        case 64: e = yz_launch<64>(l, G.Pz); break;
+        case 80: e = yz_launch<80>(l, G.Pz); break;
+        case 96: e = yz_launch<96>(l, G.Pz); break;
+        case 112: e = yz_launch<112>(l, G.Pz); break;
+        case 128: e = yz_launch<128>(l, G.Pz); break;
+        case 192: e = yz_launch<192>(l, G.Pz); break;
         default: break;
     }
+    if (e != cudaSuccess) c->launch_err = e;
 }
 
 // least shared memory of the fused y-z pass for the context's lengths (CTAs of
@@ -1738,7 +1740,8 @@ void near_launch(scd_ctx *c, K kernel, const ST *data, const C *x, int nrhs, int
     c->launches += 1;
     const size_t sh = NZ_META + a.x1_bytes + a.ring_bytes;
     if (c->timing) cudaEventRecord(c->ev[6], c->st);
-    launch_dyn<NZ_SMEM_MAX>(kernel, c->ngroups, threads, sh, c->st, a);
+    const cudaError_t e = launch_dyn<NZ_SMEM_MAX>(kernel, c->ngroups, threads, sh, c->st, a);
+    if (e != cudaSuccess) c->launch_err = e;
     if (c->timing) cudaEventRecord(c->ev[7], c->st);
 }
 
@@ -1805,10 +1808,11 @@ void gather_t(scd_ctx *c, C *y, int nrhs, const int *done) {
         constexpr int SR = 4;
         const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, GCB / 32 * SR, SCD_GATHER_CTAS);
         constexpr size_t sh = sizeof(GatherShared<C, SR>);
-        launch_dyn<sh>(
+        const cudaError_t e = launch_dyn<sh>(
             k_gather_cta<C, SR>, dim3((unsigned)c->ngroups, (nrhs + sp - 1) / sp), GCB, sh, c->st, Res<C>::R(c),
             Res<C>::P(c), c->T, c->d_grp_off, c->d_grp_cube, G, k2, Res<C>::part(c), c->part_len, c->d_pslot_base,
             c->d_pslot_cnt, y, c->n, done, nrhs, sp);
+        if (e != cudaSuccess) c->launch_err = e;
     } else if (nrhs >= 4) {
         const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, 4, SCD_GATHER_WARPS);
         k_gather<C, 4><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(

@@ -573,7 +573,8 @@ static void near_mma_pass(scd_ctx *c, const cf *x, int r0, int rg, const int *do
     a.part = c->f_nzpart; a.part_len = c->part_len; a.skip = done; a.r0 = r0; a.rg = rg; a.xinv = c->d_xinv;
     a.x1_bytes = c->nzm_x1[w]; a.ring_bytes = c->nzm_ring[w]; a.slack_bytes = c->nzm_slack; a.err = c->d_kerr;
     if (c->timing) cudaEventRecord(c->ev[6], c->st);
-    launch_dyn<NZM_SMEM_MAX>(k_near_mma<S>, c->ngroups, NZM_THREADS, sh, c->st, a);
+    const cudaError_t e = launch_dyn<NZM_SMEM_MAX>(k_near_mma<S>, c->ngroups, NZM_THREADS, sh, c->st, a);
+    if (e != cudaSuccess) c->launch_err = e;
     if (c->timing) cudaEventRecord(c->ev[7], c->st);
     c->launches += 3;
 }
