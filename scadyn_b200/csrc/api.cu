@@ -989,8 +989,21 @@ int scd_tune_matvec(scd_ctx *c, int32_t nrhs, int32_t precision, int32_t reps, s
                    {SCD_NEAR_CUDA_CORES, SCD_NEAR_TENSOR_SPLIT, SCD_NEAR_TENSOR_MERGED, SCD_NEAR_TENSOR_WIDE})))
         return rc;
     if ((rc = knob(&scd_tuning::fft_passes, {SCD_FFT_PASSES_FUSED_YZ, SCD_FFT_PASSES_THREE}))) return rc;
-    if (nrhs > 8 && (rc = knob(&scd_tuning::scatter_span, {0, 8, 16}))) return rc;
-    if (nrhs > 4 && (rc = knob(&scd_tuning::gather_span, {0, 4, 8, 16}))) return rc;
+    // the spans that give launches of their own: 0 and the multiples of a
+    // round, each once
+    auto span_knob = [&](int32_t scd_tuning::*field, int (*span_of)(const scd_ctx *, int, int)) -> int {
+        std::vector<int> seen{span_of(c, nrhs, best.*field)};
+        for (int32_t v : {0, 4, 16, 32, 48}) {
+            const int sp = span_of(c, nrhs, v);
+            if (std::find(seen.begin(), seen.end(), sp) != seen.end()) continue;
+            seen.push_back(sp);
+            const int r = knob(field, {v});
+            if (r) return r;
+        }
+        return SCD_OK;
+    };
+    if ((rc = span_knob(&scd_tuning::scatter_span, scatter_span_of))) return rc;
+    if ((rc = span_knob(&scd_tuning::gather_span, gather_span_of))) return rc;
     put_tuning(c, best);
     best.matvec_ms = best_ms;
     best.default_ms = default_ms;

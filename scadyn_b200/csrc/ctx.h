@@ -207,6 +207,9 @@ int ensure_work_single(scd_ctx *c, int nrhs);
 void launch_near(scd_ctx *c, const cd *x, int nrhs, const int *done);
 void launch_fft_chain(scd_ctx *c, const cd *x, int nrhs, const int *done);
 void launch_gather(scd_ctx *c, const cd *x, cd *y, int nrhs, const int *done);
+// right-hand sides per block that a matvec of nrhs takes for a tuned span
+int scatter_span_of(const scd_ctx *c, int nrhs, int tuned);
+int gather_span_of(const scd_ctx *c, int nrhs, int tuned);
 int build_twiddles(scd_ctx *c, int P, cd **out);
 // tensor-core near zone (near_mma.cu)
 int near_mma_prepare(scd_ctx *c);

@@ -27,13 +27,15 @@ constexpr int WARPS_PER_CTA = 4;
 #ifndef SCD_GATHER_MINB
 #define SCD_GATHER_MINB 3
 #endif
-// interpolation warps per SM that the spans of right-hand sides aim at
-// ... and of eight or more (k_gather_cta)
-#ifndef SCD_GATHER_CTAS
-#define SCD_GATHER_CTAS 4
-#endif
+// interpolation warps per SM that the spans of fewer than eight right-hand
+// sides aim at
 #ifndef SCD_GATHER_WARPS
 #define SCD_GATHER_WARPS 24
+#endif
+// resident CTAs per SM of the FP64 interpolation of eight or more
+// (k_gather_cta), and what the spans aim at in both precisions
+#ifndef SCD_GATHER_CTAS
+#define SCD_GATHER_CTAS 4
 #endif
 
 // slot order <-> the reference's unknown order (nb basis functions per tet:
@@ -1377,7 +1379,7 @@ k_gather(const C *__restrict__ Rg, const C *__restrict__ P, int T, const int *__
 // the slot and node reads: 32 complex64 right-hand sides of 60k tets take 238 us
 // (334 with a warp per group that reads the rows from L1 every round), 16 FP64
 // ones of 12,864 tets 57 (67); five CTAs per SM (96 registers) take 266.
-constexpr int GCB = 128;
+constexpr int GCB = 128, GC_SR = 4;
 template <typename C, int SR> struct GatherShared {
     C P[108][SCD_GROUP_MAX + 1];
     C R[GCB / 32][SR][4][27];
@@ -1631,16 +1633,14 @@ bool ensure_fyz(scd_ctx *c) {
     return true;
 }
 
-// Right-hand sides that one block of the anterpolation (one warp of the
-// interpolation) walks: a tuned span, or the most that still gives every SM
-// `per_sm` of the `items` x spans blocks (the anterpolation's five resident
-// CTAs; two waves of the interpolation's twelve warps).  A longer span reads
-// the projector rows fewer times, a shorter one keeps a small mesh from
-// leaving SMs idle: 32 complex64 right-hand sides of 6,144 tets (300 groups)
-// interpolated in 32 us with spans of 4 per warp, in 91 with one span of 32; at
-// 60k tets both took 335.
+// Right-hand sides that one block walks: a tuned span, or the most that still
+// gives every SM `per_sm` of the `items` x spans blocks, rounded up to the
+// `unit` of a round.  A longer span reads the projector rows fewer times, a
+// shorter one keeps a small mesh from leaving SMs idle: 32 complex64
+// right-hand sides of 6,144 tets (300 groups) interpolated in 32 us with spans
+// of 4 per warp, in 91 with one span of 32; at 60k tets both took 335.
 int rhs_span(const scd_ctx *c, int tuned, int nrhs, int items, int unit, int per_sm) {
-    int sp = tuned;
+    int sp = std::min(tuned, nrhs);
     if (sp <= 0) {
         const long long want = (long long)per_sm * c->nsm;
         const long long spans = std::min<long long>((nrhs + unit - 1) / unit, (want + items - 1) / std::max(items, 1));
@@ -1648,7 +1648,21 @@ int rhs_span(const scd_ctx *c, int tuned, int nrhs, int items, int unit, int per
     }
     return (sp + unit - 1) / unit * unit;
 }
+}  // namespace
 
+// the spans that a matvec of nrhs right-hand sides takes for a tuned value:
+// the anterpolation walks 16 at a time in five resident CTAs per SM, and all
+// of fewer than eight (k_scatter_few); the interpolation 16 from eight on
+// (k_gather_cta), below that two waves of twelve warps
+int scatter_span_of(const scd_ctx *c, int nrhs, int tuned) {
+    return nrhs >= 8 ? rhs_span(c, tuned, nrhs, c->ncubes, 16, 5) : nrhs;
+}
+int gather_span_of(const scd_ctx *c, int nrhs, int tuned) {
+    return nrhs >= 8 ? rhs_span(c, tuned, nrhs, c->ngroups, GCB / 32 * GC_SR, SCD_GATHER_CTAS)
+                     : rhs_span(c, tuned, nrhs, c->ngroups, nrhs >= 4 ? 4 : 1, SCD_GATHER_WARPS);
+}
+
+namespace {
 #define SCD_DISPATCH_P(PV, CALL)                     \
     switch (PV) {                                    \
         case 8: CALL(8); break;                      \
@@ -1675,7 +1689,7 @@ void fft_chain_t(scd_ctx *c, const C *x, int nrhs, const int *done) {
         constexpr int NTC = sizeof(C) == 8 ? 32 : 16, NTF = sizeof(C) == 8 ? 32 : 24;   // static shared memory: 48 KB
         const dim3 gx((unsigned)c->ncubes);
         if (nrhs >= 8) {
-            const int sp = rhs_span(c, c->scatter_span, nrhs, c->ncubes, 16, 5);
+            const int sp = scatter_span_of(c, nrhs, c->scatter_span);
             k_scatter_cta<C, NTC, 4><<<dim3((unsigned)c->ncubes, (nrhs + sp - 1) / sp), SCB, 0, c->st>>>(
                 x, c->n, P, c->T, c->d_cube_off, c->ncubes, Res<C>::bpart(c), done, nrhs, sp);
         } else if (nrhs >= 2) {
@@ -1804,9 +1818,9 @@ void gather_t(scd_ctx *c, C *y, int nrhs, const int *done) {
     if (c->ngroups == 0) return;
     typedef typename CReal<C>::type R;
     const R k2 = (R)(c->k * c->k);
+    const int sp = gather_span_of(c, nrhs, c->gather_span);
     if (nrhs >= 8) {
-        constexpr int SR = 4;
-        const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, GCB / 32 * SR, SCD_GATHER_CTAS);
+        constexpr int SR = GC_SR;
         constexpr size_t sh = sizeof(GatherShared<C, SR>);
         const cudaError_t e = launch_dyn<sh>(
             k_gather_cta<C, SR>, dim3((unsigned)c->ngroups, (nrhs + sp - 1) / sp), GCB, sh, c->st, Res<C>::R(c),
@@ -1814,12 +1828,10 @@ void gather_t(scd_ctx *c, C *y, int nrhs, const int *done) {
             c->d_pslot_cnt, y, c->n, done, nrhs, sp);
         if (e != cudaSuccess) c->launch_err = e;
     } else if (nrhs >= 4) {
-        const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, 4, SCD_GATHER_WARPS);
         k_gather<C, 4><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(
             Res<C>::R(c), Res<C>::P(c), c->T, c->d_grp_off, c->d_grp_cube, c->ngroups, G, k2, Res<C>::part(c),
             c->part_len, c->d_pslot_base, c->d_pslot_cnt, y, c->n, done, nrhs, sp);
     } else {
-        const int sp = rhs_span(c, c->gather_span, nrhs, c->ngroups, 1, SCD_GATHER_WARPS);
         k_gather<C, 1><<<dim3(gx, (nrhs + sp - 1) / sp), 32 * WARPS_PER_CTA, 0, c->st>>>(
             Res<C>::R(c), Res<C>::P(c), c->T, c->d_grp_off, c->d_grp_cube, c->ngroups, G, k2, Res<C>::part(c),
             c->part_len, c->d_pslot_base, c->d_pslot_cnt, y, c->n, done, nrhs, sp);
