@@ -61,9 +61,10 @@ SCD_HD int yz_round8(int n) { return (n + 7) & ~7; }
 template <int PY, int PZ> constexpr int yz_ex() {
     return HalfLine<PY>::EW > HalfLine<PZ>::EW ? HalfLine<PY>::EW : HalfLine<PZ>::EW;
 }
-// shared-memory elements of a CTA of `threads` for planes of nz rows
+// shared-memory elements of a CTA of `threads` for planes of nz rows; the host
+// pass (yz_plane_host) is one warp's
 template <int PY, int PZ>
-SCD_HD long long yz_smem_elems(int nz, int threads = YZ_THREADS) {
+SCD_HD long long yz_smem_elems(int nz, int threads = 32) {
     return (long long)PY + PZ + (long long)nz * YzLine<PY>::LS + (long long)(threads / 32) * yz_ex<PY, PZ>();
 }
 
