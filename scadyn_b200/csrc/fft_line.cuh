@@ -149,14 +149,17 @@ constexpr int half_row(int n1, int T) {
     while (T == 2 ? r % 16 != 8 : (r % 16 != 4 && r % 16 != 12)) ++r;
     return r;
 }
+constexpr int half_threads(int P) { return P == 40 ? 2 : P % 64 == 0 ? 8 : 4; }
+constexpr int half_es(int P) { return half_threads(P) * half_row(P / half_threads(P), half_threads(P)) + 1; }
+constexpr int half_ew(int P) { return 32 / half_threads(P) * half_es(P); }
 template <int P> struct HalfLine {
     static_assert(half_len(P), "length");
-    static constexpr int T = P == 40 ? 2 : P % 64 == 0 ? 8 : 4;
+    static constexpr int T = half_threads(P);
     static constexpr int N1 = P / T, M = N1 / 2, PER = N1 / T;
     static_assert(N1 * T == P && PER * T == N1 && 2 * M == N1, "P = T T PER");
-    static constexpr int ROW = half_row(N1, T), ES = T * ROW + 1;
+    static constexpr int ROW = half_row(N1, T), ES = half_es(P);
     static constexpr int LW = 32 / T;                // lines of a warp
-    static constexpr int EW = LW * ES;               // exchange elements of a warp
+    static constexpr int EW = half_ew(P);             // exchange elements of a warp
 };
 // thread and line of a lane: four consecutive lanes are threads 0..3
 template <int P> SCD_HD int half_t(int lane) {

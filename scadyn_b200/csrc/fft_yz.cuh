@@ -40,12 +40,11 @@
 
 constexpr int YZ_THREADS = 256;   // most threads of a CTA
 
+// plane row stride: 4 mod 8, so that four threads of four lines fall in
+// distinct banks along the rows (y) and across them (z)
+constexpr int yz_row(int PY) { return (PY + 7) / 8 * 8 + 4; }
 template <int P> struct YzLine {
-    static constexpr bool OK = half_len(P);
-    static constexpr int TPL = HalfLine<P>::T;
-    // plane row stride: 4 mod 8, so that four threads of four lines fall in
-    // distinct banks along the rows (y) and across them (z)
-    static constexpr int LS = (P + 7) / 8 * 8 + 4;
+    static constexpr int LS = yz_row(P);
 };
 
 struct YzDims {
@@ -58,15 +57,15 @@ SCD_HD int yz_fold(int u, int P) { return u <= P - u ? u : P - u; }
 SCD_HD int yz_round8(int n) { return (n + 7) & ~7; }
 
 // exchange elements of a warp
-template <int PY, int PZ> constexpr int yz_ex() {
-    return HalfLine<PY>::EW > HalfLine<PZ>::EW ? HalfLine<PY>::EW : HalfLine<PZ>::EW;
-}
+constexpr int yz_exchange(int PY, int PZ) { return half_ew(PY) > half_ew(PZ) ? half_ew(PY) : half_ew(PZ); }
+template <int PY, int PZ> constexpr int yz_ex() { return yz_exchange(PY, PZ); }
 // shared-memory elements of a CTA of `threads` for planes of nz rows; the host
 // pass (yz_plane_host) is one warp's
-template <int PY, int PZ>
-SCD_HD long long yz_smem_elems(int nz, int threads = 32) {
-    return (long long)PY + PZ + (long long)nz * YzLine<PY>::LS + (long long)(threads / 32) * yz_ex<PY, PZ>();
+constexpr long long yz_elems(int PY, int PZ, int nz, int threads) {
+    return (long long)PY + PZ + (long long)nz * yz_row(PY) + (long long)(threads / 32) * yz_exchange(PY, PZ);
 }
+template <int PY, int PZ>
+SCD_HD long long yz_smem_elems(int nz, int threads = 32) { return yz_elems(PY, PZ, nz, threads); }
 
 // ky of plane column c
 template <int PY> SCD_HD int yz_ky(int c) {

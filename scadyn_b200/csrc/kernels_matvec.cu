@@ -1595,15 +1595,9 @@ void fft_yz(scd_ctx *c, const GridDims &G, int nrg, const int *done) {
 }
 
 // least shared memory of the fused y-z pass for the context's lengths (CTAs of
-// 128 threads): the sum of fft_yz.cuh's yz_smem_elems
+// 128 threads)
 template <typename C>
-size_t yz_smem_bytes(const scd_ctx *c) {
-    auto ex = [](int P) {
-        const int T = P == 40 ? 2 : P % 64 == 0 ? 8 : 4;
-        return 32 / T * (T * half_row(P / T, T) + 1);
-    };
-    return sizeof(C) * ((size_t)c->Py + c->Pz + (size_t)c->Nz * ((c->Py + 7) / 8 * 8 + 4) + 4 * (size_t)std::max(ex(c->Py), ex(c->Pz)));
-}
+size_t yz_smem_bytes(const scd_ctx *c) { return sizeof(C) * (size_t)yz_elems(c->Py, c->Pz, c->Nz, 128); }
 
 // whether the complex64 (or FP64) chain takes the fused y-z pass: both lengths
 // have warp-synchronous line transforms and the CTA fits shared memory
