@@ -73,21 +73,41 @@ static int dalloc(scd_ctx *c, Tp **p, size_t count, const char *what) {
 }
 
 // -------------------------------------------------------------- work area
+// One allocation for all of it: the first matvec of an operator waited for nine,
+// and each can take from 50 us to milliseconds.
 int ensure_work(scd_ctx *c, int nrhs) {
-    if (c->nrhs_cap >= nrhs && c->d_x) return SCD_OK;
-    int rc;
+    if (c->nrhs_cap >= nrhs && c->d_work) return SCD_OK;
     const size_t r = (size_t)nrhs;
-    if ((rc = dalloc(c, &c->d_bpart, r * c->ncubes * 4 * 27, "box partials"))) return rc;
-    if ((rc = dalloc(c, &c->d_W, r * 4 * (size_t)c->Px * c->Py * c->Nz, "FFT work grid"))) return rc;
-    if ((rc = dalloc(c, &c->d_R, r * 4 * (size_t)c->Nx * c->Ny * c->Nz, "result grid"))) return rc;
-    if ((rc = dalloc(c, &c->d_nzpart, r * (size_t)std::max<long long>(c->part_len, 1), "near-zone partials"))) return rc;
-    if ((rc = dalloc(c, &c->d_x, r * c->n, "x"))) return rc;
-    if ((rc = dalloc(c, &c->d_y, r * c->n, "y"))) return rc;
-    if ((rc = dalloc(c, &c->d_io, r * c->n, "io"))) return rc;
-    if ((rc = dalloc(c, &c->d_rhs, r * c->n, "rhs"))) return rc;
-    if ((rc = dalloc(c, &c->d_xT, (size_t)xt_columns(nrhs) * c->n, "interleaved x"))) return rc;
-    c->nrhs_cap = nrhs;
-    return SCD_OK;
+    struct { cd **p; size_t count; } part[] = {
+        {&c->d_bpart, r * c->ncubes * 4 * 27},
+        {&c->d_W, r * 4 * (size_t)c->Px * c->Py * c->Nz},
+        {&c->d_R, r * 4 * (size_t)c->Nx * c->Ny * c->Nz},
+        {&c->d_nzpart, r * (size_t)c->part_len},
+        {&c->d_x, r * c->n},
+        {&c->d_y, r * c->n},
+        {&c->d_io, r * c->n},
+        {&c->d_rhs, r * c->n},
+        {&c->d_xT, (size_t)xt_columns(nrhs) * c->n},
+    };
+    auto whole = [](size_t count) { return (count + 15) / 16 * 16; };   // parts start on 256 bytes
+    size_t total = 0;
+    for (const auto &q : part) total += whole(q.count);
+    c->nrhs_cap = 0;
+    const int rc = dalloc(c, &c->d_work, total, "work area");
+    size_t at = 0;
+    for (const auto &q : part) {
+        *q.p = rc ? nullptr : c->d_work + at;
+        at += whole(q.count);
+    }
+    if (!rc) c->nrhs_cap = nrhs;
+    return rc;
+}
+
+// The work area of one right-hand side, at the end of set-up.  Without memory
+// for it the set-up stands, and the first call that needs it says so.
+void ensure_work_early(scd_ctx *c) {
+    const std::string err = c->err;
+    if (ensure_work(c, 1) != SCD_OK) c->err = err;
 }
 
 // The buffers a solve builds on demand -- the work areas of the right-hand
@@ -96,8 +116,8 @@ int ensure_work(scd_ctx *c, int nrhs) {
 // wavelength's once its last column is done.
 void release_work(scd_ctx *c) {
     auto fr = [](auto *&p) { if (p) { cudaFree(p); p = nullptr; } };
-    fr(c->d_bpart); fr(c->d_W); fr(c->d_R); fr(c->d_nzpart); fr(c->d_x); fr(c->d_y); fr(c->d_io); fr(c->d_rhs);
-    fr(c->d_xT);
+    fr(c->d_work);
+    c->d_bpart = c->d_W = c->d_R = c->d_nzpart = c->d_x = c->d_y = c->d_io = c->d_rhs = c->d_xT = nullptr;
     c->nrhs_cap = 0;
     fr(c->f_bpart); fr(c->f_W); fr(c->f_R); fr(c->f_nzpart); fr(c->f_xT);
     c->f_cap = 0;
@@ -476,10 +496,9 @@ int scd_destroy(scd_ctx *c) {
     cudaSetDevice(c->dev);
     if (c->st) cudaStreamSynchronize(c->st);
     void *ptrs[] = {c->d_perm, c->d_cube_off, c->d_grp_off, c->d_grp_cube, c->d_grp_tile, c->d_grp_order, c->d_kerr, c->d_P, c->d_Fo, c->d_tdata, c->d_tiles, c->d_pslot_base,
-                    c->d_pslot_cnt, c->d_tc, c->d_tvol, c->d_eps, c->d_bpart, c->d_W, c->d_R, c->d_nzpart, c->d_x,
-                    c->d_y, c->d_io, c->d_rhs,
+                    c->d_pslot_cnt, c->d_tc, c->d_tvol, c->d_eps, c->d_work,
                     c->d_bar, c->d_err, c->d_tw[0], c->d_tw[1], c->d_tw[2], c->f_P, c->f_Fo,
-                    c->f_tw[0], c->f_tw[1], c->f_tw[2], c->f_bpart, c->f_W, c->f_R, c->f_nzpart, c->d_xT, c->f_xT,
+                    c->f_tw[0], c->f_tw[1], c->f_tw[2], c->f_bpart, c->f_W, c->f_R, c->f_nzpart, c->f_xT,
                     c->d_t16, c->d_t16_off, c->d_xb, c->d_xb_off, c->d_xmax, c->d_xinv, c->d_Fyz, c->f_Fyz};
     for (void *p : ptrs) if (p) cudaFree(p);
     batch_free(c);
@@ -509,10 +528,10 @@ int scd_set_green(scd_ctx *c, const scd_c128 *Fg) {
         return set_error(c, SCD_BAD_ARG,
                          "host Fg of size (%d,%d,%d) is not a power-of-two FFT; pass NULL to build it on the device",
                          2 * c->Nx, 2 * c->Ny, 2 * c->Nz);
-    int rc = setup_green(c, Fg);
-    if (rc == SCD_OK) c->have_green = true;
-    c->f_ready = false;
+    c->have_green = c->f_ready = false;
     c->fyz_ready = c->fyz_ready_f = false;
+    const int rc = setup_green(c, Fg);
+    if (rc == SCD_OK) c->have_green = true;
     return rc;
 }
 
@@ -595,7 +614,7 @@ int scd_set_nearzone(scd_ctx *c, int64_t B, const void *sp_mat, const int32_t *s
     } else {
         rc = build_tiles<cd>(c, B, (const cd *)sp_mat, sp_ind);
     }
-    if (rc == SCD_OK) c->have_near = true;
+    if (rc == SCD_OK) { c->have_near = true; ensure_work_early(c); }
     return rc;
 }
 

@@ -137,8 +137,9 @@ struct scd_ctx {
     double *d_tvol = nullptr;            // slot-ordered tet volumes
     cd *d_eps = nullptr;                 // slot-ordered eps
 
-    // work buffers (sized for nrhs_cap right-hand sides)
+    // work buffers (sized for nrhs_cap right-hand sides), parts of d_work
     int nrhs_cap = 0;
+    cd *d_work = nullptr;
     cd *d_bpart = nullptr;               // nrhs * ncubes * 4 * 27
     cd *d_W = nullptr;                   // nrhs * 4 * Px*Py*Nz
     cd *d_R = nullptr;                   // nrhs * 4 * Nx*Ny*Nz
@@ -211,6 +212,8 @@ void launch_gather(scd_ctx *c, const cd *x, cd *y, int nrhs, const int *done);
 int scatter_span_of(const scd_ctx *c, int nrhs, int tuned);
 int gather_span_of(const scd_ctx *c, int nrhs, int tuned);
 int build_twiddles(scd_ctx *c, int P, cd **out);
+// the FP64 octant transposed for the fused y-z pass; false where the chain has three passes
+bool prepare_green_yz(scd_ctx *c);
 // tensor-core near zone (near_mma.cu)
 int near_mma_prepare(scd_ctx *c);
 void near_mma_run(scd_ctx *c, const cf *x, int nrhs, const int *done);
@@ -261,6 +264,7 @@ void launch_T_assemble(scd_ctx *c, const cd *d_mat, int ncol_total, int col0, in
 int set_error(scd_ctx *c, int code, const char *fmt, ...);
 int check_cuda(scd_ctx *c, cudaError_t e, const char *what);
 int ensure_work(scd_ctx *c, int nrhs);
+void ensure_work_early(scd_ctx *c);
 void release_work(scd_ctx *c);
 int launch_status(scd_ctx *c);   // SCD_CUDA_ERROR if a launch of a matvec was refused (and clears it)
 int near_status(scd_ctx *c);     // the same, and SCD_TIMEOUT if a near-zone pipeline wait ran out (and clears it)

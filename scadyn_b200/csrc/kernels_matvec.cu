@@ -1644,6 +1644,8 @@ int rhs_span(const scd_ctx *c, int tuned, int nrhs, int items, int unit, int per
 }
 }  // namespace
 
+bool prepare_green_yz(scd_ctx *c) { return use_yz<cd>(c) && ensure_fyz<cd>(c); }
+
 // the spans that a matvec of nrhs right-hand sides takes for a tuned value:
 // the anterpolation walks 16 at a time in five resident CTAs per SM, and all
 // of fewer than eight (k_scatter_few); the interpolation 16 from eight on

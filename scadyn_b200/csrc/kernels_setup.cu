@@ -121,9 +121,14 @@ struct TSplit {
 int setup_green(scd_ctx *c, const scd_c128 *Fg) {
     NvtxRange range("Green octant");
     const long long oct = (long long)c->Hx * c->Hy * c->Hz;
-    cd *tmp = nullptr;
-    if (c->d_Fo) { cudaFree(c->d_Fo); c->d_Fo = nullptr; }
-    if (cudaMalloc(&c->d_Fo, sizeof(cd) * oct) != cudaSuccess) return set_error(c, SCD_OOM, "Green octant");
+    auto octant = [&](cd **p) -> int {
+        if (*p || cudaMalloc(p, sizeof(cd) * oct) == cudaSuccess) return SCD_OK;
+        cudaGetLastError();
+        *p = nullptr;
+        return set_error(c, SCD_OOM, "Green octant");
+    };
+    int rc = octant(&c->d_Fo);
+    if (rc) return rc;
     const double scale = 1.0 / ((double)c->Px * (double)c->Py * (double)c->Pz);
     if (Fg) {
         // host Fg(2Nx,2Ny,2Nz) == (Px,Py,Pz): keep the octant, fold in the
@@ -135,18 +140,25 @@ int setup_green(scd_ctx *c, const scd_c128 *Fg) {
                     const scd_c128 v = Fg[(size_t)x + (size_t)c->Px * ((size_t)y + (size_t)c->Py * z)];
                     h[(size_t)x + (size_t)c->Hx * ((size_t)y + (size_t)c->Hy * z)] = cmk(v.re * scale, v.im * scale);
                 }
-        return check_cuda(c, cudaMemcpyAsync(c->d_Fo, h.data(), sizeof(cd) * oct, cudaMemcpyHostToDevice, c->st), "Green octant");
+        rc = check_cuda(c, cudaMemcpyAsync(c->d_Fo, h.data(), sizeof(cd) * oct, cudaMemcpyHostToDevice, c->st), "Green octant");
+        if (!rc) prepare_green_yz(c);
+        return rc;
     }
-    if (cudaMalloc(&tmp, sizeof(cd) * oct) != cudaSuccess) return set_error(c, SCD_OOM, "Green scratch");
+    // the axes' transforms go to and fro between the octant and the buffer that
+    // holds it transposed in the end (fft_yz.cuh), so that the first matvec
+    // neither allocates nor fills one
+    if ((rc = octant(&c->d_Fyz))) return rc;
+    cd *const tmp = c->d_Fyz;
     const int blocks = (int)std::min<long long>((oct + 255) / 256, 65535);
     k_green_spatial<<<blocks, 256, 0, c->st>>>(c->d_Fo, c->Hx, c->Hy, c->Hz, c->Nx, c->Ny, c->Nz, c->d.delta,
                                                c->d.min_coord[0], c->d.min_coord[1], c->d.min_coord[2], c->k);
     k_dct1_axis<<<blocks, 256, 0, c->st>>>(c->d_Fo, tmp, c->Hx, c->Hy, c->Hz, 0, c->Px, 1.0);
     k_dct1_axis<<<blocks, 256, 0, c->st>>>(tmp, c->d_Fo, c->Hx, c->Hy, c->Hz, 1, c->Py, 1.0);
     k_dct1_axis<<<blocks, 256, 0, c->st>>>(c->d_Fo, tmp, c->Hx, c->Hy, c->Hz, 2, c->Pz, scale);
-    int rc = check_cuda(c, cudaMemcpyAsync(c->d_Fo, tmp, sizeof(cd) * oct, cudaMemcpyDeviceToDevice, c->st), "Green");
+    rc = check_cuda(c, cudaMemcpyAsync(c->d_Fo, tmp, sizeof(cd) * oct, cudaMemcpyDeviceToDevice, c->st), "Green");
+    const bool kept = !rc && prepare_green_yz(c);
     if (!rc) rc = check_cuda(c, cudaStreamSynchronize(c->st), "Green");
-    cudaFree(tmp);
+    if (!kept) { cudaFree(c->d_Fyz); c->d_Fyz = nullptr; }
     return rc;
 }
 

@@ -760,7 +760,7 @@ int setup_nearzone_device(scd_ctx *c, int prec) {
     }
     rc = check_cuda(c, cudaGetLastError(), "near-zone launch");
     if (!rc) rc = check_cuda(c, cudaStreamSynchronize(c->st), "near-zone build");
-    if (!rc) { c->have_near = true; c->nrhs_cap = 0; c->f_cap = 0; }
+    if (!rc) { c->have_near = true; ensure_work_early(c); }
     return rc;
 }
 
