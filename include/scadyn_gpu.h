@@ -292,9 +292,9 @@ typedef struct scd_tuning {
     int32_t precision;        /* SCD_PREC_FP64 or SCD_PREC_MIXED (the complex64 matvec) */
     int32_t near_kernel;      /* SCD_NEAR_CUDA_CORES / _TENSOR_SPLIT / _TENSOR_MERGED / _TENSOR_WIDE (complex64 matvec) */
     int32_t fft_passes;       /* SCD_FFT_PASSES_FUSED_YZ or SCD_FFT_PASSES_THREE */
-    /* 0 = chosen from the sizes; rounded up to 16 from eight right-hand sides on */
+    /* 0 = chosen from the sizes; rounded up to a round of the kernel's */
     int32_t scatter_span;     /* right-hand sides per block of the anterpolation (eight or more) */
-    int32_t gather_span;      /* right-hand sides per block (below eight: per warp) of the interpolation */
+    int32_t gather_span;      /* right-hand sides per block (up to eight: per warp) of the interpolation */
     double matvec_ms;         /* the chosen setting's matvec time */
     double default_ms;        /* the library defaults' matvec time */
 } scd_tuning;

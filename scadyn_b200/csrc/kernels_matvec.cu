@@ -22,17 +22,17 @@
 namespace {
 
 constexpr int WARPS_PER_CTA = 4;
-// resident CTAs per SM the complex64 interpolation of fewer than eight
-// right-hand sides is compiled for (its register cap)
+// resident CTAs per SM the complex64 interpolation of up to eight right-hand
+// sides is compiled for (its register cap)
 #ifndef SCD_GATHER_MINB
 #define SCD_GATHER_MINB 3
 #endif
-// interpolation warps per SM that the spans of fewer than eight right-hand
-// sides aim at
+// interpolation warps per SM that the spans of up to eight right-hand sides
+// aim at
 #ifndef SCD_GATHER_WARPS
 #define SCD_GATHER_WARPS 24
 #endif
-// resident CTAs per SM of the FP64 interpolation of eight or more
+// resident CTAs per SM of the FP64 interpolation of more than eight
 // (k_gather_cta), and what the spans aim at in both precisions
 #ifndef SCD_GATHER_CTAS
 #define SCD_GATHER_CTAS 4
@@ -1372,14 +1372,17 @@ k_gather(const C *__restrict__ Rg, const C *__restrict__ P, int T, const int *__
     }
 }
 
-// The same interpolation for eight or more right-hand sides, one CTA per
+// The same interpolation for more than eight right-hand sides, one CTA per
 // (group, span): the group's 108 projector rows are staged in shared memory by
 // asynchronous copies, and the four warps take SR right-hand sides each per
 // round, in k_gather's order of sums (the same bits).  Bound by the latency of
 // the slot and node reads: 32 complex64 right-hand sides of 60k tets take 238 us
 // (334 with a warp per group that reads the rows from L1 every round), 16 FP64
 // ones of 12,864 tets 57 (67); five CTAs per SM (96 registers) take 266.
-constexpr int GCB = 128, GC_SR = 4;
+// Eight right-hand sides are two rounds of k_gather's four, which occupies more
+// warps: 8 complex64 of 43,248 tets take 104 us there and 117 here, 8 FP64 of
+// 12,864 tets 49 and 56; 9 take 130 and 124, 63 and 58.
+constexpr int GCB = 128, GC_SR = 4, GC_MIN = 9;
 template <typename C, int SR> struct GatherShared {
     C P[108][SCD_GROUP_MAX + 1];
     C R[GCB / 32][SR][4][27];
@@ -1648,14 +1651,14 @@ bool prepare_green_yz(scd_ctx *c) { return use_yz<cd>(c) && ensure_fyz<cd>(c); }
 
 // the spans that a matvec of nrhs right-hand sides takes for a tuned value:
 // the anterpolation walks 16 at a time in five resident CTAs per SM, and all
-// of fewer than eight (k_scatter_few); the interpolation 16 from eight on
-// (k_gather_cta), below that two waves of twelve warps
+// of fewer than eight (k_scatter_few); the interpolation 16 above eight
+// (k_gather_cta), up to eight two waves of twelve warps
 int scatter_span_of(const scd_ctx *c, int nrhs, int tuned) {
     return nrhs >= 8 ? rhs_span(c, tuned, nrhs, c->ncubes, 16, 5) : nrhs;
 }
 int gather_span_of(const scd_ctx *c, int nrhs, int tuned) {
-    return nrhs >= 8 ? rhs_span(c, tuned, nrhs, c->ngroups, GCB / 32 * GC_SR, SCD_GATHER_CTAS)
-                     : rhs_span(c, tuned, nrhs, c->ngroups, nrhs >= 4 ? 4 : 1, SCD_GATHER_WARPS);
+    return nrhs >= GC_MIN ? rhs_span(c, tuned, nrhs, c->ngroups, GCB / 32 * GC_SR, SCD_GATHER_CTAS)
+                          : rhs_span(c, tuned, nrhs, c->ngroups, nrhs >= 4 ? 4 : 1, SCD_GATHER_WARPS);
 }
 
 namespace {
@@ -1815,7 +1818,7 @@ void gather_t(scd_ctx *c, C *y, int nrhs, const int *done) {
     typedef typename CReal<C>::type R;
     const R k2 = (R)(c->k * c->k);
     const int sp = gather_span_of(c, nrhs, c->gather_span);
-    if (nrhs >= 8) {
+    if (nrhs >= GC_MIN) {
         constexpr int SR = GC_SR;
         constexpr size_t sh = sizeof(GatherShared<C, SR>);
         const cudaError_t e = launch_dyn<sh>(
