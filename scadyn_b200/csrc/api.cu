@@ -758,8 +758,8 @@ int scd_solve_columns(scd_ctx *c, int32_t nmat, const scd_c128 *mat, int32_t col
     if (iters) for (int j = 0; j < ncol; ++j) iters[j] = it[j];
     if (worst == SCD_OK || worst == SCD_NOT_CONVERGED) {
         // T_mat(:, col0+j) = mat^H x_j over all nmat rows (src/T_matrix.f90:260)
-        launch_T_assemble(c, c->d_mat, nmat, 0, ncol, d_X, d_T);
-        rc = check_cuda(c, cudaMemcpyAsync(Tcols, d_T, sizeof(cd) * (size_t)nmat * ncol, cudaMemcpyDeviceToHost, c->st), "T");
+        rc = launch_T_assemble(c, c->d_mat, nmat, 0, ncol, d_X, d_T);
+        if (!rc) rc = check_cuda(c, cudaMemcpyAsync(Tcols, d_T, sizeof(cd) * (size_t)nmat * ncol, cudaMemcpyDeviceToHost, c->st), "T");
         if (!rc && X) {
             for (int col = 0; col < ncol && !rc; ++col) {
                 launch_permute_out(c, d_X + (size_t)n * col, c->d_io, 1, n);
@@ -1134,22 +1134,21 @@ static int compute_T_list(scd_ctx *c, int32_t Nmax, const scd_solve_opts *o, int
     if (iters) for (int j = 0; j < ncol; ++j) iters[j] = it[j];
     if (worst == SCD_OK || worst == SCD_NOT_CONVERGED) {
         if (resident) {
-            launch_T_assemble(c, c->d_mat, ntot, 0, ncol, d_X, d_T);
+            rc = launch_T_assemble(c, c->d_mat, ntot, 0, ncol, d_X, d_T);
         } else {
             // rows c0 .. c0 + cw - 1 of T from the chunk's columns; every
             // entry is summed as in the resident path (same K split)
             for (int c0 = 0; c0 < ntot && !rc; c0 += VSWF_CHUNK) {
                 const int cw = std::min(VSWF_CHUNK, ntot - c0);
                 if ((rc = setup_vswf(c, Nmax, d_chunk, c0, cw))) break;
-                launch_T_assemble(c, d_chunk, cw, 0, ncol, d_X, d_Tc);
+                if ((rc = launch_T_assemble(c, d_chunk, cw, 0, ncol, d_X, d_Tc))) break;
                 rc = check_cuda(c, cudaMemcpy2DAsync(d_T + c0, sizeof(cd) * ntot, d_Tc, sizeof(cd) * cw, sizeof(cd) * cw,
                                                      ncol, cudaMemcpyDeviceToDevice, c->st), "T rows");
             }
-            if (rc) worst = rc;
         }
         cudaEventRecord(c->ev[5], c->st);
         std::vector<cd> h((size_t)ntot * ncol);
-        rc = check_cuda(c, cudaMemcpyAsync(h.data(), d_T, sizeof(cd) * h.size(), cudaMemcpyDeviceToHost, c->st), "T");
+        if (!rc) rc = check_cuda(c, cudaMemcpyAsync(h.data(), d_T, sizeof(cd) * h.size(), cudaMemcpyDeviceToHost, c->st), "T");
         if (!rc) rc = check_cuda(c, cudaStreamSynchronize(c->st), who);
         if (!rc) {
             // T_mat * i k^3 (src/T_matrix.f90:270-275)
@@ -1273,9 +1272,9 @@ int scd_solve_sweep(scd_ctx *const *ctxs, int32_t nw, const int32_t *Nmax, const
         cd *d_T = nullptr;
         if ((rc = dalloc(c, &d_T, (size_t)ncol * ncol, "sweep T"))) break;
         cudaStreamWaitEvent(cw->st, c->ev[5], 0);
-        launch_T_assemble(cw, cw->d_mat, ncol, 0, ncol, src.X[w], d_T);
+        if ((rc = launch_T_assemble(cw, cw->d_mat, ncol, 0, ncol, src.X[w], d_T))) set_error(c, rc, "wavelength %d: %s", w, cw->err.c_str());
         std::vector<cd> h((size_t)ncol * ncol);
-        rc = check_cuda(c, cudaMemcpyAsync(h.data(), d_T, sizeof(cd) * h.size(), cudaMemcpyDeviceToHost, cw->st), "T");
+        if (!rc) rc = check_cuda(c, cudaMemcpyAsync(h.data(), d_T, sizeof(cd) * h.size(), cudaMemcpyDeviceToHost, cw->st), "T");
         if (!rc) rc = check_cuda(c, cudaStreamSynchronize(cw->st), "sweep T");
         cudaFree(d_T);
         if (rc) break;

@@ -257,7 +257,7 @@ int setup_projectors_device(scd_ctx *c);
 int setup_nearzone_device(scd_ctx *c, int prec);
 // slot-ordered (n, 2nm), or columns c0 .. c0 + cw - 1 of it (n, cw)
 int setup_vswf(scd_ctx *c, int Nmax, cd *d_mat, int c0 = 0, int cw = -1);
-void launch_T_assemble(scd_ctx *c, const cd *d_mat, int ncol_total, int col0, int ncb,
+int launch_T_assemble(scd_ctx *c, const cd *d_mat, int ncol_total, int col0, int ncb,
                        const cd *d_X, cd *d_T);
 
 // ---- helpers (api.cu) ----

@@ -162,16 +162,27 @@ int setup_green(scd_ctx *c, const scd_c128 *Fg) {
     return rc;
 }
 
-void launch_T_assemble(scd_ctx *c, const cd *d_mat, int ncol, int col0, int ncb, const cd *d_X, cd *d_T) {
+int launch_T_assemble(scd_ctx *c, const cd *d_mat, int ncol, int col0, int ncb, const cd *d_X, cd *d_T) {
     const long long n = c->n;
     const TSplit split(n);
+    // the partial sums of as many columns at a time as there is memory for (64
+    // splits of 1,350 x 1,350 outputs are 1.9 GB)
     cd *part = nullptr;
-    cudaMallocAsync(&part, sizeof(cd) * (size_t)split.n * ncol * ncb, c->st);
-    dim3 grid(split.n, (ncol + TB - 1) / TB, (ncb + TB - 1) / TB);
-    k_tgemm_partial<<<grid, dim3(TB, TB), 0, c->st>>>(d_mat, n, ncol, d_X + (size_t)col0 * n, ncb, split.chunk, part);
-    k_tgemm_reduce<<<(ncol * ncb + 255) / 256, 256, 0, c->st>>>(part, split.n, ncol, ncb, d_T + (size_t)col0 * ncol, ncol);
+    int nb = ncb;
+    while (cudaMallocAsync(&part, sizeof(cd) * (size_t)split.n * ncol * nb, c->st) != cudaSuccess) {
+        cudaGetLastError();
+        if (nb <= 1) return set_error(c, SCD_OOM, "partial sums of T");
+        nb = (nb + 1) / 2;
+    }
+    for (int c0 = col0; c0 < col0 + ncb; c0 += nb) {
+        const int bc = std::min(nb, col0 + ncb - c0);
+        dim3 grid(split.n, (ncol + TB - 1) / TB, (bc + TB - 1) / TB);
+        k_tgemm_partial<<<grid, dim3(TB, TB), 0, c->st>>>(d_mat, n, ncol, d_X + (size_t)c0 * n, bc, split.chunk, part);
+        k_tgemm_reduce<<<(ncol * bc + 255) / 256, 256, 0, c->st>>>(part, split.n, ncol, bc, d_T + (size_t)c0 * ncol, ncol);
+        c->launches += 2;
+    }
     cudaFreeAsync(part, c->st);
-    c->launches += 2;
+    return SCD_OK;
 }
 
 

@@ -278,8 +278,8 @@ struct PoolSource final : ColumnSource {
             }
         }
         if (!rc) {
-            launch_T_assemble(c, r->d_mat, ncol, 0, ncol, r->d_X, d_T);
-            rc = check_cuda(c, cudaMemcpyAsync(h.data(), d_T, sizeof(cd) * h.size(), cudaMemcpyDeviceToHost, c->st), "T");
+            rc = launch_T_assemble(c, r->d_mat, ncol, 0, ncol, r->d_X, d_T);
+            if (!rc) rc = check_cuda(c, cudaMemcpyAsync(h.data(), d_T, sizeof(cd) * h.size(), cudaMemcpyDeviceToHost, c->st), "T");
             if (!rc) rc = check_cuda(c, cudaStreamSynchronize(c->st), "T");
         }
         cudaFree(d_T);
