@@ -867,7 +867,10 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
         if (threadIdx.x < a.ns && sact[threadIdx.x]) shn[threadIdx.x] = sqrt(tot[threadIdx.x][0]);
         __syncthreads();
     }
-    // ---- conditional re-orthogonalisation (src/gmres_module.f90:251-258)
+    // ---- conditional re-orthogonalisation (src/gmres_module.f90:251-258).
+    // Each warp keeps its items throughout: w is updated and then read for the
+    // next dot, or the norm, with no barrier between, which the work queue's
+    // warps would need
     for (int s = threadIdx.x; s < a.ns; s += blockDim.x)
         sro[s] = smode[s] == SLOT_ARNOLDI && snormav[s] + (double)0.001f * shn[s] == snormav[s];
     int jmax = 0;
@@ -875,8 +878,8 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
         for (int s = 0; s < a.ns; ++s)
             if (sro[s]) jmax = max(jmax, sstep[s] + 1);
     for (int j = 1; j <= jmax; ++j) {
-        for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-            const int s = sorder[q.it / nch], c = q.it % nch;
+        for (int it = ch.gw; it < nitems; it += ch.nw) {
+            const int s = it / nch, c = it % nch;
             if (!sro[s] || j > sstep[s] + 1) continue;
             const long long qa = c * ch.L, qb = min(n, qa + ch.L);
             const C *vj = basis_of(a, ch, s, c) + (j - 1) * ch.L;
@@ -910,8 +913,8 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
                 Hc[j - 1] = cadd(Hc[j - 1], cmk(tot[s][0], tot[s][1]));
             }
         }
-        for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-            const int s = sorder[q.it / nch], c = q.it % nch;
+        for (int it = ch.gw; it < nitems; it += ch.nw) {
+            const int s = it / nch, c = it % nch;
             if (!sact[s]) continue;
             const cd hr = cmk(tot[s][0], tot[s][1]);
             const long long qa = c * ch.L, qb = min(n, qa + ch.L);
@@ -937,8 +940,8 @@ __global__ void __launch_bounds__(BT, sizeof(C) == 8 ? SCD_TICK_MINB : 2) k_tick
         __syncthreads();   // sact / tot are rewritten by the next round
     }
     if (jmax > 0) {
-        for (WorkQueue q(a.qctr + ph++, nitems, ch); q.next();) {
-            const int s = sorder[q.it / nch], c = q.it % nch;
+        for (int it = ch.gw; it < nitems; it += ch.nw) {
+            const int s = it / nch, c = it % nch;
             if (!sro[s]) continue;
             const long long qa = c * ch.L, qb = min(n, qa + ch.L);
             const C *ws = a.w + (size_t)swpos[s] * n;
