@@ -320,7 +320,8 @@ void pool_worker(scd_server *s, std::shared_ptr<Pool> P, Req seed) {
     if (!rc) rc = scd_set_mesh(ctx, seed.Nv, seed.coord.data(), seed.etopol.data(), seed.param.data());
     if (!rc) rc = scd_set_green(ctx, nullptr);
     if (!rc) rc = scd_build_projectors(ctx);
-    if (!rc) rc = scd_build_nearzone(ctx, seed.storage_prec);
+    // not scd_build_nearzone: the solver sizes the work area for the pool's slots
+    if (!rc) rc = setup_nearzone_device(ctx, seed.storage_prec);
     std::string err = rc ? (ctx ? scd_last_error(ctx) : "context creation failed") : "";
     if (!rc) {
         P->ctx = ctx;

@@ -760,7 +760,7 @@ int setup_nearzone_device(scd_ctx *c, int prec) {
     }
     rc = check_cuda(c, cudaGetLastError(), "near-zone launch");
     if (!rc) rc = check_cuda(c, cudaStreamSynchronize(c->st), "near-zone build");
-    if (!rc) { c->have_near = true; ensure_work_early(c); }
+    if (!rc) c->have_near = true;
     return rc;
 }
 
@@ -909,7 +909,9 @@ int scd_build_projectors(scd_ctx *c) {
 int scd_build_nearzone(scd_ctx *c, int32_t prec) {
     if (!c) return SCD_BAD_ARG;
     cudaSetDevice(c->dev);
-    return setup_nearzone_device(c, prec);
+    const int rc = setup_nearzone_device(c, prec);
+    if (!rc) ensure_work_early(c);
+    return rc;
 }
 
 int scd_get_projectors(scd_ctx *c, scd_c128 *S, scd_c128 *Sx, scd_c128 *Sy, scd_c128 *Sz, int32_t *indS) {
