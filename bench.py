@@ -609,10 +609,10 @@ def main():
                              "traffic": profile_traffic(f"near_mma_{args.config}.txt")}
     # secondary: the FP64 one-right-hand-side near zone of the plain form
     prof1 = solver.profile_matvec(20, 1)
-    roof["fp64_one_rhs"] = {"kernel": "k_near_groups (FP64, one right-hand side)", "avg_launch_ms": prof1["near_kernel_ms"],
+    roof["fp64_one_rhs"] = {"kernel": "k_near_one (FP64, one right-hand side)", "avg_launch_ms": prof1["near_kernel_ms"],
                             "achieved": round(alg_bytes / (prof1["near_kernel_ms"] / 1e3) / 1e9, 1),
                             "frac": round(alg_bytes / (prof1["near_kernel_ms"] / 1e3) / 1e9 / peak, 4),
-                            "traffic": profile_traffic(f"near_groups_{args.config}.txt")}
+                            "traffic": profile_traffic(f"near_one_{args.config}.txt")}
     # whole pFFT matvec against HBM (algorithmic bytes per right-hand side,
     # four merged convolutions, operator reads shared by the batch)
     roof["matvec"] = matvec_roofline(solver, desc, mesh.n_tet, Bref, peak, prof1["matvec_ms"], profb["matvec_ms"], S)

@@ -90,13 +90,14 @@ typedef struct scd_grid_desc {
 #define SCD_FFT_SMOOTH          2   /* smallest of the powers of two and 40, 48, 80, 96, 112, 192 that is >= 2N */
 
 /* scd_grid_desc.near_kernel: the near-zone SpMV of the complex64 matvec of the
- * mixed-precision inner solves (the FP64 matvec always runs on the CUDA cores) */
+ * mixed-precision inner solves (the FP64 matvec has kernels of its own: FMAs
+ * for one right-hand side, FP64 tensor-core MMAs for more) */
 #define SCD_NEAR_DEFAULT        0   /* SCD_NEAR_TENSOR_WIDE when the blocks are stored complex64, else CUDA cores */
 #define SCD_NEAR_CUDA_CORES     1   /* complex64 FMAs on the CUDA cores */
 #define SCD_NEAR_TENSOR_SPLIT   2   /* tcgen05 MMAs on f16 hi/lo tile planes, 9 MMAs per K step */
 #define SCD_NEAR_TENSOR_MERGED  3   /* the same with x hi/lo merged into one operand, 6 MMAs per K step */
 #define SCD_NEAR_TENSOR_WIDE    4   /* the merged schedule over 32 right-hand sides per pass while more than
-                                       16 remain (each tile read once per 32, one CTA per SM), 16-wide for
+                                       16 remain (each tile read once per 32, two CTAs per SM), 16-wide for
                                        the rest; the same bits as SCD_NEAR_TENSOR_MERGED */
 
 /* near-zone storage precision */

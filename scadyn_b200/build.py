@@ -11,7 +11,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libscadyn_gpu.so")
 SOURCES = ["api.cu", "kernels_matvec.cu", "kernels_setup.cu", "setup_device.cu", "batch.cu", "server.cu", "selftest.cu", "near_mma.cu",
            "fft_yz_a.cu", "fft_yz_b.cu", "fft_yz_c.cu", "fft_yz_d.cu", "fft_yz_e.cu"]
-HEADERS = ["common.cuh", "ctx.h", "fft_reg.cuh", "near_mma.cuh", "linear_basis.h", "fft_mixed.cuh", "fft_yz.cuh", "fft_yz_py.cuh", "fft_line.cuh",
+HEADERS = ["common.cuh", "ctx.h", "fft_reg.cuh", "near_mma.cuh", "linear_basis.h", "fft_yz.cuh", "fft_yz_py.cuh", "fft_line.cuh",
            "geom.cuh", "near_pair.cuh", "lin_setup.cuh", "layout_check.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",

@@ -526,7 +526,7 @@ int scd_set_green(scd_ctx *c, const scd_c128 *Fg) {
     if (!Fg && !c->have_k) return set_error(c, SCD_NOT_READY, "scd_set_green(NULL) needs scd_set_wavenumber first");
     if (Fg && (c->Px != 2 * c->Nx || c->Py != 2 * c->Ny || c->Pz != 2 * c->Nz))
         return set_error(c, SCD_BAD_ARG,
-                         "host Fg of size (%d,%d,%d) is not a power-of-two FFT; pass NULL to build it on the device",
+                         "host Fg of size (%d,%d,%d) is not of the FFT lengths; pass NULL to build it on the device",
                          2 * c->Nx, 2 * c->Ny, 2 * c->Nz);
     c->have_green = c->f_ready = false;
     c->fyz_ready = c->fyz_ready_f = false;

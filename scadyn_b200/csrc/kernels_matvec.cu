@@ -1000,7 +1000,7 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 // row sums of unknowns 8w .. 8w + 7 of the group, kept in registers across
 // the tiles, and the column sums of unknowns 8w .. 8w + 7 of each tile's g2:
 // one element read and converted per lane feeds 4 NT DMMAs.  Bound by the
-// FP64 tensor pipe (36 TFLOP/s measured; it is active 64-70 % of the time):
+// FP64 tensor pipe (37 TFLOP/s measured; 63 % active at 16 right-hand sides):
 // 16 right-hand sides of a 12,864-tet sphere take 331 us (585 with register
 // tiles of FMAs), 16 of 3,000 tets 130 (172).
 constexpr int ND_WARPS = (3 * SCD_GROUP_MAX + 7) / 8;   // consumer warps, then the producer
