@@ -64,41 +64,66 @@ __global__ void k_dct1_axis(const cd *in, cd *out, int Hx, int Hy, int Hz, int a
 }
 
 // Tcols(r, c) = sum_i conj(mat(i, r)) X(i, c): 16x16 output tiles, split over
-// K into `nsplit` partial sums that a second kernel adds in a fixed order.
+// K into partial sums that are added in order.  Bound by shared memory (two
+// reads per complex multiply-add, 9 TFLOP/s); each step's elements are read
+// while the one before is summed: 256 x 256 outputs over 38,592 unknowns take
+// 2.26 ms, 2.52 without that, 48 x 48 89 us and 95.
 constexpr int TB = 16;
-__global__ void k_tgemm_partial(const cd *__restrict__ mat, long long n, int ncol, const cd *__restrict__ X,
-                                int ncb, long long kchunk, cd *__restrict__ part) {
-    __shared__ cd As[TB][TB + 1];
-    __shared__ cd Bs[TB][TB + 1];
+// one output's sum over k0 <= i < k1 (every thread of the tile's CTA calls it)
+__device__ __forceinline__ cd tile_sum(cd (&As)[TB][TB + 1], cd (&Bs)[TB][TB + 1], const cd *__restrict__ mat, long long n,
+                                       int ncol, const cd *__restrict__ X, int ncb, int row0, int col0, long long k0,
+                                       long long k1) {
     const int tr = threadIdx.y, tc = threadIdx.x;
-    const int r = blockIdx.y * TB + tr, cc = blockIdx.z * TB + tc;
-    const long long k0 = (long long)blockIdx.x * kchunk, k1 = min(n, k0 + kchunk);
+    const int rr = row0 + tr, c2 = col0 + tr;
+    const cd *m = rr < ncol ? mat + (long long)rr * n : nullptr, *x = c2 < ncb ? X + (long long)c2 * n : nullptr;
+    // mat(kb + tc, row0 + tr) and X(kb + tc, col0 + tr), read a step ahead
+    cd am, bx;
+    auto load = [&](long long kb) {
+        const long long kk = kb + tc;
+        am = m && kk < k1 ? m[kk] : cmk(0, 0);
+        bx = x && kk < k1 ? x[kk] : cmk(0, 0);
+    };
     cd acc = cmk(0, 0);
+    load(k0);
     for (long long kb = k0; kb < k1; kb += TB) {
-        // As[kk][rr] = mat(kb+kk, row0+rr); Bs[kk][cc] = X(kb+kk, col0+cc)
-        {
-            const long long kk = kb + tc;
-            const int rr = blockIdx.y * TB + tr;
-            As[tc][tr] = (kk < k1 && rr < ncol) ? mat[(long long)rr * n + kk] : cmk(0, 0);
-            const int c2 = blockIdx.z * TB + tr;
-            Bs[tc][tr] = (kk < k1 && c2 < ncb) ? X[(long long)c2 * n + kk] : cmk(0, 0);
-        }
+        As[tc][tr] = am;
+        Bs[tc][tr] = bx;
         __syncthreads();
+        load(kb + TB);
 #pragma unroll
         for (int kk = 0; kk < TB; ++kk) cfma_conj(acc, As[kk][tr], Bs[kk][tc]);
         __syncthreads();
     }
+    return acc;
+}
+// splits p0, p0 + 1, ... (blockIdx.x)
+__global__ void k_tgemm_partial(const cd *__restrict__ mat, long long n, int ncol, const cd *__restrict__ X,
+                                int ncb, long long kchunk, int p0, cd *__restrict__ part) {
+    __shared__ cd As[TB][TB + 1];
+    __shared__ cd Bs[TB][TB + 1];
+    const int row0 = blockIdx.y * TB, col0 = blockIdx.z * TB, r = row0 + threadIdx.y, cc = col0 + threadIdx.x;
+    const long long k0 = (p0 + (long long)blockIdx.x) * kchunk;
+    const cd acc = tile_sum(As, Bs, mat, n, ncol, X, ncb, row0, col0, k0, min(n, k0 + kchunk));
     if (r < ncol && cc < ncb) part[((long long)blockIdx.x * ncb + cc) * ncol + r] = acc;
 }
-
-// T: the first output of the block, ld rows per column
-__global__ void k_tgemm_reduce(const cd *part, int nsplit, int ncol, int ncb, cd *T, int ld) {
+// T = (first ? 0 : T) + the partial sums in order
+__global__ void k_tgemm_reduce(const cd *part, int nsplit, int nout, bool first, cd *T) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ncol * ncb) return;
+    if (i >= nout) return;
+    cd s = first ? cmk(0, 0) : T[i];
+    for (int p = 0; p < nsplit; ++p) s = cadd(s, part[(long long)p * nout + i]);
+    T[i] = s;
+}
+// every split of a tile in one CTA, the sums of k_tgemm_reduce in registers
+__global__ void k_tgemm_whole(const cd *__restrict__ mat, long long n, int ncol, const cd *__restrict__ X, int ncb,
+                              long long kchunk, cd *__restrict__ T) {
+    __shared__ cd As[TB][TB + 1];
+    __shared__ cd Bs[TB][TB + 1];
+    const int row0 = blockIdx.x * TB, col0 = blockIdx.y * TB, r = row0 + threadIdx.y, cc = col0 + threadIdx.x;
     cd s = cmk(0, 0);
-    for (int p = 0; p < nsplit; ++p) s = cadd(s, part[(long long)p * ncol * ncb + i]);
-    const int r = i % ncol, cc = i / ncol;
-    T[(long long)cc * ld + r] = s;
+    for (long long k0 = 0; k0 < n; k0 += kchunk)
+        s = cadd(s, tile_sum(As, Bs, mat, n, ncol, X, ncb, row0, col0, k0, min(n, k0 + kchunk)));
+    if (r < ncol && cc < ncb) T[(long long)cc * ncol + r] = s;
 }
 
 // The split of the sums over n unknowns, a rule on n alone, so that an entry
@@ -177,8 +202,8 @@ int launch_T_assemble(scd_ctx *c, const cd *d_mat, int ncol, int col0, int ncb, 
     for (int c0 = col0; c0 < col0 + ncb; c0 += nb) {
         const int bc = std::min(nb, col0 + ncb - c0);
         dim3 grid(split.n, (ncol + TB - 1) / TB, (bc + TB - 1) / TB);
-        k_tgemm_partial<<<grid, dim3(TB, TB), 0, c->st>>>(d_mat, n, ncol, d_X + (size_t)c0 * n, bc, split.chunk, part);
-        k_tgemm_reduce<<<(ncol * bc + 255) / 256, 256, 0, c->st>>>(part, split.n, ncol, bc, d_T + (size_t)c0 * ncol, ncol);
+        k_tgemm_partial<<<grid, dim3(TB, TB), 0, c->st>>>(d_mat, n, ncol, d_X + (size_t)c0 * n, bc, split.chunk, 0, part);
+        k_tgemm_reduce<<<(ncol * bc + 255) / 256, 256, 0, c->st>>>(part, split.n, ncol * bc, true, d_T + (size_t)c0 * ncol);
         c->launches += 2;
     }
     cudaFreeAsync(part, c->st);
@@ -193,8 +218,8 @@ int launch_T_assemble(scd_ctx *c, const cd *d_mat, int ncol, int col0, int ncb, 
 // OpenACC data regions), where a cudaMalloc inside the library would hold
 // memory outside that allocator's accounting and synchronise the device.
 // The split-K partial sums live in this fixed file-scope array instead of a
-// cudaMallocAsync buffer; outputs whose splits exceed it are formed block by
-// block, with the bits of launch_T_assemble.
+// cudaMallocAsync buffer; where it does not hold all splits, they are summed a
+// few at a time, with the bits of launch_T_assemble.
 #define SCD_NOALLOC_SCRATCH (1 << 18)   // complex doubles: 4 MiB per device
 static __device__ __align__(256) cd g_noalloc_scratch[SCD_NOALLOC_SCRATCH];
 
@@ -223,32 +248,33 @@ extern "C" SCD_API int scd_T_assemble_noalloc(const scd_c128 *mat, int64_t n, in
         g_noalloc_ptr[dev].store(part, std::memory_order_release);
     }
     cudaStream_t st = (cudaStream_t)stream;
-    // blocks of nr x nc outputs, whole tiles of 16 and at least 64 x 64 of them
-    // (4,096 times 64 splits fill the scratch); every partial entry is written
-    // before it is read, so nothing needs clearing between blocks or calls.
-    // One pass with the splits that fit would give other bits and be 5-8 %
-    // faster where many blocks are needed (500 x 500 over 38,592 unknowns 10.0
-    // ms against 10.5); 48 x 48 fit one block (207 -> 97 us with TSplit).
+    // as many splits at a time as the scratch holds, shared evenly over the
+    // passes (a full scratch is 1,024 CTAs' tiles, one wave); every partial entry
+    // is written before it is read, so nothing needs clearing between calls.
+    // Where the scratch holds one split, the 513 tiles or more fill the SMs by
+    // themselves: 500 x 500 over 9,000 unknowns take 1.88 ms (2.36 in a pass per
+    // split, without the reads ahead; 1.91 so in one pass); 300 x 300, two splits
+    // a pass, 759 us against 828 in one CTA a tile.
     const TSplit split(n);
-    const int most = SCD_NOALLOC_SCRATCH / split.n;
-    int nr = std::min(ncol, 64);
-    const int nc = std::min(ncb, std::max(most / nr / TB * TB, TB));
-    nr = std::min(ncol, std::max(most / nc / TB * TB, TB));
-    for (int c0 = 0; c0 < ncb; c0 += nc)
-        for (int r0 = 0; r0 < ncol; r0 += nr) {
-            const int br = std::min(nr, ncol - r0), bc = std::min(nc, ncb - c0);
-            dim3 grid(split.n, (br + TB - 1) / TB, (bc + TB - 1) / TB);
-            k_tgemm_partial<<<grid, dim3(TB, TB), 0, st>>>((const cd *)mat + r0 * n, n, br, (const cd *)X + c0 * n, bc,
-                                                           split.chunk, part);
-            if (cudaPeekAtLastError() != cudaSuccess) {
-                cudaGetLastError();   // this launch's own error
-                return SCD_CUDA_ERROR;
-            }
-            k_tgemm_reduce<<<(br * bc + 255) / 256, 256, 0, st>>>(part, split.n, br, bc, (cd *)T + (size_t)c0 * ncol + r0, ncol);
-            if (cudaPeekAtLastError() != cudaSuccess) {
-                cudaGetLastError();
-                return SCD_CUDA_ERROR;
-            }
-        }
+    const int nout = ncol * ncb, most = SCD_NOALLOC_SCRATCH / nout;
+    const int passes = (split.n + most - 1) / most, per = (split.n + passes - 1) / passes;
+    const dim3 tiles((ncol + TB - 1) / TB, (ncb + TB - 1) / TB);
+    auto refused = [] {
+        if (cudaPeekAtLastError() == cudaSuccess) return false;
+        cudaGetLastError();   // this launch's own error
+        return true;
+    };
+    if (most == 1 && split.n > 1) {
+        k_tgemm_whole<<<tiles, dim3(TB, TB), 0, st>>>((const cd *)mat, n, ncol, (const cd *)X, ncb, split.chunk, (cd *)T);
+        return refused() ? SCD_CUDA_ERROR : SCD_OK;
+    }
+    for (int p0 = 0; p0 < split.n; p0 += per) {
+        const int np = std::min(per, split.n - p0);
+        k_tgemm_partial<<<dim3(np, tiles.x, tiles.y), dim3(TB, TB), 0, st>>>((const cd *)mat, n, ncol, (const cd *)X, ncb,
+                                                                            split.chunk, p0, part);
+        if (refused()) return SCD_CUDA_ERROR;
+        k_tgemm_reduce<<<(nout + 255) / 256, 256, 0, st>>>(part, np, nout, p0 == 0, (cd *)T);
+        if (refused()) return SCD_CUDA_ERROR;
+    }
     return SCD_OK;
 }

@@ -1,6 +1,7 @@
 """scd_T_assemble_noalloc gives the bits of the T columns that scd_solve_columns
-assembles from the same solutions, over the counts of splits (1, 17, 64) and of
-outputs that fit the fixed scratch in one block or need several."""
+assembles from the same solutions, over the counts of splits (1, 3, 17, 64) and
+of outputs whose splits fit the fixed scratch together, a few at a time or (more
+than 131,072 outputs) not even two."""
 import numpy as np
 import pytest
 
@@ -10,7 +11,8 @@ from tests.diag_operator import diagonal_solver, random_columns
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("tets,ncol", [(100, 30), (3000, 130), (11000, 7), (11000, 64), (11000, 100)])
+@pytest.mark.parametrize("tets,ncol", [(100, 30), (3000, 130), (11000, 7), (11000, 64), (11000, 100),
+                                       (600, 362), (600, 363)])
 def test_same_bits(tets, ncol):
     import torch
     lam = np.where(np.arange(tets) % 2, 1.0 + 0.1j, 2.0 - 0.3j)
