@@ -1303,7 +1303,9 @@ static int launch_tick(scd_ctx *c, BatchBuffers &bb, int ns, int nact, int m, in
     const int grid = (int)std::min<long long>(std::is_same<C, cf>::value ? bb.grid_f : bb.grid, (items + BW - 1) / BW);
     // modified Gram-Schmidt keeps w resident while every warp's items of the
     // slots fit its share of shared memory (two CTAs of 96 KB per SM) and a
-    // warp can add a slot's partials itself (512: sixteen loads per lane)
+    // warp can add a slot's partials itself (512: sixteen loads per lane).  One
+    // column, 14 steps: 352 chunks 3.84 ms (streamed 3.97), 511 4.58 (4.65), 514
+    // 4.65 (4.69 streamed, as it is there), 704 5.50 (5.45), 2,040 12.36 (10.97)
     const long long warps = (long long)grid * BW, per = (items + warps - 1) / warps;
     a.res = !a.cgs && Chunks::count(n) <= 512 && per <= RES<C> ? (int)per : 0;
     const size_t dyn = (size_t)BW * a.res * CHUNK * sizeof(C);
